@@ -301,8 +301,6 @@ void launch_pcg_setup_half(const HalfMatrix& H, const double* b, const float4* d
                            float4* p0, double rtol, int max_iters, bool negate, const Reduce& red, cudaStream_t st);
 // Chronopoulos-Gear PCG on the FP16 copy in one cooperative launch (as launch_pcg_persistent variant 2);
 // x holds the unscaled solution on return.  false if the device cannot launch it cooperatively.
-// the pipelined solve on the copy does its own set-up and, with check set, the solve's check on the FP32
-// symmetric store (A32, vals32): g . x, |x|^2, |sign b - K x|^2, |b|^2 into sc->gd, dnorm2, true_rr, true_bb
 struct HalfSolveArgs {
   const double* b;  // right-hand side sign * b (the Newton gradient g with negate = 1)
   int negate;
@@ -313,13 +311,23 @@ struct HalfSolveArgs {
   SellMatrix A32;
   const float* vals32;
 };
-// pm and pa non-null: the pipelined solve (pipe_persistent_kernel's scheme, 2 nv vectors of scratch in pm)
-// with its set-up and check in the same launch (no launch_pcg_setup_half before it); otherwise
-// Chronopoulos-Gear after launch_pcg_setup_half
 bool launch_pcg_half(const HalfMatrix& H, const float4* dinv16, float4* x, float4* r, float4* z, float4* p0,
                      float4* p1, float4* q, int max_iters, const Reduce& red, unsigned long long* gsync,
-                     long long spin_limit, int extra, int max_blocks, cudaStream_t st, float4* pm = nullptr,
-                     const HalfSolveArgs* pa = nullptr);
+                     long long spin_limit, int extra, int max_blocks, cudaStream_t st);
+// grid exchange of the resident solves (kernels_pcg.cu): resident_sync_bytes() of device memory; extra and
+// spin_limit as the persistent kernels' (0: 2^21 polls, about a second)
+struct ResidentSync {
+  unsigned char* mem;
+  int extra;
+  long long spin_limit;
+};
+size_t resident_sync_bytes();
+// pipelined PCG on the copy, the whole solve in one launch (set-up, iterations, x unscaled and, with a.check, the
+// check); off_host: host copy of H.off; r, z, p, sv, w: nv vectors of scratch, m: 2 nv.  false if the device cannot
+// launch it (the caller then runs the FP32 values)
+bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, const float4* dinv16, float4* x, float4* r,
+                              float4* z, float4* p, float4* sv, float4* w, float4* m, const HalfSolveArgs& a,
+                              const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st);
 // after a solve on the FP16 copy: g . d, |d|^2 (as launch_dot_gd) and the solve's true residual on the FP32
 // symmetric values, |-g - K d|^2 and |g|^2 (sc->true_rr, sc->true_bb)
 void launch_dot_gd_check(const SellMatrix& A, const float* vals, const double* g, const float4* d, const Reduce& red,

@@ -1,0 +1,732 @@
+// kernels_pcg.cu -- resident PCG: a whole solve in one cooperative launch of one block per SM whose rows'
+// vectors stay in shared memory from the set-up to the end.
+//
+// Each block owns a contiguous range of 32-row slices.  An SpMV is cut into units of one slice's every T-th
+// entry (T warps share a slice, so a small system still fills the SM's warps and a large one divides evenly
+// over them); the units' partial products meet in shared memory, where one thread per row adds them in order
+// and makes the row's recurrences.  Only the vector that other rows gather (m, or p) is in global memory.
+//
+// The grid's reductions (exchange) have one counter: every block stores its sums, arrives with one acquire-release
+// atomic, polls the counter and then adds all blocks' sums itself, in the same order, so the totals and the scalars
+// made from them are the same bits everywhere and no block waits for another to combine or to announce them: one
+// trip through L2 where counted groups, their sums and a release word take three.
+//
+// Measured on a GB300 (us per iteration of a whole solve on the FP16 copy, against the earlier kernel of 256-row
+// virtual blocks with all vectors in global memory and counted group barriers): 1.02M-tet beam 10.4 (21.3), 192k-tet
+// bar 5.2 (12.6), 64-cube batch of 1.9M tets 43 (53).  Cycles of a beam iteration: SpMV 10,800, exchange 5,000, row
+// recurrences 4,600.
+
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "pcg_common.cuh"
+
+namespace ssim_gb {
+namespace {
+
+constexpr int kMaxBlocks = 192;  // blocks of a resident launch (one per SM), a multiple of 32
+
+struct GridExchange {
+  unsigned long long* count;  // arrivals since the launch (zeroed before it)
+  double* words;              // [2][4][kMaxBlocks] the blocks' sums of each value, double-buffered
+  unsigned int extra;         // arrivals waited for beyond the grid (test hook: every wait runs out)
+  long long spin_limit;
+};
+
+__device__ __forceinline__ void bar_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
+}
+__device__ __forceinline__ void arrive_acq_rel(unsigned long long* p) {
+  unsigned long long old;
+  asm volatile("atom.add.acq_rel.gpu.global.u64 %0, [%1], 1;" : "=l"(old) : "l"(p) : "memory");
+}
+
+// shared memory of the exchanges
+struct ExchangeShared {
+  double own[4];  // this block's sums
+  double tot[4];  // totals over the blocks
+  int fail;
+};
+
+__device__ __forceinline__ double warp_add(double v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
+// An exchange has two parts; every thread of the block calls each.  GB300's FP64 unit takes a warp's addition every
+// 64 cycles and adds no faster with more of them in flight, so each value's sums run in a warp of their own (there
+// are four units an SM).
+//
+// exchange_wait number k (0, 1, ... in a launch), after a block-wide barrier that follows the block's partials
+// sh[v * stride + i], i < np: warps 0 .. NV - 1 sum one value each (in FP64, lane-strided, then a shuffle tree), warp
+// 0 stores the sums, arrives and polls.  The closing block-wide barrier releases the others: they see the global
+// writes that any block made before the exchange.  false in every thread of a block whose wait ran out.  NV = 0: the
+// barrier alone.  (Measured on 152 blocks of 1024 threads with a global write each before it: 3,115 cycles for the
+// arrival and the wait, 1,906 of them the release's fence; polling 152 blocks' words {value, flag} instead, in one
+// place or in a mailbox per block, 6,700 to 7,700: strong loads of many addresses are slow.)
+template <typename S, int NV>
+__device__ __forceinline__ bool exchange_wait(const GridExchange& gx, unsigned long long k, const S* sh, int stride,
+                                              int np, ExchangeShared& xs) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  if constexpr (NV > 0) {
+    if (warp < NV) {
+      double v = 0.0;
+      for (int i = lane; i < np; i += 32) v += (double)sh[warp * stride + i];
+      v = warp_add(v);
+      if (lane == 0) xs.own[warp] = v;
+      bar_sync(1, 32 * NV);
+    }
+  }
+  if (warp == 0) {
+    if (lane < NV) gx.words[((k & 1) * 4 + lane) * kMaxBlocks + blockIdx.x] = xs.own[lane];
+    __syncwarp();
+    if (lane == 0) {
+      const unsigned long long target = (k + 1) * (unsigned long long)(gridDim.x + gx.extra);
+      arrive_acq_rel(gx.count);
+      long long n = 0;
+      while (ld_acquire(gx.count) < target) {
+        if (++n > gx.spin_limit) {
+          xs.fail = 1;
+          break;
+        }
+      }
+    }
+  }
+  __syncthreads();
+  return xs.fail == 0;
+}
+// exchange_total: warps 0 .. NV - 1 add one value's words of all blocks and warp 0's lane 0 hands the totals to epi; a
+// block-wide barrier has to follow before another thread reads what epi wrote.  The other warps pass straight
+// through.  Words of exchange k are overwritten by exchange k + 2, which no block reaches before every block arrived
+// at k + 1, after its reads of k.
+template <int NV, typename EPI>
+__device__ __forceinline__ void exchange_total(const GridExchange& gx, unsigned long long k, ExchangeShared& xs,
+                                               EPI&& epi) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp >= NV) return;
+  const double* w = gx.words + ((k & 1) * 4 + warp) * kMaxBlocks;
+  double v[kMaxBlocks / 32];
+#pragma unroll
+  for (int j = 0; j < kMaxBlocks / 32; ++j) v[j] = lane + 32 * j < (int)gridDim.x ? __ldcg(w + lane + 32 * j) : 0.0;
+  double t = v[0];
+#pragma unroll
+  for (int j = 1; j < kMaxBlocks / 32; ++j)
+    if (32 * j < (int)gridDim.x) t += v[j];
+  t = warp_add(t);
+  if (lane == 0) xs.tot[warp] = t;
+  if constexpr (NV > 1) bar_sync(2, 32 * NV);
+  if (threadIdx.x == 0) {
+    double tot[NV];
+#pragma unroll
+    for (int c = 0; c < NV; ++c) tot[c] = xs.tot[c];
+    epi(tot);
+  }
+}
+// the whole exchange, partials to totals
+template <typename S, int NV, typename EPI>
+__device__ __forceinline__ bool exchange(const GridExchange& gx, unsigned long long k, const S* sh, int stride, int np,
+                                         ExchangeShared& xs, EPI&& epi) {
+  __syncthreads();
+  if (!exchange_wait<S, NV>(gx, k, sh, stride, np, xs)) return false;
+  exchange_total<NV>(gx, k, xs, epi);
+  __syncthreads();
+  return true;
+}
+__device__ __forceinline__ bool exchange_barrier(const GridExchange& gx, unsigned long long k, ExchangeShared& xs) {
+  __syncthreads();
+  return exchange_wait<float, 0>(gx, k, nullptr, 0, 0, xs);
+}
+
+// One unit of y = A x on the symmetric store: slice s's upper slots part, part + T, ... and lower slots
+// T - 1 - part, ... (the two run against each other, so the parts get equal shares), two slots in flight.
+template <typename S>
+__device__ __forceinline__ void sym_unit(const SellMatrix& A, const S* __restrict__ vals, int s, int lane, int part,
+                                         int T, const V4<S>* x, S& a0, S& a1, S& a2) {
+  const int ub = A.sl_off[s], Wu = (A.sl_off[s + 1] - ub) >> 5;
+  const int lb = A.lo_off[s], Wl = (A.lo_off[s + 1] - lb) >> 5;
+  a0 = a1 = a2 = S(0);
+  for (int k = part; k < Wu; k += 2 * T) {
+    const bool two = k + T < Wu;
+    const int q0 = ub + 32 * k + lane, q1 = two ? q0 + 32 * T : q0;
+    const int c0 = A.sl_col[q0], c1 = A.sl_col[q1];
+    const S *p0 = vals + sell_base(q0), *p1 = vals + sell_base(q1);
+    S v[9], w[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) v[m] = p0[32 * m];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) w[m] = two ? p1[32 * m] : S(0);
+    const V4<S> x0 = x[c0], x1 = x[c1];
+    a0 += v[0] * x0.x + v[1] * x0.y + v[2] * x0.z;
+    a1 += v[3] * x0.x + v[4] * x0.y + v[5] * x0.z;
+    a2 += v[6] * x0.x + v[7] * x0.y + v[8] * x0.z;
+    if (two) {
+      a0 += w[0] * x1.x + w[1] * x1.y + w[2] * x1.z;
+      a1 += w[3] * x1.x + w[4] * x1.y + w[5] * x1.z;
+      a2 += w[6] * x1.x + w[7] * x1.y + w[8] * x1.z;
+    }
+  }
+  for (int k = T - 1 - part; k < Wl; k += 2 * T) {
+    const bool two = k + T < Wl;
+    const int i0 = lb + 32 * k + lane, i1 = two ? i0 + 32 * T : i0;
+    const int c0 = A.lo_col[i0], c1 = A.lo_col[i1];
+    const S *p0 = vals + sell_base(A.lo_src[i0]), *p1 = vals + sell_base(A.lo_src[i1]);
+    S v[9], w[9];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) v[m] = p0[32 * m];
+#pragma unroll
+    for (int m = 0; m < 9; ++m) w[m] = two ? p1[32 * m] : S(0);
+    const V4<S> x0 = x[c0], x1 = x[c1];
+    a0 += v[0] * x0.x + v[3] * x0.y + v[6] * x0.z;
+    a1 += v[1] * x0.x + v[4] * x0.y + v[7] * x0.z;
+    a2 += v[2] * x0.x + v[5] * x0.y + v[8] * x0.z;
+    if (two) {
+      a0 += w[0] * x1.x + w[3] * x1.y + w[6] * x1.z;
+      a1 += w[1] * x1.x + w[4] * x1.y + w[7] * x1.z;
+      a2 += w[2] * x1.x + w[5] * x1.y + w[8] * x1.z;
+    }
+  }
+}
+
+// ------------------------------------------------------------------ FP16 copy, pipelined
+// How a resident solve is laid out (resident_plan): the grid, T, how many of a block's slices keep their
+// vectors in shared memory, how many slices one pass covers, and whether the block's matrix entries fit too.
+struct HalfPlan {
+  int grid, T, spc, res, tile, cached;  // spc: most slices of a block; res, tile in slices
+  int cache_entries;                    // most entries of a block (when cached)
+  size_t smem;
+};
+
+constexpr int HT = 1024;        // threads of a block
+constexpr int kHalfState = 27;  // FP32 values of a row kept on chip: x r p s z w (18), 1/scale (3), M (6)
+
+__device__ __forceinline__ float2 unpack_h2(unsigned int w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+
+__device__ __forceinline__ void half_fma(const uint4& p, uint16_t h8, const float4& xv, float& a0, float& a1, float& a2) {
+  const float2 f01 = unpack_h2(p.x), f23 = unpack_h2(p.y), f45 = unpack_h2(p.z), f67 = unpack_h2(p.w);
+  const float f8 = __half2float(__ushort_as_half(h8));
+  a0 = fmaf(f23.x, xv.z, fmaf(f01.y, xv.y, fmaf(f01.x, xv.x, a0)));
+  a1 = fmaf(f45.y, xv.z, fmaf(f45.x, xv.y, fmaf(f23.y, xv.x, a1)));
+  a2 = fmaf(f8, xv.z, fmaf(f67.y, xv.y, fmaf(f67.x, xv.x, a2)));
+}
+
+// Entries k0, k0 + T, ... of a slice of width W (col / v8 / v1: its first entry, this lane): four at a time with all
+// their loads in flight.  The kernel is bound by the instructions it issues (59% of the issue slots in a first
+// version with run-time strides and a predicate per entry), so T is a compile-time stride (immediate offsets) and
+// only a unit's ragged end tests the width.
+template <int T>
+__device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const uint16_t* v1, int W, int k0,
+                                          const float4* x, float& a0, float& a1, float& a2) {
+  col += 32 * k0;
+  v8 += 32 * k0;
+  v1 += 32 * k0;
+  int n = W - k0;  // entries 0, T, ... < n remain
+  for (; n > 3 * T; n -= 4 * T) {
+    int c[4];
+    uint4 p[4];
+    uint16_t h[4];
+    float4 xv[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = col[32 * T * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      p[j] = v8[32 * T * j];
+      h[j] = v1[32 * T * j];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) xv[j] = x[c[j]];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) half_fma(p[j], h[j], xv[j], a0, a1, a2);
+    col += 128 * T;
+    v8 += 128 * T;
+    v1 += 128 * T;
+  }
+  if (n > 0) {  // one to three entries: the missing ones repeat the first with a zero vector
+    const int o1 = n > T ? 32 * T : 0, o2 = n > 2 * T ? 64 * T : 0;
+    const int c0 = col[0], c1 = col[o1], c2 = col[o2];
+    const uint4 p0 = v8[0], p1 = v8[o1], p2 = v8[o2];
+    const uint16_t h0 = v1[0], h1 = v1[o1], h2 = v1[o2];
+    const float4 x0 = x[c0];
+    float4 x1 = x[c1], x2 = x[c2];
+    if (n <= T) x1 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (n <= 2 * T) x2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    half_fma(p0, h0, x0, a0, a1, a2);
+    half_fma(p1, h1, x1, a0, a1, a2);
+    half_fma(p2, h2, x2, a0, a1, a2);
+  }
+}
+
+// Pipelined PCG on the FP16 copy (Ghysels & Vanroose, Parallel Computing 40(7), 2014), in the copy's scaled
+// space, as one launch: the set-up (x = 0, r~ = S (sign b), u0 = M r~), the iterations, x unscaled and, when
+// a.check is set, the solve's check on the FP32 symmetric store: g . x, |x|^2, |sign b - K x|^2 and |b|^2.
+// With u = M r, w = A u, m = M w, s = A p, z = A M s (M per vertex, so u and M s are formed where needed):
+//   prologue:  w = A u0, m_0 = M w;       partials (r, u), (w, u), (r, r)                -> exchange
+//   phase k:   n = A m_k;  z = n + beta z,  s = w + beta s,  p = M r + beta p;
+//              x += alpha p,  r -= alpha s,  w -= alpha z;  m_{k+1} = M w;  partials    -> exchange
+// One exchange per iteration both sums the dots and orders m's writes.  The scalars (cgcg_after) and the stop
+// rule are Chronopoulos-Gear's; the third dot is (r, r) of the unscaled residual.  In FP32 the recursive residual
+// drifts from the true one with the iterations and the condition number, so after pipe_iters iterations the
+// solve continues as Chronopoulos-Gear PCG from the same state (w = A u recomputed, two exchanges a round).
+// CACHED: the block's matrix entries are in shared memory too.
+template <bool CACHED, int T>
+__global__ void __launch_bounds__(HT, 1)
+    resident_half_kernel(HalfMatrix H, const float4* __restrict__ dinv, float4* x, float4* r, float4* z, float4* p,
+                         float4* sv, float4* w, float4* m, HalfSolveArgs a, HalfPlan pl, Reduce red, GridExchange gx) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ ExchangeShared xs;
+  __shared__ DevScalars sc;
+  __shared__ float s_ab[2];  // alpha, beta
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nv = H.nv, nsl = (nv + 31) >> 5;
+  constexpr int lt = T == 8 ? 3 : 2;
+  static_assert(T == 1 << lt, "T is 4 or 8");
+  const int s0 = (int)((long long)blockIdx.x * nsl / gridDim.x), ns = (int)((long long)(blockIdx.x + 1) * nsl / gridDim.x) - s0;
+  const int RS = 32 * pl.res, PR = 32 * pl.tile;
+  // shared memory: cached matrix entries (16-byte values first), row state, unit partials, per-slice dots, offsets
+  uint4* c8 = reinterpret_cast<uint4*>(smem);
+  float* st = reinterpret_cast<float*>(smem + (size_t)16 * pl.cache_entries);
+  float* pb = st + (size_t)kHalfState * RS;
+  float* shw = pb + (size_t)3 * T * PR;
+  int* off = reinterpret_cast<int*>(shw + 4 * pl.spc);
+  int* ccol = off + pl.spc + 1;
+  uint16_t* c1 = reinterpret_cast<uint16_t*>(ccol + pl.cache_entries);
+  if (tid == 0) xs.fail = 0;
+  for (int i = tid; i <= ns; i += HT) off[i] = H.off[s0 + i];
+  __syncthreads();
+  const int e0 = off[0];
+  if constexpr (CACHED) {
+    const int ne = off[ns] - e0;
+    for (int i = tid; i < ne; i += HT) {
+      c8[i] = H.v8[e0 + i];
+      ccol[i] = H.col[e0 + i];
+      c1[i] = H.v1[e0 + i];
+    }
+  }
+  unsigned long long nx = 0;  // exchanges so far
+
+  // products of the slices t0 .. t1 - 1 into the unit partials
+  auto spmv = [&](const float4* v, int t0, int t1) {
+    const int nu = (t1 - t0) << lt;
+    // warps count down: the low ones, which form the scalars meanwhile, get the round that is not full
+    for (int i = HT / 32 - 1 - warp; i < nu; i += HT / 32) {
+      const int b = off[t0 + (i >> lt)], W = (off[t0 + (i >> lt) + 1] - b) >> 5;
+      float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+      if constexpr (CACHED)
+        half_unit<T>(ccol + (b - e0) + lane, c8 + (b - e0) + lane, c1 + (b - e0) + lane, W, i & (T - 1), v, a0, a1, a2);
+      else
+        half_unit<T>(H.col + b + lane, H.v8 + b + lane, H.v1 + b + lane, W, i & (T - 1), v, a0, a1, a2);
+      float* o = pb + (size_t)3 * (i & (T - 1)) * PR + 32 * (i >> lt) + lane;
+      o[0] = a0;
+      o[PR] = a1;
+      o[2 * PR] = a2;
+    }
+  };
+  auto product = [&](int l, int t0, float& n0, float& n1, float& n2) {  // the row's product from its T partials
+    const float* o = pb + (l - 32 * t0);
+    n0 = o[0];
+    n1 = o[PR];
+    n2 = o[2 * PR];
+#pragma unroll
+    for (int q = 1; q < T; ++q) {
+      o += 3 * (size_t)PR;
+      n0 += o[0];
+      n1 += o[PR];
+      n2 += o[2 * PR];
+    }
+  };
+  // component f of row l's state: shared memory for the first RS rows, the vectors in global memory beyond
+  auto ld3 = [&](int f, const float4* g, int l, int u, float (&v)[3]) {
+    if (l < RS) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) v[c] = st[(size_t)(f + c) * RS + l];
+    } else {
+      const float4 t = g[u];
+      v[0] = t.x;
+      v[1] = t.y;
+      v[2] = t.z;
+    }
+  };
+  auto st3 = [&](int f, float4* g, int l, int u, const float (&v)[3]) {
+    if (l < RS) {
+#pragma unroll
+      for (int c = 0; c < 3; ++c) st[(size_t)(f + c) * RS + l] = v[c];
+    } else {
+      g[u] = make_float4(v[0], v[1], v[2], 0.f);
+    }
+  };
+  constexpr int FX = 0, FR = 3, FP = 6, FS = 9, FZ = 12, FW = 15, FI = 18, FM = 21;
+  auto ldm = [&](int l, int u, float (&d)[6]) {
+    if (l < RS) {
+#pragma unroll
+      for (int c = 0; c < 6; ++c) d[c] = st[(size_t)(FM + c) * RS + l];
+    } else {
+      const float4 d0 = dinv[3 * (size_t)u], d1 = dinv[3 * (size_t)u + 1], d2 = dinv[3 * (size_t)u + 2];
+      d[0] = d0.x;
+      d[1] = d0.y;
+      d[2] = d0.z;
+      d[3] = d1.y;
+      d[4] = d1.z;
+      d[5] = d2.z;
+    }
+  };
+  auto mul = [](const float (&d)[6], const float (&v)[3], float (&o)[3]) {  // the symmetric 3x3 block-Jacobi rows
+    o[0] = d[0] * v[0] + d[1] * v[1] + d[2] * v[2];
+    o[1] = d[1] * v[0] + d[3] * v[1] + d[4] * v[2];
+    o[2] = d[2] * v[0] + d[4] * v[1] + d[5] * v[2];
+  };
+  // the three dots of a 32-row slice, summed in FP32 within the warp: the first two levels split the values over
+  // the lanes (6 shuffles instead of 15)
+  auto dots = [&](int l, float d0, float d1, float d2) {
+    const bool hi = lane & 16, odd = lane & 8;
+    float u = hi ? d2 : d0, v = hi ? 0.f : d1;
+    u += __shfl_xor_sync(0xffffffffu, hi ? d0 : d2, 16);
+    v += __shfl_xor_sync(0xffffffffu, hi ? d1 : 0.f, 16);
+    float t = odd ? v : u;
+    t += __shfl_xor_sync(0xffffffffu, odd ? u : v, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if ((lane & 7) == 0 && lane < 24) shw[(lane >> 3) * pl.spc + (l >> 5)] = t;
+  };
+  auto unscaled2 = [](const float (&rv)[3], const float (&is)[3]) {
+    const float t0 = rv[0] * is[0], t1 = rv[1] * is[1], t2 = rv[2] * is[2];
+    return t0 * t0 + t1 * t1 + t2 * t2;
+  };
+
+  // set-up
+  const double sg = a.negate ? -1.0 : 1.0;
+  for (int l = tid; l < 32 * ns; l += HT) {
+    const int u = 32 * s0 + l;
+    if (u >= nv) continue;
+    const float4 s4 = H.scale[u];
+    const float rv[3] = {(float)(sg * a.b[3 * (size_t)u]) * s4.x, (float)(sg * a.b[3 * (size_t)u + 1]) * s4.y,
+                         (float)(sg * a.b[3 * (size_t)u + 2]) * s4.z};
+    const float zero[3] = {0.f, 0.f, 0.f};
+    const float4 d0 = dinv[3 * (size_t)u], d1 = dinv[3 * (size_t)u + 1], d2 = dinv[3 * (size_t)u + 2];
+    const float d[6] = {d0.x, d0.y, d0.z, d1.y, d1.z, d2.z};
+    if (l < RS) {
+      const float4 i4 = H.iscale[u];
+      const float is[3] = {i4.x, i4.y, i4.z};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) st[(size_t)(FI + c) * RS + l] = is[c];
+#pragma unroll
+      for (int c = 0; c < 6; ++c) st[(size_t)(FM + c) * RS + l] = d[c];
+    }
+    st3(FX, x, l, u, zero);
+    st3(FR, r, l, u, rv);
+    st3(FP, p, l, u, zero);
+    st3(FS, sv, l, u, zero);
+    st3(FZ, z, l, u, zero);
+    float uv[3];
+    mul(d, rv, uv);
+    m[(size_t)nv + u] = make_float4(uv[0], uv[1], uv[2], 0.f);  // u0 in the second half of m
+  }
+  bool ok = exchange_barrier(gx, nx++, xs);
+  // prologue
+  if (ok) {
+    for (int t0 = 0; t0 < ns; t0 += pl.tile) {
+      const int t1 = min(ns, t0 + pl.tile);
+      spmv(m + nv, t0, t1);
+      __syncthreads();
+      for (int l = 32 * t0 + tid; l < 32 * t1; l += HT) {
+        const int u = 32 * s0 + l;
+        float e0d = 0.f, e1d = 0.f, e2d = 0.f;
+        if (u < nv) {
+          float n[3], rv[3], is[3], d[6], uv[3], mv[3];
+          product(l, t0, n[0], n[1], n[2]);
+          ld3(FR, r, l, u, rv);
+          ld3(FI, H.iscale, l, u, is);
+          ldm(l, u, d);
+          mul(d, rv, uv);
+          mul(d, n, mv);
+          st3(FW, w, l, u, n);
+          m[u] = make_float4(mv[0], mv[1], mv[2], 0.f);
+          e0d = rv[0] * uv[0] + rv[1] * uv[1] + rv[2] * uv[2];
+          e1d = n[0] * uv[0] + n[1] * uv[1] + n[2] * uv[2];
+          e2d = unscaled2(rv, is);
+        }
+        dots(l, e0d, e1d, e2d);
+      }
+      if (t1 < ns) __syncthreads();
+    }
+  }
+  for (int k = 0; ok; ++k) {
+    const bool first = k == 0;
+    __syncthreads();
+    ok = exchange_wait<float, 3>(gx, nx, shw, pl.spc, ns, xs);
+    if (!ok) break;
+    exchange_total<3>(gx, nx++, xs, [&](const double(&t)[3]) {
+      if (first) {  // the stop test is relative to this residual
+        sc.done = 0;
+        sc.rz_old = 1.0;
+        sc.rr0 = t[2];
+        sc.tol2 = a.rtol * a.rtol * t[2];
+        sc.iters = 0;
+        sc.status = 0;
+        sc.alpha = sc.beta = 0.0;
+      }
+      cgcg_after(&sc, t[0], t[1], t[2], a.max_iters);
+      s_ab[0] = (float)sc.alpha;
+      s_ab[1] = (float)sc.beta;
+    });
+    // the scalars are made while the other warps start on n = A m, which does not need them
+    const bool pipe = k < a.pipe_iters;
+    const float4* mk = m + (size_t)(k & 1) * nv;
+    float4* mn = m + (size_t)((k + 1) & 1) * nv;
+    if (pipe) spmv(mk, 0, min(ns, pl.tile));
+    __syncthreads();
+    if (sc.done) break;
+    const float alpha = s_ab[0], beta = s_ab[1];
+    if (!pipe) {
+      // Chronopoulos-Gear: p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = M r; then w = A u
+      for (int l = tid; l < 32 * ns; l += HT) {
+        const int u = 32 * s0 + l;
+        if (u >= nv) continue;
+        float rv[3], wv[3], pv[3], ss[3], xv[3], d[6], uv[3];
+        ld3(FR, r, l, u, rv);
+        ld3(FW, w, l, u, wv);
+        ld3(FP, p, l, u, pv);
+        ld3(FS, sv, l, u, ss);
+        ld3(FX, x, l, u, xv);
+        ldm(l, u, d);
+        mul(d, rv, uv);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          pv[c] = uv[c] + beta * pv[c];
+          ss[c] = wv[c] + beta * ss[c];
+          xv[c] += alpha * pv[c];
+          rv[c] -= alpha * ss[c];
+        }
+        st3(FP, p, l, u, pv);
+        st3(FS, sv, l, u, ss);
+        st3(FX, x, l, u, xv);
+        st3(FR, r, l, u, rv);
+        mul(d, rv, uv);
+        mn[u] = make_float4(uv[0], uv[1], uv[2], 0.f);
+      }
+      ok = exchange_barrier(gx, nx++, xs);
+      if (!ok) break;
+    }
+    for (int t0 = 0; t0 < ns; t0 += pl.tile) {
+      const int t1 = min(ns, t0 + pl.tile);
+      if (!pipe || t0 > 0) {
+        spmv(pipe ? mk : mn, t0, t1);
+        __syncthreads();
+      }
+      for (int l = 32 * t0 + tid; l < 32 * t1; l += HT) {
+        const int u = 32 * s0 + l;
+        float e0d = 0.f, e1d = 0.f, e2d = 0.f;
+        if (u < nv) {
+          float n[3], rv[3], wv[3], d[6], uv[3], is[3];
+          product(l, t0, n[0], n[1], n[2]);
+          ld3(FR, r, l, u, rv);
+          ldm(l, u, d);
+          if (pipe) {
+            float v[3], q[3];
+            ld3(FW, w, l, u, wv);
+            ld3(FZ, z, l, u, v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) n[c] += beta * v[c];  // z
+            st3(FZ, z, l, u, n);
+            ld3(FS, sv, l, u, v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              v[c] = wv[c] + beta * v[c];  // s
+              wv[c] -= alpha * n[c];
+            }
+            st3(FS, sv, l, u, v);
+            st3(FW, w, l, u, wv);
+            mul(d, rv, uv);
+            ld3(FP, p, l, u, q);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+              q[c] = uv[c] + beta * q[c];  // p
+              rv[c] -= alpha * v[c];
+            }
+            st3(FP, p, l, u, q);
+            st3(FR, r, l, u, rv);
+            ld3(FX, x, l, u, v);
+#pragma unroll
+            for (int c = 0; c < 3; ++c) v[c] += alpha * q[c];
+            st3(FX, x, l, u, v);
+            mul(d, wv, v);
+            mn[u] = make_float4(v[0], v[1], v[2], 0.f);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 3; ++c) wv[c] = n[c];
+            st3(FW, w, l, u, wv);
+          }
+          mul(d, rv, uv);
+          ld3(FI, H.iscale, l, u, is);
+          e0d = rv[0] * uv[0] + rv[1] * uv[1] + rv[2] * uv[2];
+          e1d = wv[0] * uv[0] + wv[1] * uv[1] + wv[2] * uv[2];
+          e2d = unscaled2(rv, is);
+        }
+        dots(l, e0d, e1d, e2d);
+      }
+      if (t1 < ns) __syncthreads();
+    }
+  }
+  // x = S x~ (own rows)
+  for (int l = tid; l < 32 * ns; l += HT) {
+    const int u = 32 * s0 + l;
+    if (u >= nv) continue;
+    float xv[3];
+    ld3(FX, x, l, u, xv);
+    const float4 s4 = H.scale[u];
+    x[u] = make_float4(xv[0] * s4.x, xv[1] * s4.y, xv[2] * s4.z, 0.f);
+  }
+  if (ok && blockIdx.x == 0 && tid == 0) {
+    DevScalars* o = red.sc;
+    o->rz = sc.rz;
+    o->rz_old = sc.rz_old;
+    o->pq = sc.pq;
+    o->rr = sc.rr;
+    o->rr0 = sc.rr0;
+    o->tol2 = sc.tol2;
+    o->alpha = sc.alpha;
+    o->beta = sc.beta;
+    o->iters = sc.iters;
+    o->done = sc.done;
+    o->status = sc.status;
+  }
+  // the check on the FP32 values: every block's x is final after the exchange; the slices' dots go to the row
+  // state's memory (no longer needed) in FP64
+  if (ok && a.check) ok = exchange_barrier(gx, nx++, xs);
+  if (ok && a.check) {
+    double q[4] = {0, 0, 0, 0};
+    for (int t0 = 0; t0 < ns; t0 += pl.tile) {
+      const int t1 = min(ns, t0 + pl.tile), nu = (t1 - t0) << lt;
+      for (int i = warp; i < nu; i += HT / 32) {
+        const int ls = t0 + (i >> lt), part = i & (T - 1);
+        float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+        if (32 * (s0 + ls) + lane < nv) sym_unit<float>(a.A32, a.vals32, s0 + ls, lane, part, T, x, a0, a1, a2);
+        float* o = pb + (size_t)3 * part * PR + 32 * (ls - t0) + lane;
+        o[0] = a0;
+        o[PR] = a1;
+        o[2 * PR] = a2;
+      }
+      __syncthreads();
+      for (int l = 32 * t0 + tid; l < 32 * t1; l += HT) {
+        const int u = 32 * s0 + l;
+        if (u >= nv) continue;
+        float n0, n1, n2;
+        product(l, t0, n0, n1, n2);
+        const float4 dv = x[u];
+        const double g0 = a.b[3 * (size_t)u], g1 = a.b[3 * (size_t)u + 1], g2 = a.b[3 * (size_t)u + 2];
+        const double x0 = dv.x, x1 = dv.y, x2 = dv.z;
+        q[0] += g0 * x0 + g1 * x1 + g2 * x2;
+        q[1] += x0 * x0 + x1 * x1 + x2 * x2;
+        const double q0 = sg * g0 - (double)n0, q1 = sg * g1 - (double)n1, q2 = sg * g2 - (double)n2;
+        q[2] += q0 * q0 + q1 * q1 + q2 * q2;
+        q[3] += g0 * g0 + g1 * g1 + g2 * g2;
+      }
+      __syncthreads();
+    }
+    // per-warp sums to shared memory (the unit partials' space: at least 3 * 32 * 4 * 8 values)
+    double* shq = reinterpret_cast<double*>(pb);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const double t = warp_add(q[c]);
+      if (lane == 0) shq[32 * c + warp] = t;
+    }
+    ok = exchange<double, 4>(gx, nx++, shq, 32, HT / 32, xs, [&](const double(&t)[4]) {
+      if (blockIdx.x == 0) {
+        red.sc->gd = t[0];
+        red.sc->dnorm2 = t[1];
+        red.sc->true_rr = t[2];
+        red.sc->true_bb = t[3];
+      }
+    });
+  }
+  if (!ok && tid == 0) atomicExch(&red.sc->wait_failed, 1);
+}
+
+constexpr size_t kSmemReserve = 8 * 1024;  // static shared memory and the 1 KB a block costs
+
+size_t half_smem(const HalfPlan& p) {
+  const size_t f = (size_t)kHalfState * 32 * p.res + (size_t)3 * p.T * 32 * p.tile + 4 * (size_t)p.spc;
+  return (size_t)16 * p.cache_entries + 4 * f + 4 * ((size_t)p.spc + 1) + 6 * (size_t)p.cache_entries + 64;
+}
+
+}  // namespace
+
+size_t resident_sync_bytes() { return 128 + (size_t)2 * 4 * kMaxBlocks * sizeof(double); }
+
+// first slice of block c's part of nsl slices over g blocks
+static int part_begin(int c, int nsl, int g) { return (int)((long long)c * nsl / g); }
+
+static GridExchange grid_exchange(const ResidentSync& rs, cudaStream_t st) {
+  SSIM_CUDA(cudaMemsetAsync(rs.mem, 0, sizeof(unsigned long long), st));
+  return GridExchange{reinterpret_cast<unsigned long long*>(rs.mem), reinterpret_cast<double*>(rs.mem + 128),
+                      (unsigned int)rs.extra, rs.spin_limit > 0 ? rs.spin_limit : (1LL << 21)};
+}
+
+// Layout of a resident solve on the FP16 copy (host arithmetic only; off: the copy's slice offsets).
+//  T: 4 warps a slice (a 15-entry slice is four entries a unit: all of a unit's loads in flight at once), 8 where a
+//  block has fewer than 8 slices (small systems: fewer dependent rounds).
+//  The vectors of all rows stay on chip while they and one pass over the block's slices fit (about 1,440 rows a
+//  block, 219,000 rows on 152 SMs); beyond, passes of 32 slices and the rows that fit.  The matrix entries too
+//  where the block's part of them fits (about 70,000 rows): an iteration then reads nothing but the gathered
+//  vector from L2.
+static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, int max_blocks) {
+  HalfPlan p{};
+  const int nsl = div_up(nv, 32);
+  p.grid = std::max(1, std::min(std::min(nsm, kMaxBlocks), nsl));
+  if (max_blocks > 0) p.grid = std::min(p.grid, max_blocks);
+  for (int c = 0; c < p.grid; ++c) p.spc = std::max(p.spc, part_begin(c + 1, nsl, p.grid) - part_begin(c, nsl, p.grid));
+  p.T = 4;
+  p.res = p.tile = p.spc;
+  if (half_smem(p) > smem_max) {
+    p.tile = 32;
+    p.res = 0;
+    const size_t base = half_smem(p);
+    const size_t row = (size_t)4 * kHalfState * 32;
+    p.res = base < smem_max ? (int)std::min<size_t>((size_t)p.spc, (smem_max - base) / row) : 0;
+    if (base > smem_max) p.grid = 0;
+    return p;
+  }
+  HalfPlan q = p;
+  for (int c = 0; c < p.grid; ++c)
+    q.cache_entries = std::max(q.cache_entries, off[part_begin(c + 1, nsl, p.grid)] - off[part_begin(c, nsl, p.grid)]);
+  q.cached = 1;
+  if (p.spc < 8) q.T = 8;
+  return half_smem(q) <= smem_max ? q : p;
+}
+
+bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, const float4* dinv16, float4* x, float4* r,
+                              float4* z, float4* p, float4* sv, float4* w, float4* m, const HalfSolveArgs& pa,
+                              const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st) {
+  if (H.nv <= 0) return true;
+  int dev = 0, coop = 0, nsm = 0, smax = 0, per_sm = 0;
+  SSIM_CUDA(cudaGetDevice(&dev));
+  SSIM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+  SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  SSIM_CUDA(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  if (!coop) return false;
+  HalfPlan pl = half_plan(H.nv, off_host, nsm, (size_t)smax - kSmemReserve, max_blocks);
+  if (pl.grid < 1) return false;
+  pl.smem = half_smem(pl);
+  const void* fn = !pl.cached   ? (const void*)resident_half_kernel<false, 4>
+                   : pl.T == 4 ? (const void*)resident_half_kernel<true, 4>
+                               : (const void*)resident_half_kernel<true, 8>;
+  SSIM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
+  SSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, HT, pl.smem));
+  if (per_sm < 1) return false;
+  GridExchange gx = grid_exchange(rs, st);
+  HalfMatrix h = H;
+  HalfSolveArgs ha = pa;
+  Reduce rd = red;
+  void* args[] = {(void*)&h, (void*)&dinv16, (void*)&x,  (void*)&r,  (void*)&z,  (void*)&p,  (void*)&sv,
+                  (void*)&w, (void*)&m,      (void*)&ha, (void*)&pl, (void*)&rd, (void*)&gx};
+  SSIM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(pl.grid), dim3(HT), args, pl.smem, st));
+  after_launch("pcg_half_resident");
+  return true;
+}
+
+}  // namespace ssim_gb

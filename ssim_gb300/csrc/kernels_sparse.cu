@@ -3,15 +3,13 @@
 
 #include <cuda_fp16.h>
 
-#include "kernels.cuh"
+#include "pcg_common.cuh"
 
 namespace ssim_gb {
 namespace {
 
 constexpr int SB = 256;  // block of the slot / row / dof kernels (a multiple of the 32-row slice)
 
-
-__device__ __forceinline__ size_t sell_base(int q) { return (size_t)9 * (size_t)(q & ~31) + (size_t)(q & 31); }
 
 // Assembly (update_hessian, time_step.hpp:631-657): each upper slot (one 3x3 vertex-pair block of the
 // symmetric matrix) adds its precomputed list of element blocks (global_composer.hpp:103-119 builds the
@@ -409,30 +407,6 @@ __device__ __forceinline__ void pcg_update_row(int nv, const V4<S>* p, const V4<
   part[1] = ru.x * ru.x + ru.y * ru.y + ru.z * ru.z;
 }
 
-// the scalar epilogues shared by the two-launch and the persistent PCG
-__device__ __forceinline__ void pcg_after_pq(DevScalars* sc, double pq) {
-  sc->pq = pq;
-  sc->alpha = sc->rz / pq;
-  if (!(pq > 0.0)) {  // breakdown: not SPD along p (or non-finite)
-    sc->done = 1;
-    sc->status = 1;
-  }
-}
-
-__device__ __forceinline__ void pcg_after_rz(DevScalars* sc, double rz, double rr, int max_iters) {
-  sc->rz_old = sc->rz;
-  sc->rz = rz;
-  sc->beta = rz / sc->rz_old;
-  sc->rr = rr;
-  sc->iters += 1;
-  if (!isfinite(rr)) {
-    sc->done = 1;
-    sc->status = 2;
-  } else if (rr <= sc->tol2 || sc->iters >= max_iters || rz == 0.0) {
-    sc->done = 1;
-  }
-}
-
 template <typename S, bool KRON>
 __global__ void __launch_bounds__(SB)
     pcg_spmv_kernel(SellMatrix A, const S* __restrict__ vals, const V4<S>* __restrict__ z,
@@ -631,42 +605,6 @@ __device__ __forceinline__ void cgcg_update_row(int nv, bool first, S alpha, S b
   r[u] = ru;
   z[u] = mk4<S>(d0.x * ru.x + d0.y * ru.y + d0.z * ru.z, d1.x * ru.x + d1.y * ru.y + d1.z * ru.z,
                 d2.x * ru.x + d2.y * ru.y + d2.z * ru.z);
-}
-
-// scalar epilogue after phase A (one thread): stop tests on the residual of the current x, then the
-// step lengths.  iters counts the x updates; rr is |r|^2 of the current x.
-__device__ __forceinline__ void cgcg_after(DevScalars* sc, double g, double d, double rr, int max_iters) {
-  sc->rr = rr;
-  if (!isfinite(rr)) {
-    sc->done = 1;
-    sc->status = 2;
-    return;
-  }
-  if (rr <= sc->tol2 || g == 0.0 || sc->iters >= max_iters) {
-    sc->done = 1;
-    return;
-  }
-  // beta = g / g_old and den = d - beta g / alpha_old from the reciprocals kept by the previous step, so
-  // only two independent divisions remain on this serial path (FP64 divisions are slow on GB300)
-  double beta = 0.0, den = d;
-  if (sc->iters > 0) {
-    beta = g * sc->inv_rz;
-    den = d - beta * g * sc->inv_alpha;
-  }
-  if (!(den > 0.0)) {  // breakdown: not SPD along p (or non-finite)
-    sc->done = 1;
-    sc->status = 1;
-    return;
-  }
-  const double inv_den = 1.0 / den, inv_g = 1.0 / g;
-  sc->rz_old = sc->rz;
-  sc->rz = g;
-  sc->pq = den;
-  sc->beta = beta;
-  sc->alpha = g * inv_den;
-  sc->inv_rz = inv_g;
-  sc->inv_alpha = den * inv_g;
-  sc->iters += 1;
 }
 
 template <typename S, bool KRON>
@@ -966,13 +904,6 @@ __global__ void __launch_bounds__(SB, 5)
 // it reaches the tolerance of long, ill-conditioned solves), so after pipe_iters iterations the solve
 // continues as Chronopoulos-Gear PCG from the same state (x, r, p, s, w; u = M r), whose SpMV recomputes
 // w = A u every iteration.
-template <typename S>
-__device__ __forceinline__ V4<S> block_jacobi(const V4<S>* __restrict__ dinv, int u, S a0, S a1, S a2) {
-  const V4<S> d0 = dinv[3 * u], d1 = dinv[3 * u + 1], d2 = dinv[3 * u + 2];
-  return mk4<S>(d0.x * a0 + d0.y * a1 + d0.z * a2, d1.x * a0 + d1.y * a1 + d1.z * a2,
-                d2.x * a0 + d2.y * a1 + d2.z * a2);
-}
-
 template <typename S, bool KRON>
 __device__ __forceinline__ void pipe_first_row(const SellMatrix& A, const S* __restrict__ vals,
                                                const V4<S>* __restrict__ dinv, const V4<S>* u0, const V4<S>* r,
@@ -1108,219 +1039,6 @@ __global__ void __launch_bounds__(SB, sizeof(S) == 4 ? 5 : 4)
     }
   }
   // a barrier wait gave up: flag it (the host clears the flag before the launch) and leave
-  if (!ok && threadIdx.x == 0) atomicExch(&sc->wait_failed, 1);
-}
-
-// Pipelined PCG (pipe_persistent_kernel) on the FP16 copy, in its scaled space: the SpMV of m = M w reads the
-// full FP16 entries, the third dot is (r, r) of the unscaled residual, and every block unscales its own rows
-// of x after the last iteration.  After pipe_iters iterations it continues as Chronopoulos-Gear.
-__device__ __forceinline__ void pipe_half_row(const HalfMatrix& H, const float4* __restrict__ dinv, bool first,
-                                              float alpha, float beta, const float4* mk, float4* mn, float4* x,
-                                              float4* r, float4* z, float4* p, float4* sv, float4* w, int u,
-                                              int (*sidx)[32], float (&part)[3]) {
-  part[0] = part[1] = part[2] = 0.f;
-  if (u >= H.nv) return;
-  float n0, n1, n2;
-  half_row_product(H, u, mk, sidx, n0, n1, n2);
-  float4 ru = r[u], wu = w[u];
-  const float4 uu = block_jacobi<float>(dinv, u, ru.x, ru.y, ru.z);
-  float4 zu = make_float4(n0, n1, n2, 0.f), su = wu, pu = uu;
-  if (!first) {
-    const float4 zo = z[u], so = sv[u], po = p[u];
-    zu = make_float4(n0 + beta * zo.x, n1 + beta * zo.y, n2 + beta * zo.z, 0.f);
-    su = make_float4(wu.x + beta * so.x, wu.y + beta * so.y, wu.z + beta * so.z, 0.f);
-    pu = make_float4(uu.x + beta * po.x, uu.y + beta * po.y, uu.z + beta * po.z, 0.f);
-  }
-  float4 xu = x[u];
-  xu.x += alpha * pu.x;
-  xu.y += alpha * pu.y;
-  xu.z += alpha * pu.z;
-  ru.x -= alpha * su.x;
-  ru.y -= alpha * su.y;
-  ru.z -= alpha * su.z;
-  wu.x -= alpha * zu.x;
-  wu.y -= alpha * zu.y;
-  wu.z -= alpha * zu.z;
-  z[u] = zu;
-  sv[u] = su;
-  p[u] = pu;
-  x[u] = xu;
-  r[u] = ru;
-  w[u] = wu;
-  mn[u] = block_jacobi<float>(dinv, u, wu.x, wu.y, wu.z);
-  const float4 un = block_jacobi<float>(dinv, u, ru.x, ru.y, ru.z);
-  const float4 is = H.iscale[u];
-  const float t0 = ru.x * is.x, t1 = ru.y * is.y, t2 = ru.z * is.z;
-  part[0] = ru.x * un.x + ru.y * un.y + ru.z * un.z;
-  part[1] = wu.x * un.x + wu.y * un.y + wu.z * un.z;
-  part[2] = t0 * t0 + t1 * t1 + t2 * t2;
-}
-
-// The whole solve on the copy in one launch: the set-up (x = 0, r~ = S (sign b), u0 = M r~; a plain
-// barrier orders u0 before the prologue's SpMV), the pipelined iterations (Chronopoulos-Gear after
-// pipe_iters), x unscaled, and, when a.check is set, the solve's check on the FP32 symmetric store: g . x,
-// |x|^2, |sign b - K x|^2 and |b|^2 (b = the Newton gradient g, sign = -1) into sc->gd, dnorm2, true_rr,
-// true_bb.  Barriers are numbered by their own counters (the plain ones, the reducing ones) in the order
-// every block meets them.
-__global__ void __launch_bounds__(SB, 5)
-    pipe_half_kernel(HalfMatrix H, const float4* __restrict__ dinv, float4* x, float4* r, float4* z, float4* p,
-                     float4* sv, float4* w, float4* m, HalfSolveArgs a, Reduce red, GridSync gs) {
-  __shared__ double shred[SB / 32][3];
-  __shared__ double shred4[SB / 32][4];
-  __shared__ int sidx[SB / 32][ST_K][32];
-  __shared__ double s_alpha, s_beta;
-  __shared__ int s_done;
-  DevScalars* sc = red.sc;
-  const int nv = H.nv;
-  const int nvb = (nv + SB - 1) / SB;
-  double* part = red.partials;
-  double* gsum = red.partials + 3 * (size_t)nvb;
-  double* gsum4 = red.partials + 4 * (size_t)nvb;
-  auto publish = [&](int vb, float (&pr)[3]) {
-    double bs[3];
-    block_sum_s<3, SB, float>(pr, bs, shred);
-    if (threadIdx.x == 0) {
-      part[3 * vb] = bs[0];
-      part[3 * vb + 1] = bs[1];
-      part[3 * vb + 2] = bs[2];
-    }
-    __syncthreads();
-  };
-  const double sg = a.negate ? -1.0 : 1.0;
-  unsigned long long npb = 0, nrb = 0;
-  // set-up (pcg_setup_half_kernel's per-row work)
-  for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-    const int u = vb * SB + threadIdx.x;
-    if (u < nv) {
-      const float r0 = (float)(sg * a.b[u * 3 + 0]), r1 = (float)(sg * a.b[u * 3 + 1]),
-                  r2 = (float)(sg * a.b[u * 3 + 2]);
-      const float4 s4 = H.scale[u];
-      const float t0 = r0 * s4.x, t1 = r1 * s4.y, t2 = r2 * s4.z;
-      x[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-      r[u] = make_float4(t0, t1, t2, 0.f);
-      z[u] = block_jacobi<float>(dinv, u, t0, t1, t2);
-      p[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-  }
-  bool ok = plain_barrier(gs, npb++);
-  // prologue: w = A u0, m_0 = M w, the first dots
-  if (ok) {
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      const int u = vb * SB + threadIdx.x;
-      float pr[3] = {0.f, 0.f, 0.f};
-      if (u < nv) {
-        float a0, a1, a2;
-        half_row_product(H, u, z, sidx[threadIdx.x >> 5], a0, a1, a2);
-        w[u] = make_float4(a0, a1, a2, 0.f);
-        m[u] = block_jacobi<float>(dinv, u, a0, a1, a2);
-        const float4 uu = z[u], ru = r[u], is = H.iscale[u];
-        const float t0 = ru.x * is.x, t1 = ru.y * is.y, t2 = ru.z * is.z;
-        pr[0] = ru.x * uu.x + ru.y * uu.y + ru.z * uu.z;
-        pr[1] = a0 * uu.x + a1 * uu.y + a2 * uu.z;
-        pr[2] = t0 * t0 + t1 * t1 + t2 * t2;
-      }
-      publish(vb, pr);
-    }
-  }
-  for (int k = 0; ok; ++k) {
-    const bool first = k == 0;
-    ok = reduce_barrier<3>(gs, nrb++, part, gsum, nvb, [&](const double (&t)[3]) {
-      if (first) {  // the set-up's scalars: the stop test is relative to this residual
-        sc->done = 0;
-        sc->rz_old = 1.0;
-        sc->rr0 = t[2];
-        sc->tol2 = a.rtol * a.rtol * t[2];
-        sc->iters = 0;
-        sc->status = 0;
-      }
-      cgcg_after(sc, t[0], t[1], t[2], a.max_iters);
-    });
-    if (!ok) break;
-    if (threadIdx.x == 0) {
-      s_done = __ldcg(&sc->done);
-      s_alpha = __ldcg(&sc->alpha);
-      s_beta = __ldcg(&sc->beta);
-    }
-    __syncthreads();
-    if (s_done) break;
-    const float alpha = (float)s_alpha, beta = (float)s_beta;
-    if (k < a.pipe_iters) {
-      const float4* mk = m + (size_t)(k & 1) * nv;
-      float4* mn = m + (size_t)((k + 1) & 1) * nv;
-      for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-        float pr[3];
-        pipe_half_row(H, dinv, k == 0, alpha, beta, mk, mn, x, r, z, p, sv, w, vb * SB + threadIdx.x,
-                      sidx[threadIdx.x >> 5], pr);
-        publish(vb, pr);
-      }
-      continue;
-    }
-    // Chronopoulos-Gear from here on (as pipe_persistent_kernel)
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      const int u = vb * SB + threadIdx.x;
-      if (k == a.pipe_iters && u < nv) {
-        const float4 ru = r[u];
-        z[u] = block_jacobi<float>(dinv, u, ru.x, ru.y, ru.z);
-      }
-      cgcg_update_row<float>(nv, k == 0, alpha, beta, dinv, z, w, p, sv, x, r, u);
-    }
-    ok = plain_barrier(gs, npb++);
-    if (!ok) break;
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      const int u = vb * SB + threadIdx.x;
-      float pr[3] = {0.f, 0.f, 0.f};
-      if (u < nv) {
-        float a0, a1, a2;
-        half_row_product(H, u, z, sidx[threadIdx.x >> 5], a0, a1, a2);
-        w[u] = make_float4(a0, a1, a2, 0.f);
-        const float4 uu = z[u], ru = r[u], is = H.iscale[u];
-        const float t0 = ru.x * is.x, t1 = ru.y * is.y, t2 = ru.z * is.z;
-        pr[0] = ru.x * uu.x + ru.y * uu.y + ru.z * uu.z;
-        pr[1] = a0 * uu.x + a1 * uu.y + a2 * uu.z;
-        pr[2] = t0 * t0 + t1 * t1 + t2 * t2;
-      }
-      publish(vb, pr);
-    }
-  }
-  // x = S x~ (rows of this block only)
-  for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-    const int u = vb * SB + threadIdx.x;
-    if (u < nv) {
-      const float4 xv = x[u], s4 = H.scale[u];
-      x[u] = make_float4(xv.x * s4.x, xv.y * s4.y, xv.z * s4.z, 0.f);
-    }
-  }
-  // the check on the FP32 values: every block's x is final after a plain barrier
-  if (ok && a.check) ok = plain_barrier(gs, npb++);
-  if (ok && a.check) {
-    for (int vb = blockIdx.x; vb < nvb; vb += gridDim.x) {
-      const int u = vb * SB + threadIdx.x;
-      double pr[4] = {0, 0, 0, 0};
-      if (u < nv) {
-        float a0, a1, a2;
-        row_product_t<float, true>(a.A32, a.vals32, u, x, nullptr, 0.f, sidx[threadIdx.x >> 5], a0, a1, a2);
-        const float4 dv = x[u];
-        const double g0 = a.b[u * 3 + 0], g1 = a.b[u * 3 + 1], g2 = a.b[u * 3 + 2];
-        pr[0] = g0 * (double)dv.x + g1 * (double)dv.y + g2 * (double)dv.z;
-        pr[1] = (double)dv.x * dv.x + (double)dv.y * dv.y + (double)dv.z * dv.z;
-        const double q0 = sg * g0 - (double)a0, q1 = sg * g1 - (double)a1, q2 = sg * g2 - (double)a2;
-        pr[2] = q0 * q0 + q1 * q1 + q2 * q2;
-        pr[3] = g0 * g0 + g1 * g1 + g2 * g2;
-      }
-      block_sum<4, SB>(pr, shred4);
-      if (threadIdx.x == 0) {
-#pragma unroll
-        for (int c = 0; c < 4; ++c) part[4 * vb + c] = pr[c];
-      }
-      __syncthreads();
-    }
-    ok = reduce_barrier<4>(gs, nrb++, part, gsum4, nvb, [&](const double (&t)[4]) {
-      sc->gd = t[0];
-      sc->dnorm2 = t[1];
-      sc->true_rr = t[2];
-      sc->true_bb = t[3];
-    });
-  }
   if (!ok && threadIdx.x == 0) atomicExch(&sc->wait_failed, 1);
 }
 
@@ -1834,15 +1552,13 @@ void launch_half_spmv(const HalfMatrix& H, const float4* x, float4* xs, float4* 
 
 bool launch_pcg_half(const HalfMatrix& H, const float4* dinv16, float4* x, float4* r, float4* z, float4* p0,
                      float4* p1, float4* q, int max_iters, const Reduce& red, unsigned long long* gsync,
-                     long long spin_limit, int extra, int max_blocks, cudaStream_t st, float4* pm,
-                     const HalfSolveArgs* pa) {
+                     long long spin_limit, int extra, int max_blocks, cudaStream_t st) {
   int dev = 0, coop = 0, nsm = 0, per_sm = 0;
   SSIM_CUDA(cudaGetDevice(&dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   if (!coop) return false;
   SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const bool pipe = pm != nullptr && pa != nullptr;
-  const void* fn = pipe ? (const void*)pipe_half_kernel : (const void*)cgcg_half_kernel;
+  const void* fn = (const void*)cgcg_half_kernel;
   SSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, SB, 0));
   if (per_sm < 1) return false;
   int grid = std::min(div_up(H.nv, SB), per_sm * nsm);
@@ -1863,12 +1579,7 @@ bool launch_pcg_half(const HalfMatrix& H, const float4* dinv16, float4* x, float
   Reduce rd = red;
   void* args[] = {(void*)&h,  (void*)&dinv16, (void*)&x, (void*)&r,         (void*)&z,  (void*)&p0,
                   (void*)&p1, (void*)&q,      (void*)&max_iters, (void*)&rd, (void*)&gs};
-  // pipelined: p = p0, s = p1, w = q, then the two m vectors
-  HalfSolveArgs ha{};
-  if (pa) ha = *pa;
-  void* pargs[] = {(void*)&h, (void*)&dinv16, (void*)&x,  (void*)&r,  (void*)&z, (void*)&p0,
-                   (void*)&p1, (void*)&q,     (void*)&pm, (void*)&ha, (void*)&rd, (void*)&gs};
-  SSIM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SB), pipe ? pargs : args, 0, st));
+  SSIM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(SB), args, 0, st));
   after_launch("pcg_half");
   return true;
 }

@@ -150,6 +150,7 @@ struct TimeStep {
   // FP16 copy of the scaled system matrix for the mixed Newton's loose PCG solves (kernels.cuh HalfMatrix):
   // pattern built on first use, values made from the FP32 assembly before the first solve that reads them
   DBuf<int32_t> h16off, h16col, h16src;
+  std::vector<int32_t> h16off_h;
   DBuf<uint4> h16v8;
   DBuf<uint16_t> h16v1;
   DBuf<float4> h16scale, h16iscale, h16dinv;
@@ -174,6 +175,8 @@ struct TimeStep {
   DBuf<double> partials;
   DBuf<unsigned int> counter;
   DBuf<unsigned long long> gsync;  // grid-barrier state of the persistent PCG (counters, release, groups)
+  DBuf<unsigned char> rsync;       // grid exchange of the resident PCG
+  ResidentSync resident_sync() const { return ResidentSync{rsync.p, params.pcg_barrier_extra, params.pcg_spin_limit}; }
   DBuf<DevScalars> sc;
   DevScalars* hsc = nullptr;  // pinned
   DBuf<double> gprev, dscal;   // previous gradient (L-BFGS), device scalars of vdot
@@ -374,6 +377,13 @@ struct TimeStep {
     SSIM_CUDA(cudaStreamSynchronize(stream));
   }
 
+  // after sync_scalars(): a wait of the last solve's kernel that ran out (the flag is cleared for the next one)
+  void check_wait() {
+    if (!hsc->wait_failed) return;
+    SSIM_CUDA(cudaMemsetAsync(&sc.p->wait_failed, 0, sizeof(int32_t), stream));
+    throw device_timeout("a grid-barrier wait of the persistent PCG kernel gave up");
+  }
+
   // ------------------------------------------------------------------ construction
   void create(const double* Xh, int nv_, const int32_t* cells_h, int nt_, double dt_, double E_, double nu_,
               double rho_) {
@@ -546,6 +556,7 @@ struct TimeStep {
     counter.zero(stream);
     gsync.alloc(grid_sync_words(nv));
     gsync.zero(stream);
+    rsync.alloc(resident_sync_bytes());
     const size_t maxgrid = (size_t)std::max(div_up(nt, 64), div_up(std::max(3 * nv, topo.nslots), 256)) + 1;
     partials.alloc(maxgrid * 4);
     dX.upload(X, stream);
@@ -592,6 +603,7 @@ struct TimeStep {
     h16_ok = build_full_sell(topo, off, col, src);
     if (!h16_ok) return false;
     nfs = (long long)col.size();
+    h16off_h = off;
     h16off.upload(off, stream);
     h16col.upload(col, stream);
     h16src.upload(src, stream);
@@ -1004,14 +1016,16 @@ struct TimeStep {
       launch_pcg_setup_half(H, b, h16dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, eta, max_iters, negate, red(), stream);
     }
     if (profiling) SSIM_CUDA(cudaEventRecord(ev[0], stream));
-    const bool ran = launch_pcg_half(H, h16dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, s.p1.p, s.q.p, max_iters, red(),
-                                     gsync.p, params.pcg_spin_limit, params.pcg_barrier_extra, params.pcg_max_blocks,
-                                     stream, pipe ? s.pm.p : nullptr, pipe ? &ha : nullptr);
+    const bool ran =
+        pipe ? launch_pcg_half_resident(H, h16off_h.data(), h16dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, s.p1.p, s.q.p, s.pm.p,
+                                        ha, red(), resident_sync(), params.pcg_max_blocks, stream)
+             : launch_pcg_half(H, h16dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, s.p1.p, s.q.p, max_iters, red(), gsync.p,
+                               params.pcg_spin_limit, params.pcg_barrier_extra, params.pcg_max_blocks, stream);
     if (!ran) return false;
     half_checked = pipe && ha.check;
     if (profiling) SSIM_CUDA(cudaEventRecord(ev[1], stream));
     sync_scalars();
-    if (hsc->wait_failed) throw device_timeout("a grid-barrier wait of the persistent PCG kernel gave up");
+    check_wait();
     if (profiling) {
       float ms = 0;
       SSIM_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
@@ -1057,7 +1071,7 @@ struct TimeStep {
       if (ran) {
         if (prof) SSIM_CUDA(cudaEventRecord(ev[1], stream));
         sync_scalars();
-        if (hsc->wait_failed) throw device_timeout("a grid-barrier wait of the persistent PCG kernel gave up");
+        check_wait();
         if (prof) {
           float ms = 0;
           SSIM_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));

@@ -1,0 +1,92 @@
+"""The resident PCG (kernels_pcg.cu): one block per SM, the rows' vectors on chip, one grid exchange a reduction.
+
+Meshes and grid caps are chosen for the layouts' edges: a single slice and a row more, ragged last slices, blocks with
+fewer than and at least 8 slices (the two unit widths), blocks whose matrix entries fit on chip, blocks whose vectors
+fit but not their entries, and blocks that keep only some rows' vectors on chip (few blocks over many rows).
+
+FP16 copy (mixed precision, loose solves): with the oracle's FP64 matrix K the true residual |b - K x| / |b| is within
+the requested 5e-2 plus the copy's rounding (5e-3), and the iterations within 10% + 2 of the two-launch PCG's on the
+FP32 values.
+"""
+import numpy as np
+import pytest
+
+import ssim_gb300 as g
+from ssim_gb300 import mesh
+
+pytestmark = pytest.mark.gpu
+
+# hexes a side, grid cap (0: one block per SM)
+LAYOUTS = [
+    ((1, 1, 1), 0),     # 8 rows: one slice, mostly padding
+    ((3, 3, 1), 0),     # 32 rows: exactly one slice
+    ((10, 2, 1), 0),    # 66 rows: two slices and two rows
+    ((13, 9, 7), 0),    # 1,120 rows: one slice per block
+    ((13, 9, 7), 3),    # 12 slices a block, entries on chip
+    ((13, 9, 7), 2),    # 18 slices a block, entries in global memory
+    ((21, 12, 9), 1),   # 90 slices in one block: vectors only partly on chip, three passes
+    ((21, 12, 9), 2),   # 45 slices a block: near the limit of full residency
+]
+
+
+def _pair(hexes, **params):
+    from oracle import pyoracle
+
+    X, T = mesh.kuhn_box(hexes, tuple(0.1 * k for k in hexes))
+    X = mesh.jitter_interior(X, 0.008, 31)
+    E = 10.0 ** mesh.uniform(32, T.shape[0], 4.0, 6.0)
+    fixed = np.where(X[:, 0] == 0.0)[0]
+    ts = g.TimeStep(X, T, 1e-2, 1e5, 0.45, 1000.0)
+    ts.set_precision(params.pop("precision"))
+    ts.set_params(g.default_params(precond=2, cg_max_iters=20000, **params))
+    ot = pyoracle.OracleTimeStep(X, T, 1e-2, 1e5, 0.45, 1000.0)
+    u = np.random.default_rng(33).uniform(-1, 1, X.shape) * 0.01
+    for t in (ts, ot):
+        t.set_material(E, None)
+        getattr(t, "mark_dirichlet_batched", getattr(t, "mark_dirichlet", None))(
+            fixed, *([np.zeros((fixed.size, 3))] if t is ts else []))
+    ts.reset("newton")
+    ot.reset()
+    for t in (ts, ot):
+        t.set("next_deform", u)
+        t.update_hessian(False, True, True)
+    return ts, ot, np.random.default_rng(34).normal(size=X.shape)
+
+
+@pytest.mark.parametrize("hexes,blocks", LAYOUTS)
+@pytest.mark.parametrize("pipe_iters", [80, 3])
+def test_half_solve_true_residual(hexes, blocks, pipe_iters):
+    """pipe_iters = 3 makes every solve continue as Chronopoulos-Gear after three iterations."""
+    ts, ot, b = _pair(hexes, precision="mixed", pcg_max_blocks=blocks, pcg_pipe_iters=pipe_iters)
+    nb = np.linalg.norm(b)
+    x, it, rr = ts.pcg(b, rtol=5e-2)
+    assert rr <= 5e-2
+    true = np.linalg.norm(b.reshape(-1) - ot.spmv(x)) / nb
+    assert true <= 5e-2 + 5e-3, true
+    ts.set_params(pcg_persistent=0, pcg_half_matrix=0)
+    _, it0, _ = ts.pcg(b, rtol=5e-2)
+    assert abs(it - it0) <= 0.1 * it0 + 2, (it, it0)
+
+
+def test_half_solve_is_deterministic_and_caps_iterations():
+    ts, _, b = _pair((13, 9, 7), precision="mixed")
+    x0, it0, rr0 = ts.pcg(b, rtol=5e-2)
+    x1, it1, rr1 = ts.pcg(b, rtol=5e-2)
+    assert it0 == it1 and rr0 == rr1 and np.array_equal(x0, x1)
+    _, it, rr = ts.pcg(b, rtol=1e-2, max_iters=4)
+    assert it == 4 and rr > 1e-2
+    z, it, rr = ts.pcg(np.zeros_like(b), rtol=5e-2)
+    assert it == 0 and not z.any()
+
+
+def test_half_solve_wait_gives_up():
+    """A wait for an arrival that never comes ends after pcg_spin_limit polls with DeviceTimeout; the next solve on the
+    handle works."""
+    ts, _, b = _pair((6, 5, 4), precision="mixed")
+    x0, it0, _ = ts.pcg(b, rtol=5e-2)
+    ts.set_params(pcg_barrier_extra=1, pcg_spin_limit=2000)
+    with pytest.raises(g.DeviceTimeout):
+        ts.pcg(b, rtol=5e-2)
+    ts.set_params(pcg_barrier_extra=0, pcg_spin_limit=0)
+    x1, it1, _ = ts.pcg(b, rtol=5e-2)
+    assert it0 == it1 and np.array_equal(x0, x1)
