@@ -111,7 +111,9 @@ typedef struct {
                              launch (one reduction per iteration; equal to 0 up to rounding);
                              3 (default): in mixed precision 4 for the solves on the FP16 copy of the
                              scaled matrix (pcg_half_matrix, whose true-residual check covers the drift
-                             below) and 2 on the FP32 values; 0 in FP64 (the faster on GB300);
+                             below) and 2 on the FP32 values; in FP64 one launch with the vectors on chip
+                             (Chronopoulos-Gear, solves to 1e-3 or looser pipelined for pcg_pipe_iters
+                             iterations first) where they fit, 0 beyond (about 129,000 vertices);
                              4: pipelined PCG in one launch (one grid barrier per iteration, two more vertex
                              vectors, Chronopoulos-Gear after pcg_pipe_iters iterations; equal to 0 up to
                              rounding, but in FP32 its true residual drifts from the recursive one with the

@@ -328,6 +328,20 @@ size_t resident_sync_bytes();
 bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, const float4* dinv16, float4* x, float4* r,
                               float4* z, float4* p, float4* sv, float4* w, float4* m, const HalfSolveArgs& a,
                               const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st);
+// FP64 PCG on the symmetric store, the whole solve in one launch (set-up, iterations and, with check, g . x and |x|^2
+// into sc->gd, dnorm2): pipelined for pipe_iters iterations, then Chronopoulos-Gear; sl_off, lo_off: host copies of
+// A's slice offsets; m: 2 nv vectors of scratch.  false if the vectors do not fit on chip or the device cannot launch it
+struct Solve64Args {
+  const double* b;  // right-hand side sign * b (the Newton gradient g with negate = 1)
+  int negate;
+  double rtol;
+  int max_iters;
+  int pipe_iters;
+  int check;
+};
+bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int32_t* lo_off, const double* vals,
+                           const double4_32a* dinv, double4_32a* x, double4_32a* m, const Solve64Args& a, const Reduce& red,
+                           const ResidentSync& rs, int max_blocks, cudaStream_t st);
 // after a solve on the FP16 copy: g . d, |d|^2 (as launch_dot_gd) and the solve's true residual on the FP32
 // symmetric values, |-g - K d|^2 and |g|^2 (sc->true_rr, sc->true_bb)
 void launch_dot_gd_check(const SellMatrix& A, const float* vals, const double* g, const float4* d, const Reduce& red,

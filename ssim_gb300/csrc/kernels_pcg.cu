@@ -144,6 +144,21 @@ __device__ __forceinline__ bool exchange_barrier(const GridExchange& gx, unsigne
   return exchange_wait<float, 0>(gx, k, nullptr, 0, 0, xs);
 }
 
+// the solve's scalars for the host
+__device__ __forceinline__ void publish_scalars(const DevScalars& sc, DevScalars* o) {
+  o->rz = sc.rz;
+  o->rz_old = sc.rz_old;
+  o->pq = sc.pq;
+  o->rr = sc.rr;
+  o->rr0 = sc.rr0;
+  o->tol2 = sc.tol2;
+  o->alpha = sc.alpha;
+  o->beta = sc.beta;
+  o->iters = sc.iters;
+  o->done = sc.done;
+  o->status = sc.status;
+}
+
 // One unit of y = A x on the symmetric store: slice s's upper slots part, part + T, ... and lower slots
 // T - 1 - part, ... (the two run against each other, so the parts get equal shares), two slots in flight.
 template <typename S>
@@ -581,20 +596,7 @@ __global__ void __launch_bounds__(HT, 1)
     const float4 s4 = H.scale[u];
     x[u] = make_float4(xv[0] * s4.x, xv[1] * s4.y, xv[2] * s4.z, 0.f);
   }
-  if (ok && blockIdx.x == 0 && tid == 0) {
-    DevScalars* o = red.sc;
-    o->rz = sc.rz;
-    o->rz_old = sc.rz_old;
-    o->pq = sc.pq;
-    o->rr = sc.rr;
-    o->rr0 = sc.rr0;
-    o->tol2 = sc.tol2;
-    o->alpha = sc.alpha;
-    o->beta = sc.beta;
-    o->iters = sc.iters;
-    o->done = sc.done;
-    o->status = sc.status;
-  }
+  if (ok && blockIdx.x == 0 && tid == 0) publish_scalars(sc, red.sc);
   // the check on the FP32 values: every block's x is final after the exchange; the slices' dots go to the row
   // state's memory (no longer needed) in FP64
   if (ok && a.check) ok = exchange_barrier(gx, nx++, xs);
@@ -645,6 +647,275 @@ __global__ void __launch_bounds__(HT, 1)
     });
   }
   if (!ok && tid == 0) atomicExch(&red.sc->wait_failed, 1);
+}
+
+// ------------------------------------------------------------------ FP64
+struct Plan64 {
+  int grid, T, spc, cached;
+  int cache_entries;  // most entries of a block (when cached)
+  size_t smem;
+};
+
+constexpr int DT = 512;        // threads of a block
+constexpr int kState64 = 27;   // FP64 values of a row kept on chip: x r p s z w u (21), M (6)
+
+// PCG in FP64 on the symmetric store, the whole solve in one launch with the set-up and, with a.check, g . x and |x|^2
+// at its end: Chronopoulos-Gear (as cgcg_persistent_kernel), after pipe_iters pipelined iterations (as
+// resident_half_kernel, in the unscaled space) that save one of its two exchanges.  GB300 has two FP64 lanes an SM and
+// clock, so the work is laid out for them: any four warps fill the units, a lone warp fills one; the row recurrences
+// run a thread per dof (15 operations deep instead of 57), M r is carried in place of being formed twice, and T
+// partial products cost T - 1 additions, so T is 4 only where a block has fewer than four slices.  With CACHED the
+// block's rows of the matrix, lower triangle included, are copied to shared memory once a solve.  Bound by the
+// exchanges on small systems and by the FP64 units (135 operations a row in the product) beyond a few thousand rows.
+template <bool CACHED, int T>
+__global__ void __launch_bounds__(DT, 1)
+    resident64_kernel(SellMatrix A, const double* __restrict__ vals, const double4_32a* __restrict__ dinv, double4_32a* x,
+                      double4_32a* m, Solve64Args a, Plan64 pl, Reduce red, GridExchange gx) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ ExchangeShared xs;
+  __shared__ DevScalars sc;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nv = A.nv, nsl = (nv + 31) >> 5;
+  const int s0 = (int)((long long)blockIdx.x * nsl / gridDim.x), ns = (int)((long long)(blockIdx.x + 1) * nsl / gridDim.x) - s0;
+  const int RS = 32 * pl.spc, nd = 96 * ns;  // row stride of the state; dofs of this block (padding rows included)
+  constexpr int lt = T == 4 ? 2 : 1;
+  static_assert(T == 1 << lt, "T is 2 or 4");
+  double* cv = reinterpret_cast<double*>(smem);  // cached values: entry e (a multiple of 32) at 9 e + 32 c + lane
+  double* st = cv + (size_t)9 * pl.cache_entries;
+  double* pb = st + (size_t)kState64 * RS;       // unit partials
+  double* sh = pb + (size_t)3 * T * RS;          // 3 x DT partial dots
+  int* cc = reinterpret_cast<int*>(sh + 3 * DT);
+  double *X = st, *R = st + 3 * RS, *P = st + 6 * RS, *S = st + 9 * RS, *Z = st + 12 * RS, *W = st + 15 * RS,
+         *U = st + 18 * RS, *M = st + 21 * RS;
+  if (tid == 0) xs.fail = 0;
+  if constexpr (CACHED) {
+    for (int ls = warp; ls < ns; ls += DT / 32) {
+      const int s = s0 + ls, ub = A.sl_off[s], lb = A.lo_off[s];
+      const int Wu = (A.sl_off[s + 1] - ub) >> 5, Wl = (A.lo_off[s + 1] - lb) >> 5;
+      const int e0 = (ub - A.sl_off[s0]) + (lb - A.lo_off[s0]);
+      for (int k = 0; k < Wu + Wl; ++k) {
+        const bool up = k < Wu;
+        const int q = up ? ub + 32 * k + lane : A.lo_src[lb + 32 * (k - Wu) + lane];
+        // padding columns name the entry's own row, which may lie past the last vertex
+        cc[e0 + 32 * k + lane] = min(up ? A.sl_col[q] : A.lo_col[lb + 32 * (k - Wu) + lane], nv - 1);
+        const double* src = vals + sell_base(q);
+        double* dst = cv + (size_t)9 * (e0 + 32 * k) + lane;
+#pragma unroll
+        for (int c = 0; c < 9; ++c) dst[32 * c] = src[32 * (up ? c : 3 * (c % 3) + c / 3)];
+      }
+    }
+  }
+
+  auto spmv = [&](const double4_32a* v) {
+    for (int i = DT / 32 - 1 - warp; i < (ns << lt); i += DT / 32) {
+      const int ls = i >> lt, part = i & (T - 1), s = s0 + ls;
+      double a0 = 0, a1 = 0, a2 = 0;
+      if constexpr (CACHED) {
+        const int e0 = (A.sl_off[s] - A.sl_off[s0]) + (A.lo_off[s] - A.lo_off[s0]);
+        const int n = ((A.sl_off[s + 1] - A.sl_off[s]) + (A.lo_off[s + 1] - A.lo_off[s])) >> 5;
+        const double* pv = cv + (size_t)9 * e0 + lane;
+        for (int k = part; k < n; k += 2 * T) {
+          const bool two = k + T < n;
+          const int k1 = two ? k + T : k;
+          const double4_32a x0 = v[cc[e0 + 32 * k + lane]];
+          double4_32a x1 = v[cc[e0 + 32 * k1 + lane]];
+          const double *p0 = pv + 288 * k, *p1 = pv + 288 * k1;
+          a0 = fma(p0[64], x0.z, fma(p0[32], x0.y, fma(p0[0], x0.x, a0)));
+          a1 = fma(p0[160], x0.z, fma(p0[128], x0.y, fma(p0[96], x0.x, a1)));
+          a2 = fma(p0[256], x0.z, fma(p0[224], x0.y, fma(p0[192], x0.x, a2)));
+          if (two) {
+            a0 = fma(p1[64], x1.z, fma(p1[32], x1.y, fma(p1[0], x1.x, a0)));
+            a1 = fma(p1[160], x1.z, fma(p1[128], x1.y, fma(p1[96], x1.x, a1)));
+            a2 = fma(p1[256], x1.z, fma(p1[224], x1.y, fma(p1[192], x1.x, a2)));
+          }
+        }
+      } else if (32 * s + lane < nv) {
+        sym_unit<double>(A, vals, s, lane, part, T, v, a0, a1, a2);
+      }
+      double* o = pb + (size_t)3 * part * RS + 32 * ls + lane;
+      o[0] = a0;
+      o[RS] = a1;
+      o[2 * RS] = a2;
+    }
+  };
+  // dof j of the block: component j / (32 ns) of row j % (32 ns), so that a warp's threads share the component
+  auto dof = [&](int j, int& c, int& l) {
+    const int n = 32 * ns;
+    c = (j >= n) + (j >= 2 * n);
+    l = j - c * n;
+  };
+  auto product = [&](int c, int l) {
+    const double* o = pb + (size_t)c * RS + l;
+    double t = o[0];
+#pragma unroll
+    for (int q = 1; q < T; ++q) t += o[(size_t)3 * q * RS];
+    return t;
+  };
+  // component c of the symmetric M v; M holds the rows' (00, 01, 02, 11, 12, 22)
+  auto precond = [&](const double* v, int c, int l) {
+    const int i0 = c, i1 = c == 0 ? 1 : c + 2, i2 = c == 0 ? 2 : c + 3;
+    return fma(M[(size_t)i2 * RS + l], v[2 * RS + l], fma(M[(size_t)i1 * RS + l], v[RS + l], M[(size_t)i0 * RS + l] * v[l]));
+  };
+  auto put = [&](double4_32a* g, int u, int c, double v) { reinterpret_cast<double*>(g + u)[c] = v; };
+
+  // set-up
+  const double sg = a.negate ? -1.0 : 1.0;
+  for (int l = tid; l < 32 * ns; l += DT) {
+    const int u = 32 * s0 + l;
+    double4_32a d0 = mk4<double>(0, 0, 0), d1 = d0, d2 = d0;
+    if (u < nv) {
+      d0 = dinv[3 * (size_t)u];
+      d1 = dinv[3 * (size_t)u + 1];
+      d2 = dinv[3 * (size_t)u + 2];
+    }
+    const double d[6] = {d0.x, d0.y, d0.z, d1.y, d1.z, d2.z};
+#pragma unroll
+    for (int c = 0; c < 6; ++c) M[(size_t)c * RS + l] = d[c];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      R[c * RS + l] = u < nv ? sg * a.b[3 * (size_t)u + c] : 0.0;
+      X[c * RS + l] = P[c * RS + l] = S[c * RS + l] = Z[c * RS + l] = 0.0;
+    }
+  }
+  __syncthreads();
+  for (int j = tid; j < nd; j += DT) {
+    int c, l;
+    dof(j, c, l);
+    const double u0 = precond(R, c, l);
+    U[c * RS + l] = u0;
+    if (32 * s0 + l < nv) put(m + nv, 32 * s0 + l, c, u0);  // u0 in the second half of m
+  }
+  unsigned long long nx = 0;
+  bool ok = exchange_barrier(gx, nx++, xs);
+  const int np = min(DT, nd);
+  auto store_dots = [&](double d0, double d1, double d2) {
+    sh[tid] = d0;
+    sh[DT + tid] = d1;
+    sh[2 * DT + tid] = d2;
+  };
+  if (ok) {  // prologue: w = A u0, m_0 = M w
+    spmv(m + nv);
+    __syncthreads();
+    for (int j = tid; j < nd; j += DT) {
+      int c, l;
+      dof(j, c, l);
+      W[c * RS + l] = product(c, l);
+    }
+    __syncthreads();
+    double d0 = 0, d1 = 0, d2 = 0;
+    for (int j = tid; j < nd; j += DT) {
+      int c, l;
+      dof(j, c, l);
+      const double r = R[c * RS + l], u = U[c * RS + l];
+      d0 = fma(r, u, d0);
+      d1 = fma(W[c * RS + l], u, d1);
+      d2 = fma(r, r, d2);
+      if (a.pipe_iters > 0 && 32 * s0 + l < nv) put(m, 32 * s0 + l, c, precond(W, c, l));
+    }
+    store_dots(d0, d1, d2);
+  }
+  for (int k = 0; ok; ++k) {
+    const bool first = k == 0;
+    __syncthreads();
+    ok = exchange_wait<double, 3>(gx, nx, sh, DT, np, xs);
+    if (!ok) break;
+    exchange_total<3>(gx, nx++, xs, [&](const double(&t)[3]) {
+      if (first) {  // the stop test is relative to this residual
+        sc.done = 0;
+        sc.rz_old = 1.0;
+        sc.rr0 = t[2];
+        sc.tol2 = a.rtol * a.rtol * t[2];
+        sc.iters = 0;
+        sc.status = 0;
+        sc.alpha = sc.beta = 0.0;
+      }
+      cgcg_after(&sc, t[0], t[1], t[2], a.max_iters);
+    });
+    const bool pipe = k < a.pipe_iters;
+    const double4_32a* mk = m + (size_t)(k & 1) * nv;
+    double4_32a* mn = m + (size_t)((k + 1) & 1) * nv;
+    if (pipe) spmv(mk);  // n = A m while the scalars are made
+    __syncthreads();
+    if (sc.done) break;
+    const double alpha = sc.alpha, beta = sc.beta;
+    double d0 = 0, d1 = 0, d2 = 0;
+    for (int j = tid; j < nd; j += DT) {
+      int c, l;
+      dof(j, c, l);
+      const int i = c * RS + l;
+      const double w = W[i], p = fma(beta, P[i], U[i]), s = fma(beta, S[i], w);
+      P[i] = p;
+      S[i] = s;
+      X[i] = fma(alpha, p, X[i]);
+      R[i] = fma(-alpha, s, R[i]);
+      if (pipe) {
+        const double z = fma(beta, Z[i], product(c, l));
+        Z[i] = z;
+        W[i] = fma(-alpha, z, w);
+      }
+    }
+    __syncthreads();
+    for (int j = tid; j < nd; j += DT) {
+      int c, l;
+      dof(j, c, l);
+      const int i = c * RS + l;
+      const double u = precond(R, c, l);
+      U[i] = u;
+      if (pipe) {
+        const double r = R[i];
+        d0 = fma(r, u, d0);
+        d1 = fma(W[i], u, d1);
+        d2 = fma(r, r, d2);
+      }
+      if (32 * s0 + l < nv) put(mn, 32 * s0 + l, c, pipe ? precond(W, c, l) : u);
+    }
+    if (!pipe) {  // Chronopoulos-Gear: w = A u after every block's u is there
+      ok = exchange_barrier(gx, nx++, xs);
+      if (!ok) break;
+      spmv(mn);
+      __syncthreads();
+      for (int j = tid; j < nd; j += DT) {
+        int c, l;
+        dof(j, c, l);
+        const int i = c * RS + l;
+        const double r = R[i], u = U[i], w = product(c, l);
+        W[i] = w;
+        d0 = fma(r, u, d0);
+        d1 = fma(w, u, d1);
+        d2 = fma(r, r, d2);
+      }
+    }
+    store_dots(d0, d1, d2);
+  }
+  __syncthreads();
+  double q[2] = {0, 0};
+  for (int l = tid; l < 32 * ns; l += DT) {
+    const int u = 32 * s0 + l;
+    if (u >= nv) continue;
+    const double x0 = X[l], x1 = X[RS + l], x2 = X[2 * RS + l];
+    x[u] = mk4<double>(x0, x1, x2);
+    if (a.check) {
+      q[0] = fma(a.b[3 * (size_t)u + 2], x2, fma(a.b[3 * (size_t)u + 1], x1, fma(a.b[3 * (size_t)u], x0, q[0])));
+      q[1] = fma(x2, x2, fma(x1, x1, fma(x0, x0, q[1])));
+    }
+  }
+  if (ok && blockIdx.x == 0 && tid == 0) publish_scalars(sc, red.sc);
+  if (ok && a.check) {
+    sh[tid] = q[0];
+    sh[DT + tid] = q[1];
+    ok = exchange<double, 2>(gx, nx++, sh, DT, min(DT, 32 * ns), xs, [&](const double(&t)[2]) {
+      if (blockIdx.x == 0) {
+        red.sc->gd = t[0];
+        red.sc->dnorm2 = t[1];
+      }
+    });
+  }
+  if (!ok && tid == 0) atomicExch(&red.sc->wait_failed, 1);
+}
+
+size_t smem64(const Plan64& p) {
+  const size_t rs = (size_t)32 * p.spc;
+  return 8 * ((size_t)9 * p.cache_entries + kState64 * rs + 3 * p.T * rs + 3 * DT) + 4 * (size_t)p.cache_entries + 64;
 }
 
 constexpr size_t kSmemReserve = 8 * 1024;  // static shared memory and the 1 KB a block costs
@@ -699,25 +970,37 @@ static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, 
   return half_smem(q) <= smem_max ? q : p;
 }
 
-bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, const float4* dinv16, float4* x, float4* r,
-                              float4* z, float4* p, float4* sv, float4* w, float4* m, const HalfSolveArgs& pa,
-                              const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st) {
-  if (H.nv <= 0) return true;
-  int dev = 0, coop = 0, nsm = 0, smax = 0, per_sm = 0;
+// properties of the current device that a resident launch needs; false without cooperative launches
+static bool resident_device(int& nsm, size_t& smem_max) {
+  int dev = 0, coop = 0, smax = 0;
   SSIM_CUDA(cudaGetDevice(&dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-  if (!coop) return false;
-  HalfPlan pl = half_plan(H.nv, off_host, nsm, (size_t)smax - kSmemReserve, max_blocks);
+  smem_max = (size_t)smax - kSmemReserve;
+  return coop != 0;
+}
+static bool resident_fits(const void* fn, int threads, size_t smem) {
+  int per_sm = 0;
+  SSIM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
+  return per_sm >= 1;
+}
+
+bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, const float4* dinv16, float4* x, float4* r,
+                              float4* z, float4* p, float4* sv, float4* w, float4* m, const HalfSolveArgs& pa,
+                              const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st) {
+  if (H.nv <= 0) return true;
+  int nsm = 0;
+  size_t smem_max = 0;
+  if (!resident_device(nsm, smem_max)) return false;
+  HalfPlan pl = half_plan(H.nv, off_host, nsm, smem_max, max_blocks);
   if (pl.grid < 1) return false;
   pl.smem = half_smem(pl);
   const void* fn = !pl.cached   ? (const void*)resident_half_kernel<false, 4>
                    : pl.T == 4 ? (const void*)resident_half_kernel<true, 4>
                                : (const void*)resident_half_kernel<true, 8>;
-  SSIM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-  SSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, HT, pl.smem));
-  if (per_sm < 1) return false;
+  if (!resident_fits(fn, HT, pl.smem)) return false;
   GridExchange gx = grid_exchange(rs, st);
   HalfMatrix h = H;
   HalfSolveArgs ha = pa;
@@ -726,6 +1009,55 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
                   (void*)&w, (void*)&m,      (void*)&ha, (void*)&pl, (void*)&rd, (void*)&gx};
   SSIM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(pl.grid), dim3(HT), args, pl.smem, st));
   after_launch("pcg_half_resident");
+  return true;
+}
+
+// Layout of a resident FP64 solve: all rows' vectors on chip or none (about 850 rows a block, 129,000 on 152 SMs), the
+// matrix entries too where they fit (about 24,000 rows).  grid 0: does not fit.
+static Plan64 plan64(int nv, const int32_t* sl_off, const int32_t* lo_off, int nsm, size_t smem_max, int max_blocks) {
+  Plan64 p{};
+  const int nsl = div_up(nv, 32);
+  p.grid = std::max(1, std::min(std::min(nsm, kMaxBlocks), nsl));
+  if (max_blocks > 0) p.grid = std::min(p.grid, max_blocks);
+  Plan64 q{};
+  for (int c = 0; c < p.grid; ++c) {
+    const int a = part_begin(c, nsl, p.grid), b = part_begin(c + 1, nsl, p.grid);
+    p.spc = std::max(p.spc, b - a);
+    q.cache_entries = std::max(q.cache_entries, (sl_off[b] - sl_off[a]) + (lo_off[b] - lo_off[a]));
+  }
+  p.T = p.spc < 4 ? 4 : 2;
+  q.grid = p.grid;
+  q.spc = p.spc;
+  q.T = p.T;
+  q.cached = 1;
+  if (smem64(q) <= smem_max) return q;
+  p.T = 2;
+  if (smem64(p) > smem_max) p.grid = 0;
+  return p;
+}
+
+bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int32_t* lo_off, const double* vals,
+                           const double4_32a* dinv, double4_32a* x, double4_32a* m, const Solve64Args& sa, const Reduce& red,
+                           const ResidentSync& rs, int max_blocks, cudaStream_t st) {
+  if (A.nv <= 0) return true;
+  int nsm = 0;
+  size_t smem_max = 0;
+  if (!resident_device(nsm, smem_max)) return false;
+  Plan64 pl = plan64(A.nv, sl_off, lo_off, nsm, smem_max, max_blocks);
+  if (pl.grid < 1) return false;
+  pl.smem = smem64(pl);
+  const void* fn = !pl.cached   ? (const void*)resident64_kernel<false, 2>
+                   : pl.T == 2 ? (const void*)resident64_kernel<true, 2>
+                               : (const void*)resident64_kernel<true, 4>;
+  if (!resident_fits(fn, DT, pl.smem)) return false;
+  GridExchange gx = grid_exchange(rs, st);
+  SellMatrix a = A;
+  Solve64Args s = sa;
+  Reduce rd = red;
+  void* args[] = {(void*)&a, (void*)&vals, (void*)&dinv, (void*)&x,  (void*)&m,
+                  (void*)&s, (void*)&pl,   (void*)&rd,   (void*)&gx};
+  SSIM_CUDA(cudaLaunchCooperativeKernel(fn, dim3(pl.grid), dim3(DT), args, pl.smem, st));
+  after_launch("pcg64_resident");
   return true;
 }
 

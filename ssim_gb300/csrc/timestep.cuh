@@ -82,6 +82,9 @@ struct Solver {
 
 // PK_PCG counts iterations of the persistent PCG kernel (one launch per solve), so total / count is the
 // time of one PCG iteration
+// FP64 solves at least this loose run their first pcg_pipe_iters iterations pipelined
+constexpr double kPipe64MinRtol = 1e-3;
+
 enum ProfileKernel { PK_SPMV = 0, PK_HESS = 1, PK_ASM = 2, PK_GRAD = 3, PK_UPD = 4, PK_PCG = 5, PK_COUNT = 6 };
 
 struct TimeStep {
@@ -158,6 +161,7 @@ struct TimeStep {
   long long nfs = 0;
   long long asm_count = 0, h16_count = -1;  // assemblies of the FP32 values; the one the copy was made from
   bool last_half = false;  // the last pcg() ran on the FP16 copy
+  bool gd_ready = false;   // the last pcg() left g . d and |d|^2 in the scalars
   bool half_checked = false;  // ... and its kernel left g . d, |d|^2 and the true residual in the scalars
   // speculative assembly (speculative_hessian): the next Newton iteration's Hessian at the full step, built on
   // a second stream while the line search runs on the handle's stream
@@ -985,13 +989,16 @@ struct TimeStep {
   template <typename S>
   int pcg(const double* b, bool negate, double eta, int max_iters, double* rel_res) {
     Solver<S>& s = solver<S>();
-    last_half = false;
+    last_half = gd_ready = false;
     if constexpr (std::is_same<S, float>::value) {
       int it = 0;
       if (use_half(eta) && pcg_half(b, negate, eta, max_iters, rel_res, &it)) {
         last_half = true;
         return it;
       }
+    } else {
+      int it = 0;
+      if (params.pcg_persistent == 3 && pcg_resident64(b, negate, eta, max_iters, rel_res, &it)) return it;
     }
     launch_pcg_setup<S>(nv, b, s.dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, eta, max_iters, negate, red(), stream);
     return pcg_loop<S>(s.vals.p, s.dinv.p, max_iters, rel_res, true);
@@ -1040,6 +1047,37 @@ struct TimeStep {
     return true;
   }
 
+  // FP64 PCG with the vectors on chip (the automatic choice where they fit): one cooperative launch and one host wait
+  // a solve.  Loose solves (the inexact Newton's) start with pipelined iterations, whose recursive residual is off the
+  // true one by rounding only; tighter ones are Chronopoulos-Gear throughout.  Per iteration, set-up and g . d included,
+  // against two launches and their host checks: 5.6 against 28 us on 1,331 vertices, 9.7 against 28 on 16,240 (loose),
+  // 10.5 against 29.6 on 15,625 (to 1e-10)
+  bool pcg_resident64(const double* b, bool negate, double eta, int max_iters, double* rel_res, int* iters) {
+    Solver<double>& s = sd;
+    if (s.pm.n < 2 * (size_t)nv) s.pm.alloc(2 * (size_t)nv);
+    const Solve64Args sa{b, negate ? 1 : 0, eta, max_iters, eta >= kPipe64MinRtol ? params.pcg_pipe_iters : 0, negate ? 1 : 0};
+    if (profiling) SSIM_CUDA(cudaEventRecord(ev[0], stream));
+    if (!launch_pcg64_resident(A(), topo.sl_off.data(), topo.lo_off.data(), s.vals.p, s.dinv.p, s.x.p, s.pm.p, sa, red(),
+                               resident_sync(), params.pcg_max_blocks, stream))
+      return false;
+    if (profiling) SSIM_CUDA(cudaEventRecord(ev[1], stream));
+    sync_scalars();
+    check_wait();
+    gd_ready = negate;
+    if (profiling) {
+      float ms = 0;
+      SSIM_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
+      prof_ms[PK_PCG] += ms;
+      prof_launch[PK_PCG] += hsc->iters;
+      prof_bytes[PK_PCG] = spmv_bytes(sizeof(double)) + update_bytes(sizeof(double));
+    }
+    if (rel_res) *rel_res = hsc->rr0 > 0 ? std::sqrt(hsc->rr / hsc->rr0) : 0.0;
+    if (hsc->status == 2) throw numerical_error("PCG produced a non-finite residual");
+    if (solve_log.size() < (1u << 20)) solve_log.push_back(hsc->iters);
+    *iters = hsc->iters;
+    return true;
+  }
+
   // PCG on another matrix of the same block pattern (the PD matrix) with an S right-hand side
   template <typename S>
   int pcg_on(const S* vals, const V4<S>* dinv, const V4<S>* b, double eta, int max_iters, double* rel_res,
@@ -1054,8 +1092,8 @@ struct TimeStep {
                bool kron = false) {
     Solver<S>& s = solver<S>();
     int variant = params.pcg_persistent;
-    // automatic: FP64 runs two launches per iteration (its FP64 dots and updates make the persistent
-    // kernels slower on GB300), FP32 Chronopoulos-Gear.  Pipelined PCG (4) is opt-in: its recursive
+    // automatic: FP64 solves that do not fit on chip (pcg_resident64) run two launches per iteration (their FP64 dots
+    // and updates make the persistent kernels slower on GB300), FP32 Chronopoulos-Gear.  Pipelined PCG (4) is opt-in: its recursive
     // residual drifts from the true one in FP32 by an amount that grows with the iterations and the
     // condition number, which a loose tolerance does not cover for ill-conditioned systems (cloth, thin
     // sheets)
@@ -1491,7 +1529,7 @@ struct TimeStep {
       // after reset(), the first of each step) let the copy cost it a fifth more Newton iterations
       const bool checked = last_half;
       st.half_solves += last_half ? 1 : 0;
-      if (!(checked && half_checked)) {  // the pipelined solve on the copy did this in its own launch
+      if (!(checked && half_checked) && !gd_ready) {  // the resident solves did this in their own launch
         if constexpr (std::is_same<S, float>::value) {
           if (checked)
             launch_dot_gd_check(A(), s.vals.p, forces.p, s.x.p, red(), stream);

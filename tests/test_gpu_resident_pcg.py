@@ -90,3 +90,37 @@ def test_half_solve_wait_gives_up():
     ts.set_params(pcg_barrier_extra=0, pcg_spin_limit=0)
     x1, it1, _ = ts.pcg(b, rtol=5e-2)
     assert it0 == it1 and np.array_equal(x0, x1)
+
+
+@pytest.mark.parametrize("hexes,blocks", LAYOUTS)
+def test_fp64_solve_matches_two_launch(hexes, blocks):
+    """FP64 against the two-launch PCG.  Loose solves (pipelined, then Chronopoulos-Gear) and tight
+    ones (Chronopoulos-Gear): iteration counts within 2, true residuals at the tolerance (1.5 of it, as the persistent
+    variants'; at 1e-10 a drift of the recursive residual of 1e-11 is 0.1 of the tolerance), a capped solve's iterate
+    within 1e-12."""
+    ts, _, b = _pair(hexes, precision="fp64", pcg_max_blocks=blocks)
+    bn = np.linalg.norm(b)
+    for rtol in (5e-2, 1e-6, 1e-10):
+        ts.set_params(pcg_persistent=3)
+        x, it, rr = ts.pcg(b, rtol=rtol)
+        ts.set_params(pcg_persistent=0)
+        x0, it0, _ = ts.pcg(b, rtol=rtol)
+        assert rr <= rtol and abs(it - it0) <= 2, (rtol, it, it0)
+        assert np.linalg.norm(b - ts.spmv(x)) <= 1.5 * rtol * bn
+    for rtol, pipe in ((1e-2, 80), (1e-2, 3), (1e-12, 80)):
+        ts.set_params(pcg_persistent=3, pcg_pipe_iters=pipe)
+        x, it, _ = ts.pcg(b, rtol=rtol, max_iters=7)
+        ts.set_params(pcg_persistent=0)
+        x0, it0, _ = ts.pcg(b, rtol=rtol, max_iters=7)
+        assert it == it0 and np.linalg.norm(x - x0) <= 1e-12 * np.linalg.norm(x0)
+
+
+def test_fp64_solve_wait_gives_up():
+    ts, _, b = _pair((6, 5, 4), precision="fp64")
+    x0, it0, _ = ts.pcg(b, rtol=1e-8)
+    ts.set_params(pcg_barrier_extra=1, pcg_spin_limit=2000)
+    with pytest.raises(g.DeviceTimeout):
+        ts.pcg(b, rtol=1e-8)
+    ts.set_params(pcg_barrier_extra=0, pcg_spin_limit=0)
+    x1, it1, _ = ts.pcg(b, rtol=1e-8)
+    assert it0 == it1 and np.array_equal(x0, x1)
