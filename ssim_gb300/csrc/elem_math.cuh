@@ -351,27 +351,137 @@ __host__ __device__ __forceinline__ void swap_cols_keep_det(S* V, S* d, int i, i
   }
 }
 
-// Rotation-variant SVD F = U diag(s) V^T with U, V in SO(3), s0 >= s1 >= |s2|, s2 < 0 for inverted F.
-// V from the Jacobi eigenvectors of F^T F, U and s from a Givens QR of F V (the approach of McAdams et
-// al., "Computing the SVD of 3x3 matrices with minimal branching", 2011, written here with exact
-// Jacobi rotations).
-template <typename S>
-__host__ __device__ __forceinline__ void svd3(const S* F, S* U, S* s, S* V) {
-  S A[9];
+// V in SO(3) whose columns are eigenvectors of F^T F, largest first (cyclic Jacobi)
+__host__ __device__ __forceinline__ void right_basis(const float* F, float* V) {
+  float A[9];
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) A[i * 3 + j] = F[0 * 3 + i] * F[0 * 3 + j] + F[1 * 3 + i] * F[1 * 3 + j] + F[2 * 3 + i] * F[2 * 3 + j];
   sym_eig3(A, V);
-  S d[3] = {A[0], A[4], A[8]};
+  float d[3] = {A[0], A[4], A[8]};
   if (d[0] < d[1]) swap_cols_keep_det(V, d, 0, 1);
   if (d[0] < d[2]) swap_cols_keep_det(V, d, 0, 2);
   if (d[1] < d[2]) swap_cols_keep_det(V, d, 1, 2);
-  S B[9];
+}
+
+template <typename S>
+__host__ __device__ __forceinline__ void mul33(const S* F, const S* V, S* B) {  // B = F V
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) B[i * 3 + j] = F[i * 3 + 0] * V[0 * 3 + j] + F[i * 3 + 1] * V[1 * 3 + j] + F[i * 3 + 2] * V[2 * 3 + j];
+}
+
+// B = F V with orthogonal columns, V in SO(3)
+__host__ __device__ __forceinline__ void orthogonal_columns(const float* F, float* V, float* B) {
+  right_basis(F, V);
+  mul33(F, V, B);
+}
+
+// In FP64 the Jacobi sweeps from the identity were most of the element Hessian on GB300, whose FP64 units take a
+// warp's operation every 64 cycles: V comes from the FP32 problem (orthonormalised in FP64, off by 1e-7), and
+// one-sided Jacobi sweeps (Hestenes 1958) on the columns of B = F V finish it in FP64, usually two.  A rotation's
+// tangent is formed in FP32: an angle off by 1e-7 of itself leaves 1e-7 of the product it removes, which the next
+// sweep sees; the rotation itself is orthogonal to FP64 rounding.
+__host__ __device__ __forceinline__ void orthogonal_columns(const double* F, double* V, double* B) {
+  float f[9], v[9], mx = 0.f;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) {
+    f[k] = (float)F[k];
+    mx = fmaxf(mx, fabsf(f[k]));
+  }
+  const bool fine = mx > 1e-15f && mx < 1e15f;  // F^T F is well inside FP32's range
+  if (fine) {
+    right_basis(f, v);
+    double a[3] = {v[0], v[3], v[6]}, b[3] = {v[1], v[4], v[7]};
+    // 1 / |a| with |a|^2 = 1 + e, e ~ 1e-6: 1 - e / 2 + 3 e^2 / 8
+    double e = a[0] * a[0] + a[1] * a[1] + a[2] * a[2] - 1.0, r = 1.0 + e * (0.375 * e - 0.5);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) a[i] *= r;
+    const double d = a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) b[i] -= d * a[i];
+    e = b[0] * b[0] + b[1] * b[1] + b[2] * b[2] - 1.0;
+    r = 1.0 + e * (0.375 * e - 0.5);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) b[i] *= r;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      V[3 * i] = a[i];
+      V[3 * i + 1] = b[i];
+      V[3 * i + 2] = a[(i + 1) % 3] * b[(i + 2) % 3] - a[(i + 2) % 3] * b[(i + 1) % 3];
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 9; ++i) V[i] = (i % 4 == 0) ? 1.0 : 0.0;
+  }
+  mul33(F, V, B);
+  double n2 = 0;
+#pragma unroll
+  for (int i = 0; i < 9; ++i) n2 += F[i] * F[i];
+  const double low = 1e-34 * (n2 * n2);
+  for (int sweep = 0; sweep < 16; ++sweep) {
+    bool any = false;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int p = k == 2 ? 1 : 0, q = k == 0 ? 1 : 2;
+      const double al = B[p] * B[p] + B[3 + p] * B[3 + p] + B[6 + p] * B[6 + p];
+      const double be = B[q] * B[q] + B[3 + q] * B[3 + q] + B[6 + q] * B[6 + q];
+      const double ga = B[p] * B[q] + B[3 + p] * B[3 + q] + B[6 + p] * B[6 + q];
+      // columns orthogonal to rounding, or their product below it beside |F|^2 (columns that vanish)
+      if (!(ga * ga > fmax(1e-30 * (al * be), low))) continue;
+      any = true;
+      const float z = fine ? (float)(be - al) / (2.f * (float)ga) : (float)((be - al) / (2.0 * ga));
+      const float az = fabsf(z), ta = az > 1e9f ? 0.5f / az : 1.f / (az + sqrtf(1.f + az * az));
+      const double t = z < 0.f ? -(double)ta : (double)ta, t2 = t * t;
+      // 1 / sqrt(1 + t^2): its series to t^6 below 1e-2 (the next term is 2.7e-17)
+      const double c = t2 < 1e-4 ? 1.0 - t2 * (0.5 - t2 * (0.375 - 0.3125 * t2)) : 1.0 / sqrt(1.0 + t2);
+      const double s = c * t;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) {
+        const double bp = B[3 * i + p], bq = B[3 * i + q], vp = V[3 * i + p], vq = V[3 * i + q];
+        B[3 * i + p] = c * bp - s * bq;
+        B[3 * i + q] = s * bp + c * bq;
+        V[3 * i + p] = c * vp - s * vq;
+        V[3 * i + q] = s * vp + c * vq;
+      }
+    }
+    if (!any) break;
+  }
+}
+
+// Rotation-variant SVD F = U diag(s) V^T with U, V in SO(3), s0, s1 >= 0, s2 < 0 for inverted F.  V makes the columns
+// of B = F V orthogonal; U and s come from normalising them (the third column as the cross product of the first two,
+// so it is there for a flat element and carries the sign), or, where the second column is too short beside the first
+// for that, from a Givens QR of B (the approach of McAdams et al., "Computing the SVD of 3x3 matrices with minimal
+// branching", 2011, written here with exact Jacobi rotations).
+template <typename S>
+__host__ __device__ __forceinline__ void svd3(const S* F, S* U, S* s, S* V) {
+  S B[9];
+  orthogonal_columns(F, V, B);
+  const S n0 = B[0] * B[0] + B[3] * B[3] + B[6] * B[6];
+  const S i0 = S(1) / sqrt(n0);
+  const S a[3] = {B[0] * i0, B[3] * i0, B[6] * i0};
+  const S d = a[0] * B[1] + a[1] * B[4] + a[2] * B[7];
+  const S b[3] = {B[1] - d * a[0], B[4] - d * a[1], B[7] - d * a[2]};
+  const S n1 = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
+  const S flat = sizeof(S) == 8 ? S(1e-20) : S(1e-8);
+  if (n1 > flat * n0 && n0 > S(0)) {
+    const S i1 = S(1) / sqrt(n1);
+    s[0] = n0 * i0;
+    s[1] = n1 * i1;
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+      U[3 * i] = a[i];
+      U[3 * i + 1] = b[i] * i1;
+    }
+    U[2] = U[3] * U[7] - U[6] * U[4];
+    U[5] = U[6] * U[1] - U[0] * U[7];
+    U[8] = U[0] * U[4] - U[3] * U[1];
+    s[2] = U[2] * B[2] + U[5] * B[5] + U[8] * B[8];
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 9; ++i) U[i] = (i % 4 == 0) ? S(1) : S(0);
   givens_qr(B, U, 0, 1, 0);
@@ -384,16 +494,6 @@ __host__ __device__ __forceinline__ void svd3(const S* F, S* U, S* s, S* V) {
 
 // packed upper-triangular index of the 12x12 stiffness
 __host__ __device__ constexpr int kup(int i, int j) { return i * 12 - (i * (i - 1)) / 2 + (j - i); }
-
-template <typename S>
-__host__ __device__ __forceinline__ void rank1(S* K, S w, const S* g) {
-#pragma unroll
-  for (int i = 0; i < 12; ++i) {
-    const S wi = w * g[i];
-#pragma unroll
-    for (int j = i; j < 12; ++j) K[kup(i, j)] += wi * g[j];
-  }
-}
 
 // Element stiffness of the linear model, packed upper triangle (78) times scale.  Its 9x9 Hessian
 // mu (I + T) + lambda d d^T (T: the transpose permutation, d = vec I) has the eigenspaces symmetric-
@@ -436,77 +536,136 @@ __host__ __device__ __forceinline__ void linear_stiffness(const S D[4][3], S lam
 // (k the third index), and the three scaling modes U diag(q) V^T come from the 3x3 block
 //   A3 = a I + b s s^T + lambda g g^T + c [[0,s2,s1],[s2,0,s0],[s1,s0,0]],  g = (s1 s2, s0 s2, s0 s1)
 // (the mode structure of Smith, de Goes & Kim, "Analytic Eigensystems for Isotropic Distortion
-// Energies", 2019, derived here for this energy's I2/I3 form).  Each mode contracts with the shape
-// gradients D (4x3) into a 12-vector G(v*3+a) = (E D^T)(a, v), and K accumulates l_m G G^T.
-// Output: packed upper triangle (78 entries), times `scale`.
+// Energies", 2019, derived here for this energy's I2/I3 form).
+//
+// In the frame of U and V the projected H has few entries: A3+ between (i, i) and (k, k), and for i != j with third
+// index k (l_t + l_f) / 2 on (i, j) and (l_f - l_t) / 2 between (i, j) and (j, i).  Contracted with W = D V (D the shape
+// gradients) the block of vertices v, w is K_vw = U B U^T with
+//   B(i, i) = A3+(i, i) W_vi W_wi + sum_j t_ij W_vj W_wj,   B(i, k) = A3+(i, k) W_vi W_wk + f_ik W_vk W_wi.
+// Six blocks are formed so (vertices 1 to 3); the shape gradients sum to zero, so the rows of vertex 0 are minus sums
+// of them.  About 600 operations after the SVD in place of the 1,060 of nine rank-one updates, one block at a time
+// instead of 78 live sums.  A3 is only diagonalised where its Cholesky minors do not already show every eigenvalue
+// above eps (A3+ = A3 then).
+// emit(v, w, block): the ten upper 3x3 blocks (v <= w, row-major), times scale, each once.
+template <typename S, typename EMIT>
+__host__ __device__ __forceinline__ void element_stiffness_blocks(const S* F, const S D[4][3], S lam, S mu, bool spsd,
+                                                                  S scale, EMIT&& emit) {
+  S U[9], W[3][3], h[6], t[3], f[3];  // h: A3+ (00, 01, 02, 11, 12, 22); t, f by the third index
+  {
+    S s[3], V[9];
+    svd3(F, U, s, V);
+    const S I2 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
+    const S I3 = s[0] * s[1] * s[2];
+    const S alpha = S(0.75) * mu / lam + S(1);
+    const S q = S(1) / (I2 + S(1));
+    const S a = mu * (S(1) - q);
+    const S b = mu * (S(2) * q * q);
+    const S c = lam * (I3 - alpha);
+    const S eps = S(1e-3);
+#pragma unroll
+    for (int v = 0; v < 3; ++v)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        W[v][j] = D[v + 1][0] * V[0 * 3 + j] + D[v + 1][1] * V[1 * 3 + j] + D[v + 1][2] * V[2 * 3 + j];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      S lt = a + c * s[k], lf = a - c * s[k];
+      if (spsd) {
+        lt = fmax(lt, eps);
+        lf = fmax(lf, eps);
+      }
+      t[k] = S(0.5) * scale * (lf + lt);
+      f[k] = S(0.5) * scale * (lf - lt);
+    }
+    const S g0 = s[1] * s[2], g1 = s[0] * s[2], g2 = s[0] * s[1];
+    h[0] = a + b * s[0] * s[0] + lam * g0 * g0;
+    h[3] = a + b * s[1] * s[1] + lam * g1 * g1;
+    h[5] = a + b * s[2] * s[2] + lam * g2 * g2;
+    h[1] = b * s[0] * s[1] + lam * g0 * g1 + c * s[2];
+    h[2] = b * s[0] * s[2] + lam * g0 * g2 + c * s[1];
+    h[4] = b * s[1] * s[2] + lam * g1 * g2 + c * s[0];
+    if (spsd) {
+      // leading minors of A3 less eps and a rounding margin: all eigenvalues above eps
+      const S m = eps + (sizeof(S) == 8 ? S(1e-14) : S(4e-6)) * (fabs(h[0]) + fabs(h[3]) + fabs(h[5]));
+      const S p0 = h[0] - m, p1 = h[3] - m, p2 = h[5] - m;
+      const S c0 = p1 * p2 - h[4] * h[4], c1 = h[1] * p2 - h[2] * h[4], c2 = h[1] * h[4] - h[2] * p1;
+      const bool pd = p0 > S(0) && p0 * p1 - h[1] * h[1] > S(0) && p0 * c0 - h[1] * c1 + h[2] * c2 > S(0);
+      if (!pd) {
+        // scaled to entries near 1: sym_eig3 tests sums of squares
+        const S big = fmax(fmax(fabs(h[0]), fabs(h[3])), fmax(fabs(h[5]), eps)), ib = S(1) / big;
+        S A[9] = {h[0] * ib, h[1] * ib, h[2] * ib, h[1] * ib, h[3] * ib, h[4] * ib, h[2] * ib, h[4] * ib, h[5] * ib}, Q[9];
+        sym_eig3(A, Q);
+        const S l0 = fmax(A[0] * big, eps), l1 = fmax(A[4] * big, eps), l2 = fmax(A[8] * big, eps);
+        h[0] = l0 * Q[0] * Q[0] + l1 * Q[1] * Q[1] + l2 * Q[2] * Q[2];
+        h[1] = l0 * Q[0] * Q[3] + l1 * Q[1] * Q[4] + l2 * Q[2] * Q[5];
+        h[2] = l0 * Q[0] * Q[6] + l1 * Q[1] * Q[7] + l2 * Q[2] * Q[8];
+        h[3] = l0 * Q[3] * Q[3] + l1 * Q[4] * Q[4] + l2 * Q[5] * Q[5];
+        h[4] = l0 * Q[3] * Q[6] + l1 * Q[4] * Q[7] + l2 * Q[5] * Q[8];
+        h[5] = l0 * Q[6] * Q[6] + l1 * Q[7] * Q[7] + l2 * Q[8] * Q[8];
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; ++k) h[k] *= scale;
+  }
+  S k0[3][9], k00[9];  // the rows of vertex 0
+#pragma unroll
+  for (int i = 0; i < 9; ++i) k0[0][i] = k0[1][i] = k0[2][i] = k00[i] = S(0);
+#pragma unroll
+  for (int v = 0; v < 3; ++v)
+#pragma unroll
+    for (int w = v; w < 3; ++w) {
+      const S* x = W[v];
+      const S* y = W[w];
+      const S p0 = x[0] * y[0], p1 = x[1] * y[1], p2 = x[2] * y[2];
+      S B[9];
+      B[0] = h[0] * p0 + t[2] * p1 + t[1] * p2;
+      B[4] = t[2] * p0 + h[3] * p1 + t[0] * p2;
+      B[8] = t[1] * p0 + t[0] * p1 + h[5] * p2;
+      const S x01 = x[0] * y[1], x02 = x[0] * y[2], x12 = x[1] * y[2];
+      const S x10 = x[1] * y[0], x20 = x[2] * y[0], x21 = x[2] * y[1];
+      B[1] = h[1] * x01 + f[2] * x10;
+      B[2] = h[2] * x02 + f[1] * x20;
+      B[5] = h[4] * x12 + f[0] * x21;
+      B[3] = h[1] * x10 + f[2] * x01;
+      B[6] = h[2] * x20 + f[1] * x02;
+      B[7] = h[4] * x21 + f[0] * x12;
+      S C[9], K[9];
+      mul33(U, B, C);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j)
+          K[3 * i + j] = v == w && j < i ? K[3 * j + i]
+                                         : C[3 * i] * U[3 * j] + C[3 * i + 1] * U[3 * j + 1] + C[3 * i + 2] * U[3 * j + 2];
+      emit(v + 1, w + 1, K);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          k0[w][3 * i + j] -= K[3 * i + j];
+          if (v != w) k0[v][3 * i + j] -= K[3 * j + i];
+          if (j >= i) k00[3 * i + j] += v != w ? K[3 * i + j] + K[3 * j + i] : K[3 * i + j];
+        }
+    }
+  k00[3] = k00[1];
+  k00[6] = k00[2];
+  k00[7] = k00[5];
+  emit(0, 0, k00);
+#pragma unroll
+  for (int w = 0; w < 3; ++w) emit(0, w + 1, k0[w]);
+}
+
+// the same as the packed upper triangle of the 12x12 matrix (78 entries)
 template <typename S>
 __host__ __device__ __forceinline__ void element_stiffness(const S* F, const S D[4][3], S lam, S mu, bool spsd, S scale,
-                                                  S* K) {
-  S U[9], s[3], V[9];
-  svd3(F, U, s, V);
-  const S I2 = s[0] * s[0] + s[1] * s[1] + s[2] * s[2];
-  const S I3 = s[0] * s[1] * s[2];
-  const S alpha = S(0.75) * mu / lam + S(1);
-  const S a = mu * (S(1) - S(1) / (I2 + S(1)));
-  const S b = mu * (S(2) / ((I2 + S(1)) * (I2 + S(1))));
-  const S c = lam * (I3 - alpha);
-  const S eps = S(1e-3);
-  // W = D V : W[v][j] = sum_l D[v][l] V[l][j]
-  S W[4][3];
+                                                           S* K) {
+  element_stiffness_blocks<S>(F, D, lam, mu, spsd, scale, [&](int v, int w, const S* b) {
 #pragma unroll
-  for (int v = 0; v < 4; ++v)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) W[v][j] = D[v][0] * V[0 * 3 + j] + D[v][1] * V[1 * 3 + j] + D[v][2] * V[2 * 3 + j];
-#pragma unroll
-  for (int i = 0; i < 78; ++i) K[i] = S(0);
-  // twist / flip pairs (i, j) with remaining index k
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    const int i = (m == 0) ? 1 : 0;
-    const int j = (m == 2) ? 1 : 2;
-    const int k = m;
-    S lt = a + c * s[k];
-    S lf = a - c * s[k];
-    if (spsd) {
-      lt = fmax(lt, eps);
-      lf = fmax(lf, eps);
-    }
-    S gt[12], gf[12];
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        const S x = U[d * 3 + i] * W[v][j];
-        const S y = U[d * 3 + j] * W[v][i];
-        gt[v * 3 + d] = x - y;
-        gf[v * 3 + d] = x + y;
-      }
-    rank1(K, S(0.5) * lt * scale, gt);
-    rank1(K, S(0.5) * lf * scale, gf);
-  }
-  // scaling block
-  S A3[9], Q[9];
-  const S g0 = s[1] * s[2], g1 = s[0] * s[2], g2 = s[0] * s[1];
-  A3[0] = a + b * s[0] * s[0] + lam * g0 * g0;
-  A3[4] = a + b * s[1] * s[1] + lam * g1 * g1;
-  A3[8] = a + b * s[2] * s[2] + lam * g2 * g2;
-  A3[1] = A3[3] = b * s[0] * s[1] + lam * g0 * g1 + c * s[2];
-  A3[2] = A3[6] = b * s[0] * s[2] + lam * g0 * g2 + c * s[1];
-  A3[5] = A3[7] = b * s[1] * s[2] + lam * g1 * g2 + c * s[0];
-  sym_eig3(A3, Q);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    S l = A3[m * 4];
-    if (spsd) l = fmax(l, eps);
-    S g[12];
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        g[v * 3 + d] = Q[0 * 3 + m] * U[d * 3 + 0] * W[v][0] + Q[1 * 3 + m] * U[d * 3 + 1] * W[v][1] +
-                       Q[2 * 3 + m] * U[d * 3 + 2] * W[v][2];
-    rank1(K, l * scale, g);
-  }
+      for (int j = 0; j < 3; ++j)
+        if (3 * v + i <= 3 * w + j) K[kup(3 * v + i, 3 * w + j)] = b[3 * i + j];
+  });
 }
 
 }  // namespace ssim_gb

@@ -25,13 +25,13 @@ struct ElemSel<double> {
 };
 
 // K_e = dt^2 V_e pfpx^T H(+) pfpx of tet e (wrapped_pfpx, time_step.hpp:23-60, with the gather weight V_e
-// and alpha = dt^2 of time_step.hpp:646-651 folded in) as the packed upper triangle of the 12 x 12 matrix
-// (row = vertex * 3 + dof).  Positions: X + u in FP64 rounded to S, or the FP32 positions xf (XF).
-template <typename S, bool XF>
-__device__ __forceinline__ void element_hessian_at(const ElemFP64& e64, const ElemFP32& e32,
+// and alpha = dt^2 of time_step.hpp:646-651 folded in): emit(v, w, block) gets each of its ten upper 3x3 vertex blocks
+// (v <= w, row-major) once.  Positions: X + u in FP64 rounded to S, or the FP32 positions xf (XF).
+template <typename S, bool XF, typename EMIT>
+__device__ __forceinline__ void element_hessian_blocks(const ElemFP64& e64, const ElemFP32& e32,
                                                    const double* __restrict__ X, const double* __restrict__ u,
                                                    const float4* __restrict__ xf, S dt2, int spsd, int e,
-                                                   S (&K)[78]) {
+                                                   EMIT&& emit) {
   const int nt = e64.nt;
   const int4 c = e64.cells[e];
   const int vid[4] = {c.x, c.y, c.z, c.w};
@@ -67,12 +67,42 @@ __device__ __forceinline__ void element_hessian_at(const ElemFP64& e64, const El
     D[3][j] = Dm[2 * 3 + j];
     D[0][j] = -(Dm[0 * 3 + j] + Dm[1 * 3 + j] + Dm[2 * 3 + j]);
   }
-  if (e64.model == 1)
-    linear_stiffness<S>(D, ElemSel<S>::lam(e64, e32, e), ElemSel<S>::mu(e64, e32, e), spsd != 0,
-                        dt2 * ElemSel<S>::vol(e64, e32, e), K);
-  else
-    element_stiffness<S>(F, D, ElemSel<S>::lam(e64, e32, e), ElemSel<S>::mu(e64, e32, e), spsd != 0,
-                         dt2 * ElemSel<S>::vol(e64, e32, e), K);
+  const S lam = ElemSel<S>::lam(e64, e32, e), mu = ElemSel<S>::mu(e64, e32, e), sc = dt2 * ElemSel<S>::vol(e64, e32, e);
+  if (e64.model == 1) {
+    S K[78];
+    linear_stiffness<S>(D, lam, mu, spsd != 0, sc, K);
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+      for (int w = v; w < 4; ++w) {
+        S b[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int j = 0; j < 3; ++j) {
+            const int r = 3 * v + i, c = 3 * w + j;
+            b[3 * i + j] = r <= c ? K[kup(r, c)] : K[kup(c, r)];
+          }
+        emit(v, w, b);
+      }
+  } else {
+    element_stiffness_blocks<S>(F, D, lam, mu, spsd != 0, sc, emit);
+  }
+}
+
+// the packed upper triangle of the 12 x 12 matrix (row = vertex * 3 + dof)
+template <typename S, bool XF>
+__device__ __forceinline__ void element_hessian_at(const ElemFP64& e64, const ElemFP32& e32,
+                                                   const double* __restrict__ X, const double* __restrict__ u,
+                                                   const float4* __restrict__ xf, S dt2, int spsd, int e,
+                                                   S (&K)[78]) {
+  element_hessian_blocks<S, XF>(e64, e32, X, u, xf, dt2, spsd, e, [&](int v, int w, const S* b) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        if (3 * v + i <= 3 * w + j) K[kup(3 * v + i, 3 * w + j)] = b[3 * i + j];
+  });
 }
 
 }  // namespace ssim_gb

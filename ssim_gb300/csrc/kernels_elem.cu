@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 
 #include "hessian_elem.cuh"
+#include "topology.h"
 
 namespace ssim_gb {
 
@@ -480,8 +481,10 @@ __global__ void __launch_bounds__(GB)
 // ------------------------------------------------------------------ element Hessian
 // One thread per tet: K_e = dt^2 V_e pfpx^T H+ pfpx (the gather weight V_e and alpha = dt^2 of
 // time_step.hpp:646-651 folded in), written as the 10 upper 3x3 vertex blocks, staged through shared
-// memory so the global writes are contiguous.  Launch bounds of 8 blocks per SM (128 registers, a few
-// spills) beat the unconstrained 168 registers: 168 against 192 us per launch at 1.02M tets.
+// memory so the global writes are contiguous.  Bound by FP32 arithmetic (FP64: by the FP64 units).  The blocks leave
+// as they are formed (element_stiffness_blocks): 96 registers in FP32, 119 with FP16 blocks, 190 in FP64, no spills;
+// with 78 sums held to the end it was 128 and 176 bytes of spills.  1.02M tets, FP16 blocks: 102 us (169 before); 192k
+// tets, FP32 blocks: 21 us (37); FP64, 84,474 tets: 223 us (531), 30,498 tets: 92 us (195).
 // H16 (FP32 arithmetic only): each block written as twelve FP16 words, the nine values scaled by 2^-k and
 // k (the power of two that puts the block's largest magnitude in [2^14, 2^15)) in word 9: 24 bytes a block
 // instead of 36, read back with three 8-byte loads (kernels_sparse.cu assemble_kernel).
@@ -505,38 +508,24 @@ __device__ __forceinline__ void pack_block16(const float* v, uint2* out) {
 }
 
 template <typename S, bool XF, int HB, bool H16 = false>
-__global__ void __launch_bounds__(HB, 512 / HB)
+__global__ void __launch_bounds__(HB, (sizeof(S) == 8 ? 256 : 512) / HB)
     elem_hessian_kernel(ElemFP64 e64, ElemFP32 e32, const double* __restrict__ X, const double* __restrict__ u,
                         const float4* __restrict__ xf, S dt2, int spsd, S* __restrict__ Kbuf) {
-  __shared__ S stage[HB * 90];
+  __shared__ S stage[HB * (H16 ? 60 : 90)];
   const int nt = e64.nt;
   const int e0 = blockIdx.x * HB;
   const int e = e0 + threadIdx.x;
   if (e < nt) {
-    S K[78];
-    element_hessian_at<S, XF>(e64, e32, X, u, xf, dt2, spsd, e, K);
-    int blk = 0;
+    element_hessian_blocks<S, XF>(e64, e32, X, u, xf, dt2, spsd, e, [&](int v, int w, const S* bv) {
+      const int blk = upper_block_id(v, w);
+      if constexpr (H16) {
+        // packed straight from registers: thread t's 30 words at 30 t (the element's global order)
+        pack_block16(bv, reinterpret_cast<uint2*>(stage) + threadIdx.x * 30 + 3 * blk);
+      } else {
 #pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-      for (int w = v; w < 4; ++w) {
-        S bv[9];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-          for (int b = 0; b < 3; ++b) {
-            const int i = v * 3 + a, j = w * 3 + b;
-            bv[a * 3 + b] = (i <= j) ? K[kup(i, j)] : K[kup(j, i)];
-          }
-        if constexpr (H16) {
-          // packed straight from registers: thread t's 30 words at 30 t (the element's global order)
-          pack_block16(bv, reinterpret_cast<uint2*>(stage) + threadIdx.x * 30 + 3 * blk);
-        } else {
-#pragma unroll
-          for (int c = 0; c < 9; ++c) stage[threadIdx.x * 90 + blk * 9 + c] = bv[c];
-        }
-        ++blk;
+        for (int c = 0; c < 9; ++c) stage[threadIdx.x * 90 + blk * 9 + c] = bv[c];
       }
+    });
   }
   __syncthreads();
   const int nvalid = min(HB, nt - e0);

@@ -71,7 +71,7 @@ bool build_full_sell(const Topology& t, std::vector<int32_t>& off, std::vector<i
                      std::vector<int32_t>& src);
 
 // the upper-triangular block id of the local vertex pair (v <= w) used by the element Hessian kernel
-inline int upper_block_id(int v, int w) { return v * 4 - (v * (v - 1)) / 2 + (w - v); }
+constexpr int upper_block_id(int v, int w) { return v * 4 - (v * (v - 1)) / 2 + (w - v); }
 
 // SELL slot of the upper block (u, w), u <= w, w a neighbour of u
 int upper_slot(const Topology& t, int u, int w);
