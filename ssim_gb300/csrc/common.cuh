@@ -75,33 +75,29 @@ struct BlockPartials {
   double v[NV];
 };
 
+// Block sum of FP64 values, result valid in thread 0: every thread stores its values, warp k adds value k (BLOCK / 32
+// per lane, then a shuffle tree).  A tree in every warp costs five additions a warp and value instead of BLOCK / 32 + 5
+// a block, and GB300's FP64 units take a warp's addition every 64 cycles.
 template <int NV, int BLOCK>
 __device__ __forceinline__ void block_sum(double (&vals)[NV], double (*sh)[NV]) {
-  // warp reduce then shared reduce; result valid in thread 0
-  // the NV sums advance level by level together, so their FP64 latency chains overlap (FP64 latency is
-  // long on GB300); each sum's order of additions is that of a per-value tree
+  static_assert(BLOCK / 32 >= NV, "a warp per value");
+  __shared__ double all[NV][BLOCK];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
+  for (int k = 0; k < NV; ++k) all[k][threadIdx.x] = vals[k];
+  __syncthreads();
+  if (warp < NV) {
+    double s = all[warp][lane];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) vals[k] += __shfl_down_sync(0xffffffffu, vals[k], o);
-  }
-  if (lane == 0) {
+    for (int w = 1; w < BLOCK / 32; ++w) s += all[warp][lane + 32 * w];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) sh[warp][k] = vals[k];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) sh[0][warp] = s;
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    double s[NV];
 #pragma unroll
-    for (int k = 0; k < NV; ++k) s[k] = 0;
-#pragma unroll
-    for (int w = 0; w < BLOCK / 32; ++w) {
-#pragma unroll
-      for (int k = 0; k < NV; ++k) s[k] += sh[w][k];
-    }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) vals[k] = s[k];
+    for (int k = 0; k < NV; ++k) vals[k] = sh[0][k];
   }
 }
 

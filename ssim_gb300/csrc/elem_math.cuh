@@ -90,6 +90,34 @@ __host__ __device__ __forceinline__ S snh_eval(const S* F, S lam, S mu, S alpha,
   return S(0.5) * (t1 + t2 - t3) - psi0;
 }
 
+// The same in FP64 with every operation counted (the FP64 element pass is bound by GB300's FP64 units): P times sV
+// (dt^2 V_e, folded into its two factors), and log(I_c + 1) and 1 / (I_c + 1) from the caller's lr(x, rcp).
+template <bool STRESS, typename LR>
+__host__ __device__ __forceinline__ double snh_eval_scaled(const double* F, double lam, double mu, double alpha, double psi0,
+                                                           double sV, double* P, double& scale, LR&& lr) {
+  double Ic = F[0] * F[0];
+#pragma unroll
+  for (int i = 1; i < 9; ++i) Ic += F[i] * F[i];
+  double C[9], J;
+  if (STRESS) {
+    cofactor(F, C);
+    J = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
+  } else {
+    J = det3(F);
+  }
+  const double Jm = J - alpha, lj = lam * Jm;
+  double rcp;
+  const double lg = lr(Ic + 1.0, rcp);
+  if (STRESS) {
+    const double sF = sV * (mu - mu * rcp), sC = sV * lj;
+#pragma unroll
+    for (int i = 0; i < 9; ++i) P[i] = sC * C[i] + sF * F[i];
+  }
+  const double t1 = mu * (Ic - 3.0), t2 = lj * Jm, t3 = mu * lg;
+  scale = 0.5 * (fabs(t1) + t2 + fabs(t3)) + fabs(psi0);
+  return 0.5 * (t1 + t2 - t3) - psi0;
+}
+
 // cof(A + B) - cof(A) - cof(B): the part of the cofactor (quadratic in its argument) bilinear in A and B,
 // for cofactor()'s convention C[k] = F[a] F[b] - F[c] F[d]
 template <typename S>

@@ -154,11 +154,13 @@ __device__ __forceinline__ void precond_rows(const S* a, int precond, V4<S>* out
 // lf[e] = dt^2 V_e * local elastic force + element inertia force M_e (u - x_tilde); energy reduced into
 // sc->energy.  When trial, u is replaced by u + alpha * d and the energy goes to sc->trial_energy (forces
 // at the trial point are written when with_forces: an accepted line-search trial is the next gradient).
+// The energy is complete; the forces lack M_i (u_i (+ alpha d_i) - x~_i), which launch_vertex_gather adds: M_i = rho
+// mnode_i, mnode the sum of V_e / 20 around each vertex (launch_node_mass).
 template <typename SD>
-void launch_elem_energy_grad(const ElemFP64& el, const double* X, const double* u, const double* xt,
-                             const V4<SD>* d, double alpha, double dt2, double rho, double* lf, bool with_forces,
+void launch_elem_energy_grad(const ElemFP64& el, const double* u, const double* xt, const V4<SD>* d, double alpha,
+                             double dt2, double rho, int nv, const double* mnode, double* lf, bool with_forces,
                              bool trial, const Reduce& red, cudaStream_t st);
-// g[v] = sum over incident (e, i) of lf[e][i], Dirichlet dofs zeroed; |g|^2 into sc->gnorm2
+void launch_node_mass(int nv, const int* vptr, const int* vinc, const double* vol, double* mnode, cudaStream_t st);
 // the mixed steppers' FP32 element pass: per-vertex FP32 split of u (hi + lo) and of w = u - x~ (made by
 // launch_split32 once per base point), FP32 element arithmetic, forces to lf32[t][4][3]
 void launch_split32(int nv, const double* u, const double* xt, float4* uh, float4* ul, float4* w, cudaStream_t st);
@@ -201,8 +203,12 @@ void launch_spring_gather32(int nv, const int* vptr, const int* vinc, const floa
 // spring Hessian blocks Kbuf[s][3][9] (scaled by dt^2), the compressed transverse part dropped when spsd
 template <typename S>
 void launch_spring_hessian(const SpringData& sp, const double* u, double dt2, bool spsd, S* Kbuf, cudaStream_t st);
+// g[v] = sum over incident (e, i) of lf[e][i] (+ rho mnode[v] (u (+ alpha d) - x~) with mnode), Dirichlet dofs zeroed;
+// |g|^2 into sc->gnorm2
+template <typename SD>
 void launch_vertex_gather(int nv, const int* vptr, const int* vinc, const double* lf, const uint8_t* mask,
-                          double* g, const Reduce& red, cudaStream_t st);
+                          const double* mnode, double rho, const double* u, const double* xt, const V4<SD>* d,
+                          double alpha, double* g, const Reduce& red, cudaStream_t st);
 
 // ---------------- 2D triangles (kernels_tri.cu) ----------------
 // cells int4 (x, y, z = the triangle), dminv rows 0..3 = the row-major 2x2 Dm^-1, vol = area; local forces

@@ -6,6 +6,7 @@
 #include <cuda_fp16.h>
 
 #include "hessian_elem.cuh"
+#include "log_rcp.cuh"
 #include "topology.h"
 
 namespace ssim_gb {
@@ -29,11 +30,17 @@ __device__ __forceinline__ S comp(const V4<S>& v, int k) {
 // (bilinears.hpp:140-148), (M_e d)_i = rho V_e / 20 (d_i + sum_j d_j) and
 // 1/2 d^T M_e d = rho V_e / 40 (sum_i |d_i|^2 + |sum_i d_i|^2).  Summed over tets this is exactly the
 // unfiltered mass matrix product of time_step.hpp:589-592.
+//
+// Bound by the FP64 units (two lanes an SM and clock; about 300 operations a tet before, 210 now).  The part of the
+// inertia that is diagonal is summed per vertex instead of per element: with m_e = rho V_e / 20 and M_i the sum of m_e
+// around vertex i, 1/2 sum_e m_e sum_i |d_i|^2 = 1/2 sum_i M_i |d_i|^2 (each thread adds its vertices' share of the
+// energy) and the force M_i d_i is added by the vertex gather; the element keeps m_e s, s = sum_j d_j.  The stress
+// leaves snh_eval_scaled times dt^2 V_e.
 template <typename SD, bool FORCES, bool TRIAL>
 __global__ void __launch_bounds__(EB)
-    elem_energy_grad_kernel(ElemFP64 el, const double* __restrict__ X, const double* __restrict__ u,
-                            const double* __restrict__ xt, const V4<SD>* __restrict__ d, double alpha, double dt2,
-                            double rho, double* __restrict__ lf, Reduce red) {
+    elem_energy_grad_kernel(ElemFP64 el, const double* __restrict__ u, const double* __restrict__ xt,
+                            const V4<SD>* __restrict__ d, double alpha, double dt2, double rho, int nv,
+                            const double* __restrict__ mnode, double* __restrict__ lf, Reduce red) {
   __shared__ double stage[FORCES ? EB * 12 : 1];
   __shared__ double shred[EB / 32][2];
   const int e0 = blockIdx.x * EB;
@@ -43,7 +50,7 @@ __global__ void __launch_bounds__(EB)
   if (e < el.nt) {
     const int4 c = el.cells[e];
     const int vid[4] = {c.x, c.y, c.z, c.w};
-    double uu[4][3], dd[4][3];
+    double uu[4][3], sd[3];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       V4<SD> dv;
@@ -53,7 +60,8 @@ __global__ void __launch_bounds__(EB)
         double uk = u[vid[i] * 3 + k];
         if (TRIAL) uk += alpha * (double)comp<SD>(dv, k);
         uu[i][k] = uk;
-        dd[i][k] = uk - xt[vid[i] * 3 + k];
+        const double dd = uk - xt[vid[i] * 3 + k];
+        sd[k] = i == 0 ? dd : sd[k] + dd;
       }
     }
     double Dm[9];
@@ -66,42 +74,62 @@ __global__ void __launch_bounds__(EB)
     for (int r = 0; r < 3; ++r)
 #pragma unroll
       for (int k = 0; k < 3; ++k) Du[r * 3 + k] = uu[k + 1][r] - uu[0][r];
-    double G[9], F[9];  // displacement gradient and F = I + G
+    double G[9];  // displacement gradient
 #pragma unroll
     for (int r = 0; r < 3; ++r)
 #pragma unroll
-      for (int cc = 0; cc < 3; ++cc) {
+      for (int cc = 0; cc < 3; ++cc)
         G[r * 3 + cc] = Du[r * 3 + 0] * Dm[0 * 3 + cc] + Du[r * 3 + 1] * Dm[1 * 3 + cc] + Du[r * 3 + 2] * Dm[2 * 3 + cc];
-        F[r * 3 + cc] = (r == cc ? 1.0 : 0.0) + G[r * 3 + cc];
-      }
     const double lam = el.lam[e], mu = el.mu[e], V = el.vol[e];
-    const double m = rho * V * (1.0 / 20.0);
-    double sd[3];
+    const double m = (rho * (1.0 / 20.0)) * V, sV = dt2 * V;
+    double P[9], sc, psi;
+    if (el.model == 1) {
+      psi = linear_eval<double, FORCES>(G, lam, mu, P, sc);
+      if (FORCES) {
 #pragma unroll
-    for (int k = 0; k < 3; ++k) sd[k] = dd[0][k] + dd[1][k] + dd[2][k] + dd[3][k];
-    double q = sd[0] * sd[0] + sd[1] * sd[1] + sd[2] * sd[2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) q += dd[i][0] * dd[i][0] + dd[i][1] * dd[i][1] + dd[i][2] * dd[i][2];
-    double P[9], sc;
-    const double psi = el.model == 1 ? linear_eval<double, FORCES>(G, lam, mu, P, sc)
-                                     : snh_eval<double, FORCES>(F, lam, mu, el.alpha[e], el.psi0[e], P, sc);
+        for (int k = 0; k < 9; ++k) P[k] *= sV;
+      }
+    } else {
+      G[0] += 1.0;
+      G[4] += 1.0;
+      G[8] += 1.0;
+      psi = snh_eval_scaled<FORCES>(G, lam, mu, el.alpha[e], el.psi0[e], sV, P, sc,
+                                    [](double x, double& rcp) { return log_rcp(x, rcp); });
+    }
     if (FORCES) {
-      const double s = dt2 * V;
-      double tot[3] = {0, 0, 0};
+      double tot[3];
 #pragma unroll
-      for (int i = 1; i < 4; ++i)
+      for (int j = 0; j < 3; ++j) {
+        const double ms = m * sd[j];
 #pragma unroll
-        for (int j = 0; j < 3; ++j) {
+        for (int i = 1; i < 4; ++i) {
           const double h = P[j * 3 + 0] * Dm[(i - 1) * 3 + 0] + P[j * 3 + 1] * Dm[(i - 1) * 3 + 1] +
                            P[j * 3 + 2] * Dm[(i - 1) * 3 + 2];
-          tot[j] += h;
-          lfv[i * 3 + j] = s * h + m * (dd[i][j] + sd[j]);
+          tot[j] = i == 1 ? h : tot[j] + h;
+          lfv[i * 3 + j] = h + ms;
         }
-#pragma unroll
-      for (int j = 0; j < 3; ++j) lfv[j] = -s * tot[j] + m * (dd[0][j] + sd[j]);
+        lfv[j] = ms - tot[j];
+      }
     }
-    energy = dt2 * V * psi + 0.5 * m * q;
-    escale = dt2 * V * sc + 0.5 * m * q;
+    const double q = (0.5 * m) * (sd[0] * sd[0] + sd[1] * sd[1] + sd[2] * sd[2]);
+    energy = sV * psi + q;
+    escale = sV * sc + q;
+  }
+  // the vertices' share of the inertia energy
+  for (int v = e; v < nv; v += gridDim.x * EB) {
+    V4<SD> dv;
+    if (TRIAL) dv = d[v];
+    double q = 0;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double uk = u[(size_t)v * 3 + k];
+      if (TRIAL) uk += alpha * (double)comp<SD>(dv, k);
+      const double dd = uk - xt[(size_t)v * 3 + k];
+      q += dd * dd;
+    }
+    q *= (0.5 * rho) * mnode[v];
+    energy += q;
+    escale += q;
   }
   if (FORCES) {
     if (e < el.nt) {
@@ -125,6 +153,18 @@ __global__ void __launch_bounds__(EB)
       red.sc->energy_scale = tot[1];
     }
   }
+}
+
+// sum over the tets around vertex i of V_e / 20 (M_i over the density)
+__global__ void __launch_bounds__(256)
+    node_mass_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc, const double* __restrict__ vol,
+                     double* __restrict__ mnode) {
+  const int v = blockIdx.x * 256 + threadIdx.x;
+  if (v >= nv) return;
+  double s = 0;
+  const int k1 = vptr[v + 1];
+  for (int k = vptr[v]; k < k1; ++k) s += vol[vinc[k] >> 2];
+  mnode[v] = s * (1.0 / 20.0);
 }
 
 // The same pass with the element arithmetic in FP32 (the mixed steppers' early iterations).  Per vertex,
@@ -370,39 +410,6 @@ __global__ void __launch_bounds__(EB)
   }
 }
 
-// forces as the reference's FP64 forces plus the FP32 local force increments lf32[(e, i)][3] summed per
-// vertex, Dirichlet dofs zeroed; |g|^2 in FP64
-template <int B>
-__global__ void __launch_bounds__(B)
-    vertex_gather_delta32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
-                                 const float* __restrict__ lf32, const uint8_t* __restrict__ mask,
-                                 const double* __restrict__ gref, double* __restrict__ g, Reduce red) {
-  __shared__ double shred[B / 32][1];
-  const int v = blockIdx.x * B + threadIdx.x;
-  double part[1] = {0.0};
-  if (v < nv) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    const int k1 = vptr[v + 1];
-    for (int k = vptr[v]; k < k1; ++k) {
-      const float* s = lf32 + (size_t)vinc[k] * 3;
-      a0 += s[0];
-      a1 += s[1];
-      a2 += s[2];
-    }
-    const uint8_t mk = mask[v];
-    const double g0 = (mk & 1) ? 0.0 : gref[3 * v] + (double)a0;
-    const double g1 = (mk & 2) ? 0.0 : gref[3 * v + 1] + (double)a1;
-    const double g2 = (mk & 4) ? 0.0 : gref[3 * v + 2] + (double)a2;
-    g[3 * v] = g0;
-    g[3 * v + 1] = g1;
-    g[3 * v + 2] = g2;
-    part[0] = g0 * g0 + g1 * g1 + g2 * g2;
-  }
-  block_sum<1, B>(part, shred);
-  double tot[1];
-  if (grid_sum_last<1, B>(part, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
-}
-
 // x_b = u - u_ref per vertex, rounded once to FP32 (the base point of the increment evaluations)
 __global__ void __launch_bounds__(256)
     delta_base_kernel(int nv, const double* __restrict__ u, const double* __restrict__ uref, float4* __restrict__ db) {
@@ -412,32 +419,47 @@ __global__ void __launch_bounds__(256)
                       (float)(u[3 * v + 2] - uref[3 * v + 2]), 0.f);
 }
 
-// forces from FP32 local forces lf32[(e, i)][3], summed per vertex in FP32, Dirichlet dofs zeroed; |g|^2
+constexpr int GB = 256;
+constexpr int GL = 4;  // lanes of a vertex in the force gathers
+
+// the sums of a, b, c over a vertex's GL = 4 lanes: lane q of them ends with component q (lane 3 with nothing); the
+// first exchange splits the values over the lanes, 3 additions instead of 6
+template <typename S>
+__device__ __forceinline__ S quad_sum(S a, S b, S c, int q) {
+  const bool hi = q & 2;
+  S u = hi ? c : a, v = hi ? S(0) : b;
+  u += __shfl_xor_sync(0xffffffffu, hi ? a : c, 2);
+  v += __shfl_xor_sync(0xffffffffu, hi ? b : S(0), 2);
+  const bool odd = q & 1;
+  const S t = odd ? v : u;
+  return t + __shfl_xor_sync(0xffffffffu, odd ? u : v, 1);
+}
+
+// forces from FP32 local forces lf32[(e, i)][3], summed per vertex in FP32 (four lanes a vertex), Dirichlet dofs zeroed;
+// |g|^2
 template <int B>
 __global__ void __launch_bounds__(B)
     vertex_gather32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
                            const float* __restrict__ lf32, const uint8_t* __restrict__ mask, double* __restrict__ g,
                            Reduce red) {
   __shared__ double shred[B / 32][1];
-  const int v = blockIdx.x * B + threadIdx.x;
-  float part[1] = {0.f};
+  const int i = blockIdx.x * B + threadIdx.x, v = i / GL, q = i % GL;
+  float a0 = 0.f, a1 = 0.f, a2 = 0.f, part[1] = {0.f};
   if (v < nv) {
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
     const int k1 = vptr[v + 1];
-    for (int k = vptr[v]; k < k1; ++k) {
+#pragma unroll 2
+    for (int k = vptr[v] + q; k < k1; k += GL) {
       const float* s = lf32 + (size_t)vinc[k] * 3;
       a0 += s[0];
       a1 += s[1];
       a2 += s[2];
     }
-    const uint8_t mk = mask[v];
-    if (mk & 1) a0 = 0.f;
-    if (mk & 2) a1 = 0.f;
-    if (mk & 4) a2 = 0.f;
-    g[3 * v] = a0;
-    g[3 * v + 1] = a1;
-    g[3 * v + 2] = a2;
-    part[0] = a0 * a0 + a1 * a1 + a2 * a2;
+  }
+  float t = quad_sum<float>(a0, a1, a2, q);
+  if (v < nv && q < 3) {
+    if ((mask[v] >> q) & 1) t = 0.f;
+    g[(size_t)v * 3 + q] = t;
+    part[0] = t * t;
   }
   double v1[1];
   block_sum_s<1, B, float>(part, v1, shred);
@@ -445,32 +467,70 @@ __global__ void __launch_bounds__(B)
   if (grid_sum_last<1, B>(v1, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
 }
 
-constexpr int GB = 256;
+// forces as the reference's FP64 forces plus the FP32 local force increments lf32[(e, i)][3] summed per
+// vertex (four lanes a vertex), Dirichlet dofs zeroed; |g|^2 in FP64
+template <int B>
+__global__ void __launch_bounds__(B)
+    vertex_gather_delta32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
+                                 const float* __restrict__ lf32, const uint8_t* __restrict__ mask,
+                                 const double* __restrict__ gref, double* __restrict__ g, Reduce red) {
+  __shared__ double shred[B / 32][1];
+  const int i = blockIdx.x * B + threadIdx.x, v = i / GL, q = i % GL;
+  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+  double part[1] = {0.0};
+  if (v < nv) {
+    const int k1 = vptr[v + 1];
+#pragma unroll 2
+    for (int k = vptr[v] + q; k < k1; k += GL) {
+      const float* s = lf32 + (size_t)vinc[k] * 3;
+      a0 += s[0];
+      a1 += s[1];
+      a2 += s[2];
+    }
+  }
+  const float t = quad_sum<float>(a0, a1, a2, q);
+  if (v < nv && q < 3) {
+    const double gq = ((mask[v] >> q) & 1) ? 0.0 : gref[(size_t)v * 3 + q] + (double)t;
+    g[(size_t)v * 3 + q] = gq;
+    part[0] = gq * gq;
+  }
+  block_sum<1, B>(part, shred);
+  double tot[1];
+  if (grid_sum_last<1, B>(part, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
+}
 
+// Four lanes share a vertex: one lane a vertex walked its 24 incidences as a chain of dependent loads (62 us at 180,285
+// vertices, 12.7 us at 1,331, where nothing else was in flight).  mnode (tets): the force M_i (u_i (+ alpha d_i) - x~_i)
+// that the element pass leaves to the vertices, nullptr otherwise.
+template <typename SD>
 __global__ void __launch_bounds__(GB)
     vertex_gather_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
-                         const double* __restrict__ lf, const uint8_t* __restrict__ mask, double* __restrict__ g,
-                         Reduce red) {
+                         const double* __restrict__ lf, const uint8_t* __restrict__ mask, const double* __restrict__ mnode, double rho,
+                         const double* __restrict__ u, const double* __restrict__ xt, const V4<SD>* __restrict__ d,
+                         double alpha, double* __restrict__ g, Reduce red) {
   __shared__ double shred[GB / 32][1];
-  const int v = blockIdx.x * GB + threadIdx.x;
-  double part = 0;
+  const int i = blockIdx.x * GB + threadIdx.x, v = i / GL, q = i % GL;
+  double a0 = 0, a1 = 0, a2 = 0, part = 0;
   if (v < nv) {
-    double a0 = 0, a1 = 0, a2 = 0;
     const int k1 = vptr[v + 1];
-    for (int k = vptr[v]; k < k1; ++k) {
+#pragma unroll 2
+    for (int k = vptr[v] + q; k < k1; k += GL) {
       const double* s = lf + (size_t)vinc[k] * 3;
       a0 += s[0];
       a1 += s[1];
       a2 += s[2];
     }
-    const uint8_t m = mask[v];  // boundary_condition::grads (boundary.hpp:45-51)
-    if (m & 1) a0 = 0;
-    if (m & 2) a1 = 0;
-    if (m & 4) a2 = 0;
-    g[v * 3 + 0] = a0;
-    g[v * 3 + 1] = a1;
-    g[v * 3 + 2] = a2;
-    part = a0 * a0 + a1 * a1 + a2 * a2;
+  }
+  double t = quad_sum<double>(a0, a1, a2, q);
+  if (v < nv && q < 3) {
+    if (mnode != nullptr) {
+      double x = u[(size_t)v * 3 + q];
+      if (d != nullptr) x += alpha * (double)reinterpret_cast<const SD*>(d + v)[q];
+      t += (rho * mnode[v]) * (x - xt[(size_t)v * 3 + q]);
+    }
+    if ((mask[v] >> q) & 1) t = 0;  // boundary_condition::grads (boundary.hpp:45-51)
+    g[(size_t)v * 3 + q] = t;
+    part = t * t;
   }
   double v1[1] = {part};
   block_sum<1, GB>(v1, shred);
@@ -542,28 +602,28 @@ __global__ void __launch_bounds__(HB, (sizeof(S) == 8 ? 256 : 512) / HB)
 }  // namespace
 
 template <typename SD>
-void launch_elem_energy_grad(const ElemFP64& el, const double* X, const double* u, const double* xt,
-                             const V4<SD>* d, double alpha, double dt2, double rho, double* lf, bool with_forces,
+void launch_elem_energy_grad(const ElemFP64& el, const double* u, const double* xt, const V4<SD>* d, double alpha,
+                             double dt2, double rho, int nv, const double* mnode, double* lf, bool with_forces,
                              bool trial, const Reduce& red, cudaStream_t st) {
   if (el.nt <= 0) return;
   const int grid = div_up(el.nt, EB);
-  if (trial && with_forces) {
-    elem_energy_grad_kernel<SD, true, true><<<grid, EB, 0, st>>>(el, X, u, xt, d, alpha, dt2, rho, lf, red);
-  } else if (trial) {
-    elem_energy_grad_kernel<SD, false, true><<<grid, EB, 0, st>>>(el, X, u, xt, d, alpha, dt2, rho, lf, red);
-  } else if (with_forces) {
-    elem_energy_grad_kernel<SD, true, false><<<grid, EB, 0, st>>>(el, X, u, xt, d, alpha, dt2, rho, lf, red);
-  } else {
-    elem_energy_grad_kernel<SD, false, false><<<grid, EB, 0, st>>>(el, X, u, xt, d, alpha, dt2, rho, lf, red);
-  }
+  auto go = [&](auto fn) { fn<<<grid, EB, 0, st>>>(el, u, xt, d, alpha, dt2, rho, nv, mnode, lf, red); };
+  if (trial && with_forces)
+    go(elem_energy_grad_kernel<SD, true, true>);
+  else if (trial)
+    go(elem_energy_grad_kernel<SD, false, true>);
+  else if (with_forces)
+    go(elem_energy_grad_kernel<SD, true, false>);
+  else
+    go(elem_energy_grad_kernel<SD, false, false>);
   after_launch("elem_energy_grad");
 }
-template void launch_elem_energy_grad<float>(const ElemFP64&, const double*, const double*, const double*,
-                                             const float4*, double, double, double, double*, bool, bool,
-                                             const Reduce&, cudaStream_t);
-template void launch_elem_energy_grad<double>(const ElemFP64&, const double*, const double*, const double*,
-                                              const double4_32a*, double, double, double, double*, bool, bool,
-                                              const Reduce&, cudaStream_t);
+template void launch_elem_energy_grad<float>(const ElemFP64&, const double*, const double*, const float4*, double, double,
+                                             double, int, const double*, double*, bool, bool, const Reduce&,
+                                             cudaStream_t);
+template void launch_elem_energy_grad<double>(const ElemFP64&, const double*, const double*, const double4_32a*, double,
+                                              double, double, int, const double*, double*, bool, bool, const Reduce&,
+                                              cudaStream_t);
 
 void launch_split32(int nv, const double* u, const double* xt, float4* uh, float4* ul, float4* w, cudaStream_t st) {
   if (nv <= 0) return;
@@ -625,7 +685,7 @@ void launch_vertex_gather_delta32(int nv, const int* vptr, const int* vinc, cons
   if (nv <= 0) return;
   auto go = [&](auto B) {
     constexpr int b = decltype(B)::value;
-    vertex_gather_delta32_kernel<b><<<div_up(nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, gref, g, red);
+    vertex_gather_delta32_kernel<b><<<div_up((long long)GL * nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, gref, g, red);
   };
   dispatch_block<128, 256, 512>(block == 0 ? 256 : block, go);
   after_launch("vertex_gather_delta32");
@@ -641,16 +701,30 @@ void launch_vertex_gather32(int nv, const int* vptr, const int* vinc, const floa
   if (nv <= 0) return;
   auto go = [&](auto B) {
     constexpr int b = decltype(B)::value;
-    vertex_gather32_kernel<b><<<div_up(nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, g, red);
+    vertex_gather32_kernel<b><<<div_up((long long)GL * nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, g, red);
   };
   dispatch_block<128, 256, 512>(block == 0 ? 256 : block, go);
   after_launch("vertex_gather32");
 }
+template <typename SD>
 void launch_vertex_gather(int nv, const int* vptr, const int* vinc, const double* lf, const uint8_t* mask,
-                          double* g, const Reduce& red, cudaStream_t st) {
+                          const double* mnode, double rho, const double* u, const double* xt, const V4<SD>* d,
+                          double alpha, double* g, const Reduce& red, cudaStream_t st) {
   if (nv <= 0) return;
-  vertex_gather_kernel<<<div_up(nv, GB), GB, 0, st>>>(nv, vptr, vinc, lf, mask, g, red);
+  vertex_gather_kernel<SD><<<div_up((long long)GL * nv, GB), GB, 0, st>>>(nv, vptr, vinc, lf, mask, mnode, rho, u, xt, d,
+                                                                         alpha, g, red);
   after_launch("vertex_gather");
+}
+template void launch_vertex_gather<float>(int, const int*, const int*, const double*, const uint8_t*, const double*, double,
+                                          const double*, const double*, const float4*, double, double*, const Reduce&,
+                                          cudaStream_t);
+template void launch_vertex_gather<double>(int, const int*, const int*, const double*, const uint8_t*, const double*, double,
+                                           const double*, const double*, const double4_32a*, double, double*,
+                                           const Reduce&, cudaStream_t);
+void launch_node_mass(int nv, const int* vptr, const int* vinc, const double* vol, double* mnode, cudaStream_t st) {
+  if (nv <= 0) return;
+  node_mass_kernel<<<div_up(nv, 256), 256, 0, st>>>(nv, vptr, vinc, vol, mnode);
+  after_launch("node_mass");
 }
 
 template <typename S>

@@ -137,6 +137,7 @@ struct TimeStep {
   DBuf<int4> dcells;
   DBuf<double> dminv, vol, lam, mu, snh_alpha, snh_psi0, snh_delta;
   DBuf<float> fdminv, fvol, flam, fmu;
+  DBuf<double> mnode;  // tets: sum of V_e / 20 around each vertex (the FP64 passes' diagonal inertia)
   DBuf<float> fdelta;  // triangles: the 2D stable Neo-Hookean delta per element in FP32
   // ---- device: state [n] (time_step.hpp:668-679)
   DBuf<double> deformation, prev_deform, inertia, next, velocity, ext_accel, forces, dbc_values, work;
@@ -301,7 +302,7 @@ struct TimeStep {
       launch_tri_energy_grad<S>(e64(), next.p, inertia.p, d, alpha, dt * dt, rho, forces ? lf.p : nullptr, forces,
                                 true, red(), stream);
     else
-      launch_elem_energy_grad<S>(e64(), dX.p, next.p, inertia.p, d, alpha, dt * dt, rho, forces ? lf.p : nullptr,
+      launch_elem_energy_grad<S>(e64(), next.p, inertia.p, d, alpha, dt * dt, rho, nv, mnode.p, forces ? lf.p : nullptr,
                                  forces, true, red(), stream);
   }
   // forces at next (+ alpha d: the point of the last trial pass) from the last pass's local forces,
@@ -320,7 +321,8 @@ struct TimeStep {
     else if (fp32)
       launch_vertex_gather32(nv, vptr.p, vinc.p, lf32t.p, mask.p, forces.p, red(), stream, shapes.gather);
     else
-      launch_vertex_gather(nv, vptr.p, vinc.p, lf.p, mask.p, forces.p, red(), stream);
+      launch_vertex_gather<S>(nv, vptr.p, vinc.p, lf.p, mask.p, tri2d ? nullptr : mnode.p, rho, next.p, inertia.p, d,
+                              alpha, forces.p, red(), stream);
   }
   // mass per upper slot: consistent (tets) or lumped on the diagonal (springs)
   void slot_mass_values(std::vector<double>& smass) {
@@ -423,6 +425,8 @@ struct TimeStep {
     }
     dminv.upload(dm, stream);
     vol.upload(vol_h, stream);
+    mnode.alloc(nv);
+    launch_node_mass(nv, vptr.p, vinc.p, vol.p, mnode.p, stream);
     std::vector<float> f(dm.begin(), dm.end());
     fdminv.upload(f, stream);
     std::vector<float> fv(vol_h.begin(), vol_h.end());
@@ -833,10 +837,10 @@ struct TimeStep {
       launch_tri_energy_grad<double>(e64(), next.p, inertia.p, nullptr, 0.0, dt * dt, rho, lf.p, true, false, red(),
                                      stream);
     else if (mixed())
-      launch_elem_energy_grad<float>(e64(), dX.p, next.p, inertia.p, nullptr, 0.0, dt * dt, rho, lf.p, true, false,
+      launch_elem_energy_grad<float>(e64(), next.p, inertia.p, nullptr, 0.0, dt * dt, rho, nv, mnode.p, lf.p, true, false,
                                      red(), stream);
     else
-      launch_elem_energy_grad<double>(e64(), dX.p, next.p, inertia.p, nullptr, 0.0, dt * dt, rho, lf.p, true, false,
+      launch_elem_energy_grad<double>(e64(), next.p, inertia.p, nullptr, 0.0, dt * dt, rho, nv, mnode.p, lf.p, true, false,
                                       red(), stream);
     if (profiling) prof_end(e0, e1, PK_GRAD, 0);
     gather_forces();
@@ -884,10 +888,10 @@ struct TimeStep {
       launch_tri_energy_grad<double>(e64(), u_dev, inertia.p, sd.tmp.p, 0.0, dt * dt, rho, nullptr, false, true,
                                      red(), stream);
     else if (mixed())
-      launch_elem_energy_grad<float>(e64(), dX.p, u_dev, inertia.p, sf.tmp.p, 0.0, dt * dt, rho, nullptr, false,
+      launch_elem_energy_grad<float>(e64(), u_dev, inertia.p, sf.tmp.p, 0.0, dt * dt, rho, nv, mnode.p, nullptr, false,
                                      true, red(), stream);
     else
-      launch_elem_energy_grad<double>(e64(), dX.p, u_dev, inertia.p, sd.tmp.p, 0.0, dt * dt, rho, nullptr, false,
+      launch_elem_energy_grad<double>(e64(), u_dev, inertia.p, sd.tmp.p, 0.0, dt * dt, rho, nv, mnode.p, nullptr, false,
                                       true, red(), stream);
     sync_scalars();
     return hsc->trial_energy;
