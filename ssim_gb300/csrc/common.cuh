@@ -103,9 +103,15 @@ __device__ __forceinline__ void block_sum(double (&vals)[NV], double (*sh)[NV]) 
 
 // Block sum of per-thread values of type S: the warp-level tree runs in S (FP32 on the mixed path, so the
 // scarce FP64 pipe is not used per element), each warp's sum is widened to FP64 and the warps are added in
-// FP64 in a fixed order.  Result (FP64) valid in thread 0.
+// FP64 in a fixed order.  FP64 values: block_sum.  Result (FP64) valid in thread 0.
 template <int NV, int BLOCK, typename S>
 __device__ __forceinline__ void block_sum_s(const S (&vals)[NV], double (&out)[NV], double (*sh)[NV]) {
+  if constexpr (sizeof(S) == 8) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) out[k] = vals[k];
+    block_sum<NV, BLOCK>(out, sh);
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   S x[NV];
 #pragma unroll

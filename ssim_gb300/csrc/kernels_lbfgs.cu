@@ -139,103 +139,173 @@ __global__ void __launch_bounds__(LB)
 // One pass forms S^T g, Y^T g and the newest pair's column of S^T Y and Y^T Y (all vectors read once); the
 // last block solves the small triangular systems; a second pass forms d = -H g.
 
+// the exchanges of sums of N values (a power of two up to 32) over a warp: each halves the values a lane still carries (N - 1
+// additions instead of 5 N); what is left is summed over the lanes that differ in the bits from 32 / N up and belongs to the
+// value those bits name, lowest first
+template <int N, typename S>
+__device__ __forceinline__ S warp_transpose_sum(const S (&v)[N]) {
+  if constexpr (N == 1) {
+    return v[0];
+  } else {
+    constexpr int o = N / 2;  // values kept; the lanes' distance at this level is 16 for the first one
+    const int lane = threadIdx.x & 31;
+    S w[o];
+    constexpr int dist = N == 32 ? 1 : N == 16 ? 2 : N == 8 ? 4 : N == 4 ? 8 : 16;
+    const bool hi = lane & dist;
+#pragma unroll
+    for (int k = 0; k < o; ++k) {
+      const S keep = hi ? v[2 * k + 1] : v[2 * k], give = hi ? v[2 * k] : v[2 * k + 1];
+      w[k] = keep + __shfl_xor_sync(0xffffffffu, give, dist);
+    }
+    return warp_transpose_sum<o, S>(w);
+  }
+}
+
 // per vertex: a_j = s_j.g, b_j = y_j.g, c_j = s_j.y_new, e_j = y_j.y_new (j in age order, oldest first);
-// the last block keeps the new column in the slot-indexed S^T Y / Y^T Y tables and writes the coefficients
-template <typename S>
+// the last block keeps the new column in the slot-indexed S^T Y / Y^T Y tables and writes the coefficients.
+// PG warps share 32 vertices, each taking 8 / PG of the pairs: 1 for large systems, 4 where the vertices are too few to
+// occupy the SMs otherwise (in FP64 a thread's 96 products then cost 24).  In FP64 the kernel is bound by the FP64 units
+// (a warp's operation every 64 cycles): the 32 sums take 31 additions a warp instead of 160, and the small triangular
+// systems are solved by eight lanes with the diagonal's reciprocals instead of by one thread with 16 divisions.
+// 9,225 vertices, FP64: 10.5 us (38.4 before).
+template <typename S, int PG>
 __global__ void __launch_bounds__(LB)
     lbfgs_multidot_kernel(int nv, const double* __restrict__ g, LbfgsHist<S> h, double* __restrict__ partials,
                           double* __restrict__ tab, unsigned int* counter) {
-  constexpr int NV = 4 * kLbfgsMaxCompact;
-  static_assert(LB % NV == 0 && LB / NV <= LB / 32, "the last block's group sums reuse the warp-sum table");
+  constexpr int NV = 4 * kLbfgsMaxCompact, NP = kLbfgsMaxCompact / PG, NA = 4 * NP;
+  constexpr int VB = LB / PG;  // vertices of a block at a time
+  static_assert(NV == 32 && LB % NV == 0, "a lane per value");
   __shared__ double shred[LB / 32][NV];
-  __shared__ double tot[NV];
   __shared__ bool am_last;
-  S acc[NV];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, pg = warp % PG;
+  S acc[NA];
 #pragma unroll
-  for (int k = 0; k < NV; ++k) acc[k] = S(0);
+  for (int k = 0; k < NA; ++k) acc[k] = S(0);
   // a grid of a few blocks per SM striding over the vertices: the block sums and the last block's sum
   // over the grid (NV values per block) stay short
-  for (int u = blockIdx.x * LB + threadIdx.x; u < nv; u += gridDim.x * LB) {
+  for (int u = blockIdx.x * VB + 32 * (warp / PG) + lane; u < nv; u += gridDim.x * VB) {
     const V4<S> gv = mk4<S>((S)g[3 * u], (S)g[3 * u + 1], (S)g[3 * u + 2]);
     const V4<S> yn = h.y[h.n - 1][u];
 #pragma unroll
-    for (int j = 0; j < kLbfgsMaxCompact; ++j) {
+    for (int i = 0; i < NP; ++i) {
+      const int j = NP * pg + i;
       if (j < h.n) {
         const V4<S> sv = h.s[j][u], yv = h.y[j][u];
-        acc[4 * j + 0] += dot3<S>(sv, gv);
-        acc[4 * j + 1] += dot3<S>(yv, gv);
-        acc[4 * j + 2] += dot3<S>(sv, yn);
-        acc[4 * j + 3] += dot3<S>(yv, yn);
+        acc[4 * i + 0] += dot3<S>(sv, gv);
+        acc[4 * i + 1] += dot3<S>(yv, gv);
+        acc[4 * i + 2] += dot3<S>(sv, yn);
+        acc[4 * i + 3] += dot3<S>(yv, yn);
       }
     }
   }
   // block sums (FP32 within a warp, FP64 across warps), then the grid sum in FP64 by the last block
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  {
+    S x = warp_transpose_sum<NA, S>(acc);
 #pragma unroll
-  for (int k = 0; k < NV; ++k) {
-    S x = acc[k];
+    for (int o = 16 / NA; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    // the lanes' bits, lowest distance first, name the value: level by level the low bit of the index
+    int k = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) shred[warp][k] = (double)x;
+    for (int b = 0; (1 << b) < NA; ++b) {
+      constexpr int first = NA == 32 ? 0 : NA == 16 ? 1 : 2;
+      k |= ((lane >> (first + b)) & 1) << b;
+    }
+    if (NA == 32 || (lane & ((32 / NA) - 1)) == 0) shred[warp][NA * pg + k] = (double)x;
   }
   __syncthreads();
   if (threadIdx.x < NV) {
     double b = 0;
+    const int own = threadIdx.x / NA;  // the warps that carry this value
 #pragma unroll
-    for (int w = 0; w < LB / 32; ++w) b += shred[w][threadIdx.x];
+    for (int w = 0; w < LB / 32 / PG; ++w) b += shred[PG * w + own][threadIdx.x];
     partials[(size_t)blockIdx.x * NV + threadIdx.x] = b;
   }
   __syncthreads();  // orders the partials before thread 0's release
   if (threadIdx.x == 0) am_last = (atom_inc_acq_rel_gpu(counter) == gridDim.x - 1);
   __syncthreads();
   if (!am_last) return;
-  {  // LB / NV groups of threads each sum every (LB / NV)-th block's partials, then the groups in order
+  // LB / NV groups of threads each sum every (LB / NV)-th block's partials (four chains), then the groups in order
+  double tot = 0;  // lane k of warp 0: value k
+  {
     constexpr int G = LB / NV;
     const int k = threadIdx.x % NV, grp = threadIdx.x / NV;
-    double t = 0;
-    for (int b = grp; b < (int)gridDim.x; b += G) t += __ldcg(partials + (size_t)b * NV + k);
-    shred[grp][k] = t;
-    __syncthreads();
-    if (threadIdx.x < NV) {
-      double a = 0;
+    double t[4] = {0, 0, 0, 0};
+    for (int b = grp; b < (int)gridDim.x; b += 4 * G) {
+      double v[4];
 #pragma unroll
-      for (int q = 0; q < G; ++q) a += shred[q][threadIdx.x];
-      tot[threadIdx.x] = a;
+      for (int i = 0; i < 4; ++i) v[i] = b + i * G < (int)gridDim.x ? __ldcg(partials + (size_t)(b + i * G) * NV + k) : 0.0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (b + i * G < (int)gridDim.x) t[i] += v[i];
     }
+    shred[grp][k] = (t[0] + t[1]) + (t[2] + t[3]);
+    __syncthreads();
+    if (threadIdx.x >= NV) return;
+#pragma unroll
+    for (int q = 0; q < G; ++q) tot += shred[q][threadIdx.x];
   }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  *counter = 0;
+  if (threadIdx.x == 0) *counter = 0;
   // tables: tab[0 .. M*M) = S^T Y by slot (row s-slot, column y-slot), tab[M*M .. 2 M*M) = Y^T Y by slot;
-  // coefficients written to tab[2 M*M ..): p (age order), q (age order), gamma
+  // coefficients written to tab[2 M*M ..): p (age order), q (age order), gamma.  Lane j < n works on row j.
   constexpr int M = kLbfgsMaxCompact;
   double* SY = tab;
   double* YY = tab + M * M;
   double* out = tab + 2 * M * M;
-  const int n = h.n, sn = h.slot[n - 1];
-  for (int j = 0; j < n; ++j) {
-    SY[h.slot[j] * M + sn] = tot[4 * j + 2];
-    YY[h.slot[j] * M + sn] = tot[4 * j + 3];
-    YY[sn * M + h.slot[j]] = tot[4 * j + 3];
+  const int n = h.n, sn = h.slot[n - 1], j = lane < n ? lane : n - 1;
+  int sj = 0;
+#pragma unroll
+  for (int i = 0; i < M; ++i) sj = i == j ? h.slot[i] : sj;
+  const double aj = __shfl_sync(0xffffffffu, tot, 4 * j), bj = __shfl_sync(0xffffffffu, tot, 4 * j + 1);
+  const double cj = __shfl_sync(0xffffffffu, tot, 4 * j + 2), ej = __shfl_sync(0xffffffffu, tot, 4 * j + 3);
+  if (lane < n) {
+    SY[sj * M + sn] = cj;
+    YY[sj * M + sn] = ej;
+    YY[sn * M + sj] = ej;
   }
-  const double gamma = SY[sn * M + sn] / YY[sn * M + sn];
-  double q[M], p[M];
-  for (int j = n - 1; j >= 0; --j) {  // R q = a, R[j][k] = s_j.y_k (k >= j)
-    double r = tot[4 * j + 0];
-    for (int k = j + 1; k < n; ++k) r -= SY[h.slot[j] * M + h.slot[k]] * q[k];
-    q[j] = r / SY[h.slot[j] * M + h.slot[j]];
+  __syncwarp();
+  double sy[M], yy[M], syt[M];  // row j of S^T Y and Y^T Y, column j of S^T Y, in age order
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    const bool in = i < n;
+    const int si = h.slot[i];
+    sy[i] = in ? SY[sj * M + si] : 0.0;
+    syt[i] = in ? SY[si * M + sj] : 0.0;
+    yy[i] = in ? YY[sj * M + si] : 0.0;
   }
-  for (int j = 0; j < n; ++j) {  // t = (D + gamma Y^T Y) q - gamma b, then R^T p = t
-    double t = SY[h.slot[j] * M + h.slot[j]] * q[j] - gamma * tot[4 * j + 1];
-    for (int k = 0; k < n; ++k) t += gamma * YY[h.slot[j] * M + h.slot[k]] * q[k];
-    for (int k = 0; k < j; ++k) t -= SY[h.slot[k] * M + h.slot[j]] * p[k];
-    p[j] = t / SY[h.slot[j] * M + h.slot[j]];
+  double djj = 0, dyy = 0;
+#pragma unroll
+  for (int i = 0; i < M; ++i) {
+    djj = i == j ? sy[i] : djj;
+    dyy = i == j ? yy[i] : dyy;
   }
-  for (int j = 0; j < n; ++j) {
-    out[j] = p[j];
-    out[M + j] = -gamma * q[j];
+  const double inv = 1.0 / djj;
+  const double gamma = __shfl_sync(0xffffffffu, djj / dyy, n - 1);
+  // R q = a, R[j][k] = s_j.y_k (k >= j): the newest first, each solved value leaving the rows before it
+  double r = aj, q = 0, t = -gamma * bj;
+#pragma unroll
+  for (int k = M - 1; k >= 0; --k) {
+    if (k < n) {
+      const double qk = __shfl_sync(0xffffffffu, r * inv, k);
+      if (j == k) q = qk;
+      if (j < k) r -= sy[k] * qk;
+      t += gamma * yy[k] * qk;  // t = (D + gamma Y^T Y) q - gamma b, less the diagonal
+    }
   }
-  out[2 * M] = gamma;
+  t += djj * q;
+  double p = 0;  // R^T p = t, the oldest first
+#pragma unroll
+  for (int k = 0; k < M; ++k) {
+    if (k < n) {
+      const double pk = __shfl_sync(0xffffffffu, t * inv, k);
+      if (j == k) p = pk;
+      if (j > k) t -= syt[k] * pk;
+    }
+  }
+  if (lane < n) {
+    out[j] = p;
+    out[M + j] = -gamma * q;
+  }
+  if (lane == 0) out[2 * M] = gamma;
 }
 
 // d = -(gamma g + sum_j p_j s_j + sum_j q'_j y_j) (coefficients from the multidot pass; gamma_host when
@@ -285,18 +355,27 @@ __global__ void __launch_bounds__(LB)
 
 }  // namespace
 
-// 2 blocks per SM (each thread then sums several vertices in FP32 before the block sums)
-int multidot_grid(int nv) {
+// 2 blocks per SM (each thread then sums several vertices in FP32 before the block sums); with four warps to 32 vertices
+// where blocks of 64 vertices are no more than that
+constexpr int kMultidotGroups = 4;
+static void multidot_shape(int nv, int& grid, int& groups) {
   int dev = 0, nsm = 0;
   SSIM_CUDA(cudaGetDevice(&dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  return std::max(1, std::min(div_up(nv, LB), 2 * std::max(nsm, 1)));
+  const int most = 2 * std::max(nsm, 1), small = div_up(nv, LB / kMultidotGroups);
+  groups = small <= most ? kMultidotGroups : 1;
+  grid = groups == 1 ? std::max(1, std::min(div_up(nv, LB), most)) : std::max(1, small);
 }
 
 template <typename S>
 void launch_lbfgs_multidot(int nv, const double* g, const LbfgsHist<S>& h, double* partials, double* tab,
                            unsigned int* counter, cudaStream_t st) {
-  lbfgs_multidot_kernel<S><<<multidot_grid(nv), LB, 0, st>>>(nv, g, h, partials, tab, counter);
+  int grid, groups;
+  multidot_shape(nv, grid, groups);
+  if (groups == 1)
+    lbfgs_multidot_kernel<S, 1><<<grid, LB, 0, st>>>(nv, g, h, partials, tab, counter);
+  else
+    lbfgs_multidot_kernel<S, kMultidotGroups><<<grid, LB, 0, st>>>(nv, g, h, partials, tab, counter);
   after_launch("lbfgs_multidot");
 }
 
@@ -307,7 +386,11 @@ void launch_lbfgs_combine(int nv, const double* g, const LbfgsHist<S>& h, const 
   after_launch("lbfgs_combine");
 }
 
-int lbfgs_multidot_partials(int nv) { return div_up(nv, LB) * 4 * kLbfgsMaxCompact; }
+int lbfgs_multidot_partials(int nv) {
+  int grid, groups;
+  multidot_shape(nv, grid, groups);
+  return grid * 4 * kLbfgsMaxCompact;
+}
 
 template <typename S>
 void launch_lbfgs_pass(int nv, const V4<S>* vin, const double* g, V4<S>* vout, const V4<S>* w, const double* cA,
