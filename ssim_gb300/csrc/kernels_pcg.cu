@@ -144,19 +144,84 @@ __device__ __forceinline__ bool exchange_barrier(const GridExchange& gx, unsigne
   return exchange_wait<float, 0>(gx, k, nullptr, 0, 0, xs);
 }
 
+// The scalars of a solve, one copy per block (the same bits in each): Chronopoulos-Gear's
+//   beta = g / g_old,  den = d - beta g / alpha_old,  alpha = g / den   (first: 0, d, g / d)
+// from g = (r, u), d = (w, u), with the reciprocals of the last step kept: ig = 1 / g_old, c = ig / alpha_old.
+struct Scalars {
+  double ig, c, g, den, rr, rr0, tol2, alpha, beta;
+  int iters, done, status;
+};
+
+__device__ __forceinline__ bool positive(double x) {  // x > 0, by its bits (a comparison costs the FP64 unit 64 cycles)
+  const long long b = __double_as_longlong(x);
+  return b > 0 && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ bool is_zero(double x) { return (__double_as_longlong(x) << 1) == 0; }
+__device__ __forceinline__ bool is_finite(double x) {
+  return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff;
+}
+
+// one thread, after the dots: stop tests on the residual of the current x (first: relative to this one), then the step
+// lengths.  rr and tol2 are not negative, so they compare as integers.  FP32STEP: alpha and beta are used in FP32, so a
+// reciprocal to 2^-45 (FP32's, improved by one Newton step) is enough for alpha.  This chain is what a small system's
+// iteration waits for: about 700 cycles against 2,000 with comparisons, two divisions and the next step's reciprocals.
+template <bool FP32STEP>
+__device__ __forceinline__ void step_scalars(Scalars& s, bool first, double g, double d, double rr, double rtol,
+                                             int max_iters) {
+  if (first) {
+    s.rr0 = rr;
+    s.tol2 = rtol * rtol * rr;
+    s.iters = s.done = s.status = 0;
+    s.alpha = s.beta = 0.0;
+  }
+  s.rr = rr;
+  if (!is_finite(rr)) {
+    s.done = 1;
+    s.status = 2;
+    return;
+  }
+  if (__double_as_longlong(rr) <= __double_as_longlong(s.tol2) || is_zero(g) || s.iters >= max_iters) {
+    s.done = 1;
+    return;
+  }
+  double den = d;
+  if (s.iters > 0) den = fma(-(g * g), s.c, d);
+  if (!positive(den)) {  // breakdown: not SPD along p (or non-finite)
+    s.done = 1;
+    s.status = 1;
+    return;
+  }
+  if constexpr (FP32STEP) {
+    const float df = (float)den;
+    if (df > 1e-30f && df < 1e30f) {
+      const double r = (double)(1.f / df);
+      s.alpha = g * fma(r, fma(-den, r, 1.0), r);
+    } else {
+      s.alpha = g / den;
+    }
+  } else {
+    s.alpha = g / den;
+  }
+  s.beta = s.iters > 0 ? g * s.ig : 0.0;
+  s.g = g;
+  s.den = den;
+  s.iters += 1;
+}
+// one thread, any time before the next step_scalars: the reciprocals it will use
+__device__ __forceinline__ void next_reciprocals(Scalars& s) {
+  s.ig = 1.0 / s.g;
+  s.c = s.den * s.ig * s.ig;
+}
 // the solve's scalars for the host
-__device__ __forceinline__ void publish_scalars(const DevScalars& sc, DevScalars* o) {
-  o->rz = sc.rz;
-  o->rz_old = sc.rz_old;
-  o->pq = sc.pq;
-  o->rr = sc.rr;
-  o->rr0 = sc.rr0;
-  o->tol2 = sc.tol2;
-  o->alpha = sc.alpha;
-  o->beta = sc.beta;
-  o->iters = sc.iters;
-  o->done = sc.done;
-  o->status = sc.status;
+__device__ __forceinline__ void publish_scalars(const Scalars& s, DevScalars* o) {
+  o->rr = s.rr;
+  o->rr0 = s.rr0;
+  o->tol2 = s.tol2;
+  o->alpha = s.alpha;
+  o->beta = s.beta;
+  o->iters = s.iters;
+  o->done = s.done;
+  o->status = s.status;
 }
 
 // One unit of y = A x on the symmetric store: slice s's upper slots part, part + T, ... and lower slots
@@ -295,7 +360,7 @@ __global__ void __launch_bounds__(HT, 1)
                          float4* sv, float4* w, float4* m, HalfSolveArgs a, HalfPlan pl, Reduce red, GridExchange gx) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ExchangeShared xs;
-  __shared__ DevScalars sc;
+  __shared__ Scalars sc;
   __shared__ float s_ab[2];  // alpha, beta
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nv = H.nv, nsl = (nv + 31) >> 5;
@@ -476,16 +541,7 @@ __global__ void __launch_bounds__(HT, 1)
     ok = exchange_wait<float, 3>(gx, nx, shw, pl.spc, ns, xs);
     if (!ok) break;
     exchange_total<3>(gx, nx++, xs, [&](const double(&t)[3]) {
-      if (first) {  // the stop test is relative to this residual
-        sc.done = 0;
-        sc.rz_old = 1.0;
-        sc.rr0 = t[2];
-        sc.tol2 = a.rtol * a.rtol * t[2];
-        sc.iters = 0;
-        sc.status = 0;
-        sc.alpha = sc.beta = 0.0;
-      }
-      cgcg_after(&sc, t[0], t[1], t[2], a.max_iters);
+      step_scalars<true>(sc, first, t[0], t[1], t[2], a.rtol, a.max_iters);
       s_ab[0] = (float)sc.alpha;
       s_ab[1] = (float)sc.beta;
     });
@@ -496,6 +552,7 @@ __global__ void __launch_bounds__(HT, 1)
     if (pipe) spmv(mk, 0, min(ns, pl.tile));
     __syncthreads();
     if (sc.done) break;
+    if (tid == HT - 32) next_reciprocals(sc);
     const float alpha = s_ab[0], beta = s_ab[1];
     if (!pipe) {
       // Chronopoulos-Gear: p = u + beta p, s = w + beta s, x += alpha p, r -= alpha s, u = M r; then w = A u
@@ -673,7 +730,7 @@ __global__ void __launch_bounds__(DT, 1)
                       double4_32a* m, Solve64Args a, Plan64 pl, Reduce red, GridExchange gx) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ ExchangeShared xs;
-  __shared__ DevScalars sc;
+  __shared__ Scalars sc;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nv = A.nv, nsl = (nv + 31) >> 5;
   const int s0 = (int)((long long)blockIdx.x * nsl / gridDim.x), ns = (int)((long long)(blockIdx.x + 1) * nsl / gridDim.x) - s0;
@@ -820,16 +877,7 @@ __global__ void __launch_bounds__(DT, 1)
     ok = exchange_wait<double, 3>(gx, nx, sh, DT, np, xs);
     if (!ok) break;
     exchange_total<3>(gx, nx++, xs, [&](const double(&t)[3]) {
-      if (first) {  // the stop test is relative to this residual
-        sc.done = 0;
-        sc.rz_old = 1.0;
-        sc.rr0 = t[2];
-        sc.tol2 = a.rtol * a.rtol * t[2];
-        sc.iters = 0;
-        sc.status = 0;
-        sc.alpha = sc.beta = 0.0;
-      }
-      cgcg_after(&sc, t[0], t[1], t[2], a.max_iters);
+      step_scalars<false>(sc, first, t[0], t[1], t[2], a.rtol, a.max_iters);
     });
     const bool pipe = k < a.pipe_iters;
     const double4_32a* mk = m + (size_t)(k & 1) * nv;
@@ -837,6 +885,7 @@ __global__ void __launch_bounds__(DT, 1)
     if (pipe) spmv(mk);  // n = A m while the scalars are made
     __syncthreads();
     if (sc.done) break;
+    if (tid == DT - 32) next_reciprocals(sc);
     const double alpha = sc.alpha, beta = sc.beta;
     double d0 = 0, d1 = 0, d2 = 0;
     for (int j = tid; j < nd; j += DT) {
