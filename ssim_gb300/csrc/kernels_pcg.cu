@@ -280,6 +280,7 @@ __device__ __forceinline__ void sym_unit(const SellMatrix& A, const S* __restric
 struct HalfPlan {
   int grid, T, spc, res, tile, cached;  // spc: most slices of a block; res, tile in slices
   int cache_entries;                    // most entries of a block (when cached)
+  int keep;                             // slices whose entries L2 is asked to keep; -1: no hints
   size_t smem;
 };
 
@@ -296,13 +297,47 @@ __device__ __forceinline__ void half_fma(const uint4& p, uint16_t h8, const floa
   a2 = fmaf(f8, xv.z, fmaf(f67.y, xv.y, fmaf(f67.x, xv.x, a2)));
 }
 
+// loads with an L2 replacement priority (HINT), or plain ones
+template <bool HINT>
+__device__ __forceinline__ uint4 ld_hint(const uint4* p, unsigned long long pol) {
+  if constexpr (HINT) {
+    uint4 v;
+    asm("ld.global.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+        : "l"(p), "l"(pol));
+    return v;
+  } else {
+    return *p;
+  }
+}
+template <bool HINT>
+__device__ __forceinline__ uint16_t ld_hint(const uint16_t* p, unsigned long long pol) {
+  if constexpr (HINT) {
+    uint16_t v;
+    asm("ld.global.L2::cache_hint.u16 %0, [%1], %2;" : "=h"(v) : "l"(p), "l"(pol));
+    return v;
+  } else {
+    return *p;
+  }
+}
+template <bool HINT>
+__device__ __forceinline__ int ld_hint(const int* p, unsigned long long pol) {
+  if constexpr (HINT) {
+    int v;
+    asm("ld.global.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(pol));
+    return v;
+  } else {
+    return *p;
+  }
+}
+
 // Entries k0, k0 + T, ... of a slice of width W (col / v8 / v1: its first entry, this lane): four at a time with all
 // their loads in flight.  The kernel is bound by the instructions it issues (59% of the issue slots in a first
 // version with run-time strides and a predicate per entry), so T is a compile-time stride (immediate offsets) and
 // only a unit's ragged end tests the width.
-template <int T>
+template <int T, bool HINT>
 __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const uint16_t* v1, int W, int k0,
-                                          const float4* x, float& a0, float& a1, float& a2) {
+                                          const float4* x, unsigned long long pol, float& a0, float& a1, float& a2) {
   col += 32 * k0;
   v8 += 32 * k0;
   v1 += 32 * k0;
@@ -313,11 +348,11 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
     uint16_t h[4];
     float4 xv[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) c[j] = col[32 * T * j];
+    for (int j = 0; j < 4; ++j) c[j] = ld_hint<HINT>(col + 32 * T * j, pol);
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      p[j] = v8[32 * T * j];
-      h[j] = v1[32 * T * j];
+      p[j] = ld_hint<HINT>(v8 + 32 * T * j, pol);
+      h[j] = ld_hint<HINT>(v1 + 32 * T * j, pol);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) xv[j] = x[c[j]];
@@ -329,9 +364,9 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
   }
   if (n > 0) {  // one to three entries: the missing ones repeat the first with a zero vector
     const int o1 = n > T ? 32 * T : 0, o2 = n > 2 * T ? 64 * T : 0;
-    const int c0 = col[0], c1 = col[o1], c2 = col[o2];
-    const uint4 p0 = v8[0], p1 = v8[o1], p2 = v8[o2];
-    const uint16_t h0 = v1[0], h1 = v1[o1], h2 = v1[o2];
+    const int c0 = ld_hint<HINT>(col, pol), c1 = ld_hint<HINT>(col + o1, pol), c2 = ld_hint<HINT>(col + o2, pol);
+    const uint4 p0 = ld_hint<HINT>(v8, pol), p1 = ld_hint<HINT>(v8 + o1, pol), p2 = ld_hint<HINT>(v8 + o2, pol);
+    const uint16_t h0 = ld_hint<HINT>(v1, pol), h1 = ld_hint<HINT>(v1 + o1, pol), h2 = ld_hint<HINT>(v1 + o2, pol);
     const float4 x0 = x[c0];
     float4 x1 = x[c1], x2 = x[c2];
     if (n <= T) x1 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -353,8 +388,8 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
 // rule are Chronopoulos-Gear's; the third dot is (r, r) of the unscaled residual.  In FP32 the recursive residual
 // drifts from the true one with the iterations and the condition number, so after pipe_iters iterations the
 // solve continues as Chronopoulos-Gear PCG from the same state (w = A u recomputed, two exchanges a round).
-// CACHED: the block's matrix entries are in shared memory too.
-template <bool CACHED, int T>
+// CACHED: the block's matrix entries are in shared memory too.  HINT: they are loaded with L2 priorities (pl.keep).
+template <bool CACHED, int T, bool HINT = false>
 __global__ void __launch_bounds__(HT, 1)
     resident_half_kernel(HalfMatrix H, const float4* __restrict__ dinv, float4* x, float4* r, float4* z, float4* p,
                          float4* sv, float4* w, float4* m, HalfSolveArgs a, HalfPlan pl, Reduce red, GridExchange gx) {
@@ -389,6 +424,11 @@ __global__ void __launch_bounds__(HT, 1)
     }
   }
   unsigned long long nx = 0;  // exchanges so far
+  unsigned long long pol_keep = 0, pol_pass = 0;
+  if constexpr (HINT) {
+    asm volatile("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol_keep));
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol_pass));
+  }
 
   // products of the slices t0 .. t1 - 1 into the unit partials
   auto spmv = [&](const float4* v, int t0, int t1) {
@@ -398,9 +438,11 @@ __global__ void __launch_bounds__(HT, 1)
       const int b = off[t0 + (i >> lt)], W = (off[t0 + (i >> lt) + 1] - b) >> 5;
       float a0 = 0.f, a1 = 0.f, a2 = 0.f;
       if constexpr (CACHED)
-        half_unit<T>(ccol + (b - e0) + lane, c8 + (b - e0) + lane, c1 + (b - e0) + lane, W, i & (T - 1), v, a0, a1, a2);
+        half_unit<T, false>(ccol + (b - e0) + lane, c8 + (b - e0) + lane, c1 + (b - e0) + lane, W, i & (T - 1), v, 0, a0, a1,
+                            a2);
       else
-        half_unit<T>(H.col + b + lane, H.v8 + b + lane, H.v1 + b + lane, W, i & (T - 1), v, a0, a1, a2);
+        half_unit<T, HINT>(H.col + b + lane, H.v8 + b + lane, H.v1 + b + lane, W, i & (T - 1), v,
+                           t0 + (i >> lt) < pl.keep ? pol_keep : pol_pass, a0, a1, a2);
       float* o = pb + (size_t)3 * (i & (T - 1)) * PR + 32 * (i >> lt) + lane;
       o[0] = a0;
       o[PR] = a1;
@@ -987,6 +1029,15 @@ static GridExchange grid_exchange(const ResidentSync& rs, cudaStream_t st) {
                       (unsigned int)rs.extra, rs.spin_limit > 0 ? rs.spin_limit : (1LL << 21)};
 }
 
+// 22 bytes an entry against the double-buffered m and the vectors of the rows that are not on chip
+static HalfPlan l2_hints(HalfPlan p, int nv, const int32_t* off, size_t l2) {
+  const double matrix = 22.0 * off[div_up(nv, 32)];
+  const double other = 32.0 * nv + 176.0 * nv * (p.spc - p.res) / std::max(p.spc, 1);
+  if (p.grid > 0 && matrix + other > 0.8 * (double)l2)
+    p.keep = (int)(p.spc * std::min(1.0, std::max(0.0, 0.6 * (double)l2 - other) / matrix));
+  return p;
+}
+
 // Layout of a resident solve on the FP16 copy (host arithmetic only; off: the copy's slice offsets).
 //  T: 4 warps a slice (a 15-entry slice is four entries a unit: all of a unit's loads in flight at once), 8 where a
 //  block has fewer than 8 slices (small systems: fewer dependent rounds).
@@ -994,8 +1045,14 @@ static GridExchange grid_exchange(const ResidentSync& rs, cudaStream_t st) {
 //  block, 219,000 rows on 152 SMs); beyond, passes of 32 slices and the rows that fit.  The matrix entries too
 //  where the block's part of them fits (about 70,000 rows): an iteration then reads nothing but the gathered
 //  vector from L2.
-static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, int max_blocks) {
+//  L2 hints where what an iteration cycles through does not fit: swept in order, an LRU-like cache then keeps nothing.
+//  The entries of the first slices of every block are loaded with evict_last, the others with evict_first.  Measured on
+//  batches of cubes, 126 MB of L2 (matrix / other bytes, MB; Newton iterations, ms): 77 / 8 6.43 without and 6.77 with
+//  60 MB kept; 92 / 17 10.1, 8.87 with 60; 108 / 28 15.1, 12.9 with 50; 118 / 35 18.0, 15.4 with 40; 157 / 60 22.7, 20.3
+//  with 20; 250 / 122 36.9, 36.6.  So: hints above 0.8 of L2, 0.6 of L2 less the other bytes kept.
+static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, size_t l2, int max_blocks) {
   HalfPlan p{};
+  p.keep = -1;
   const int nsl = div_up(nv, 32);
   p.grid = std::max(1, std::min(std::min(nsm, kMaxBlocks), nsl));
   if (max_blocks > 0) p.grid = std::min(p.grid, max_blocks);
@@ -1009,24 +1066,26 @@ static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, 
     const size_t row = (size_t)4 * kHalfState * 32;
     p.res = base < smem_max ? (int)std::min<size_t>((size_t)p.spc, (smem_max - base) / row) : 0;
     if (base > smem_max) p.grid = 0;
-    return p;
+    return l2_hints(p, nv, off, l2);
   }
   HalfPlan q = p;
   for (int c = 0; c < p.grid; ++c)
     q.cache_entries = std::max(q.cache_entries, off[part_begin(c + 1, nsl, p.grid)] - off[part_begin(c, nsl, p.grid)]);
   q.cached = 1;
   if (p.spc < 8) q.T = 8;
-  return half_smem(q) <= smem_max ? q : p;
+  return half_smem(q) <= smem_max ? q : l2_hints(p, nv, off, l2);
 }
 
 // properties of the current device that a resident launch needs; false without cooperative launches
-static bool resident_device(int& nsm, size_t& smem_max) {
-  int dev = 0, coop = 0, smax = 0;
+static bool resident_device(int& nsm, size_t& smem_max, size_t& l2) {
+  int dev = 0, coop = 0, smax = 0, l2b = 0;
   SSIM_CUDA(cudaGetDevice(&dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   SSIM_CUDA(cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+  SSIM_CUDA(cudaDeviceGetAttribute(&l2b, cudaDevAttrL2CacheSize, dev));
   smem_max = (size_t)smax - kSmemReserve;
+  l2 = (size_t)l2b;
   return coop != 0;
 }
 static bool resident_fits(const void* fn, int threads, size_t smem) {
@@ -1041,14 +1100,15 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
                               const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st) {
   if (H.nv <= 0) return true;
   int nsm = 0;
-  size_t smem_max = 0;
-  if (!resident_device(nsm, smem_max)) return false;
-  HalfPlan pl = half_plan(H.nv, off_host, nsm, smem_max, max_blocks);
+  size_t smem_max = 0, l2 = 0;
+  if (!resident_device(nsm, smem_max, l2)) return false;
+  HalfPlan pl = half_plan(H.nv, off_host, nsm, smem_max, l2, max_blocks);
   if (pl.grid < 1) return false;
   pl.smem = half_smem(pl);
-  const void* fn = !pl.cached   ? (const void*)resident_half_kernel<false, 4>
-                   : pl.T == 4 ? (const void*)resident_half_kernel<true, 4>
-                               : (const void*)resident_half_kernel<true, 8>;
+  const void* fn = pl.keep >= 0 ? (const void*)resident_half_kernel<false, 4, true>
+                   : !pl.cached ? (const void*)resident_half_kernel<false, 4>
+                   : pl.T == 4  ? (const void*)resident_half_kernel<true, 4>
+                                : (const void*)resident_half_kernel<true, 8>;
   if (!resident_fits(fn, HT, pl.smem)) return false;
   GridExchange gx = grid_exchange(rs, st);
   HalfMatrix h = H;
@@ -1090,8 +1150,8 @@ bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int
                            const ResidentSync& rs, int max_blocks, cudaStream_t st) {
   if (A.nv <= 0) return true;
   int nsm = 0;
-  size_t smem_max = 0;
-  if (!resident_device(nsm, smem_max)) return false;
+  size_t smem_max = 0, l2 = 0;
+  if (!resident_device(nsm, smem_max, l2)) return false;
   Plan64 pl = plan64(A.nv, sl_off, lo_off, nsm, smem_max, max_blocks);
   if (pl.grid < 1) return false;
   pl.smem = smem64(pl);
