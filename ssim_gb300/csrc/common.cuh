@@ -44,6 +44,18 @@ struct vec4<double> {
 
 inline int div_up(long long a, long long b) { return (int)((a + b - 1) / b); }
 
+// Blocks of a grid-stride launch over n threads' work: no more than the SMs hold at once (threads_per_sm, from the kernel's
+// registers), so the block sums, the arrival's fence and the last block's sum are paid once per resident block instead of
+// once per `block` items.
+inline int wave_grid(long long n, int block, int threads_per_sm) {
+  int dev = 0, nsm = 0;
+  SSIM_CUDA(cudaGetDevice(&dev));
+  SSIM_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const long long most = (long long)(nsm > 0 ? nsm : 1) * (threads_per_sm / block > 0 ? threads_per_sm / block : 1);
+  const long long need = (n + block - 1) / block;
+  return (int)(need < most ? need : most);
+}
+
 // scalars shared by the reductions of one handle (device memory, one block per handle)
 struct DevScalars {
   // gradient / energy
@@ -257,6 +269,21 @@ __device__ __forceinline__ bool grid_sum_last(const double (&blockval)[NV], doub
     return true;
   }
   return false;
+}
+
+constexpr int GL = 4;  // lanes of a vertex in the force gathers
+
+// the sums of a, b, c over a vertex's GL = 4 lanes: lane q of them ends with component q (lane 3 with nothing); the
+// first exchange splits the values over the lanes, 3 additions instead of 6
+template <typename S>
+__device__ __forceinline__ S quad_sum(S a, S b, S c, int q) {
+  const bool hi = q & 2;
+  S u = hi ? c : a, v = hi ? S(0) : b;
+  u += __shfl_xor_sync(0xffffffffu, hi ? a : c, 2);
+  v += __shfl_xor_sync(0xffffffffu, hi ? b : S(0), 2);
+  const bool odd = q & 1;
+  const S t = odd ? v : u;
+  return t + __shfl_xor_sync(0xffffffffu, odd ? u : v, 1);
 }
 
 }  // namespace ssim_gb

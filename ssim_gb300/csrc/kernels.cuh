@@ -11,7 +11,7 @@
 //                128-byte (FP32) or 256-byte (FP64) line; lower blocks are transposed upper slots
 //   dinv         vec4<S>[3V]  rows of the inverse 3x3 diagonal block (block-Jacobi preconditioner)
 //   Kbuf         S[T][10][9]  scaled element stiffness blocks (v <= w) awaiting assembly
-//   lf           double[T][4][3] scaled element forces awaiting the vertex gather
+//   lf           double[4][T][4] scaled element forces (xyz0) awaiting the vertex gather; triangles [T][3][4], springs [T][4]
 //   vectors      vec4<S>[V]  CG vectors, one padded xyz triple per vertex
 #pragma once
 #include <type_traits>
@@ -85,6 +85,7 @@ struct SpringData {
   const double* X;      // [V][3] rest positions
   const double* rest;   // [ns] rest lengths
   const double* k;      // [ns] stiffness
+  const double* e64;    // [3][ns] rest edge X_i - X_j
   const float4* e0;     // [ns] FP32 rest edge X_i - X_j and rest length (the FP32 spring pass)
   const float* k32;     // [ns] FP32 stiffness
 };
@@ -162,7 +163,7 @@ void launch_elem_energy_grad(const ElemFP64& el, const double* u, const double* 
                              bool trial, const Reduce& red, cudaStream_t st);
 void launch_node_mass(int nv, const int* vptr, const int* vinc, const double* vol, double* mnode, cudaStream_t st);
 // the mixed steppers' FP32 element pass: per-vertex FP32 split of u (hi + lo) and of w = u - x~ (made by
-// launch_split32 once per base point), FP32 element arithmetic, forces to lf32[t][4][3]
+// launch_split32 once per base point), FP32 element arithmetic, forces to lf32 ([4][t] 4-wide vectors)
 void launch_split32(int nv, const double* u, const double* xt, float4* uh, float4* ul, float4* w, cudaStream_t st);
 void launch_elem_energy_grad32(const ElemFP64& el, const ElemFP32& ef, const Split32& sp, const float4* d,
                                double alpha, double dt2, double rho, float* lf32, bool with_forces, bool trial,
@@ -174,12 +175,12 @@ void launch_elem_delta32(const ElemFP64& el, const ElemFP32& ef, const Split32& 
                          double alpha, double dt2, double rho, double e_ref, double escale_ref, float* lf32,
                          bool with_forces, bool trial, const Reduce& red, cudaStream_t st, int block = 0);
 // g = gref + the gathered increments (Dirichlet dofs zeroed), |g|^2 into sc->gnorm2
-void launch_vertex_gather_delta32(int nv, const int* vptr, const int* vinc, const float* lf32, const uint8_t* mask,
+void launch_vertex_gather_delta32(int nv, const int* vptr, const int* vinc, int soa, const float* lf32, const uint8_t* mask,
                                   const double* gref, double* g, const Reduce& red, cudaStream_t st, int block = 0);
 void launch_delta_base(int nv, const double* u, const double* uref, float4* db, cudaStream_t st);
-void launch_vertex_gather32(int nv, const int* vptr, const int* vinc, const float* lf32, const uint8_t* mask,
+void launch_vertex_gather32(int nv, const int* vptr, const int* vinc, int soa, const float* lf32, const uint8_t* mask,
                             double* g, const Reduce& red, cudaStream_t st, int block = 0);
-// mass-spring energy (+ spring forces into lf[s][2][3]) at u (+ alpha d), plus the lumped inertia energy
+// mass-spring energy (+ spring forces into lf, a 4-wide vector a spring) at u (+ alpha d), plus the lumped inertia energy
 template <typename SD>
 void launch_spring_energy_grad(const SpringData& sp, const double* u, const double* xt, const double* m, int nv,
                                const V4<SD>* d, double alpha, double dt2, double* lf, bool with_forces, bool trial,
@@ -203,16 +204,17 @@ void launch_spring_gather32(int nv, const int* vptr, const int* vinc, const floa
 // spring Hessian blocks Kbuf[s][3][9] (scaled by dt^2), the compressed transverse part dropped when spsd
 template <typename S>
 void launch_spring_hessian(const SpringData& sp, const double* u, double dt2, bool spsd, S* Kbuf, cudaStream_t st);
-// g[v] = sum over incident (e, i) of lf[e][i] (+ rho mnode[v] (u (+ alpha d) - x~) with mnode), Dirichlet dofs zeroed;
+// Local forces are 4-wide vectors: [4][t] for tets (soa = t), [t][3] for triangles (soa = 0).
+// g[v] = sum over incident (e, i) of the local forces (+ rho mnode[v] (u (+ alpha d) - x~) with mnode), Dirichlet dofs zeroed;
 // |g|^2 into sc->gnorm2
 template <typename SD>
-void launch_vertex_gather(int nv, const int* vptr, const int* vinc, const double* lf, const uint8_t* mask,
+void launch_vertex_gather(int nv, const int* vptr, const int* vinc, int soa, const double* lf, const uint8_t* mask,
                           const double* mnode, double rho, const double* u, const double* xt, const V4<SD>* d,
                           double alpha, double* g, const Reduce& red, cudaStream_t st);
 
 // ---------------- 2D triangles (kernels_tri.cu) ----------------
 // cells int4 (x, y, z = the triangle), dminv rows 0..3 = the row-major 2x2 Dm^-1, vol = area; local forces
-// lf[t][3][3] (z = 0), element blocks Kbuf[t][6][9] (the 6 upper 3x3 vertex blocks, z rows/columns 0)
+// lf[t][3] (4-wide, z = 0), element blocks Kbuf[t][6][9] (the 6 upper 3x3 vertex blocks, z rows/columns 0)
 template <typename SD>
 void launch_tri_energy_grad(const ElemFP64& el, const double* u, const double* xt, const V4<SD>* d, double alpha,
                             double dt2, double rho, double* lf, bool with_forces, bool trial, const Reduce& red,
@@ -220,7 +222,7 @@ void launch_tri_energy_grad(const ElemFP64& el, const double* u, const double* x
 template <typename S>
 void launch_tri_hessian(const ElemFP64& el, const double* u, double dt2, bool spsd, S* Kbuf, cudaStream_t st);
 // the FP32 pass of the mixed path for triangles (as launch_elem_energy_grad32): delta32 the per-element
-// FP32 stable Neo-Hookean delta, forces lf32[t][3][3] for launch_vertex_gather32
+// FP32 stable Neo-Hookean delta, forces lf32[t][3] (4-wide) for launch_vertex_gather32
 void launch_tri_energy_grad32(const ElemFP64& el, const ElemFP32& ef, const float* delta32, const Split32& sp,
                               const float4* d, double alpha, double dt2, double rho, float* lf32, bool with_forces,
                               bool trial, const Reduce& red, cudaStream_t st);

@@ -41,13 +41,11 @@ __global__ void __launch_bounds__(EB)
     elem_energy_grad_kernel(ElemFP64 el, const double* __restrict__ u, const double* __restrict__ xt,
                             const V4<SD>* __restrict__ d, double alpha, double dt2, double rho, int nv,
                             const double* __restrict__ mnode, double* __restrict__ lf, Reduce red) {
-  __shared__ double stage[FORCES ? EB * 12 : 1];
   __shared__ double shred[EB / 32][2];
-  const int e0 = blockIdx.x * EB;
-  const int e = e0 + threadIdx.x;
+  const int stride = gridDim.x * EB, first = blockIdx.x * EB + threadIdx.x;
   double energy = 0, escale = 0;
-  double lfv[12];
-  if (e < el.nt) {
+  for (int e = first; e < el.nt; e += stride) {
+    double lfv[12];
     const int4 c = el.cells[e];
     const int vid[4] = {c.x, c.y, c.z, c.w};
     double uu[4][3], sd[3];
@@ -110,13 +108,16 @@ __global__ void __launch_bounds__(EB)
         }
         lfv[j] = ms - tot[j];
       }
+      double4_32a* o = reinterpret_cast<double4_32a*>(lf) + e;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[(size_t)i * el.nt] = mk4<double>(lfv[3 * i], lfv[3 * i + 1], lfv[3 * i + 2]);
     }
     const double q = (0.5 * m) * (sd[0] * sd[0] + sd[1] * sd[1] + sd[2] * sd[2]);
-    energy = sV * psi + q;
-    escale = sV * sc + q;
+    energy += sV * psi + q;
+    escale += sV * sc + q;
   }
   // the vertices' share of the inertia energy
-  for (int v = e; v < nv; v += gridDim.x * EB) {
+  for (int v = first; v < nv; v += stride) {
     V4<SD> dv;
     if (TRIAL) dv = d[v];
     double q = 0;
@@ -130,16 +131,6 @@ __global__ void __launch_bounds__(EB)
     q *= (0.5 * rho) * mnode[v];
     energy += q;
     escale += q;
-  }
-  if (FORCES) {
-    if (e < el.nt) {
-#pragma unroll
-      for (int k = 0; k < 12; ++k) stage[threadIdx.x * 12 + k] = lfv[k];
-    }
-    __syncthreads();
-    const int nvalid = min(EB, el.nt - e0);
-    double* dst = lf + (size_t)e0 * 12;
-    for (int i = threadIdx.x; i < nvalid * 12; i += EB) dst[i] = stage[i];
   }
   double v2[2] = {energy, escale};
   block_sum<2, EB>(v2, shred);
@@ -172,8 +163,7 @@ __global__ void __launch_bounds__(256)
 // once (split32_kernel, once per base point), so the element forms its displacement differences
 // (hi_j - hi_i) + (lo_j - lo_i) (+ alpha (d_j - d_i)) in FP32 with rounding relative to the difference:
 // no FP64 arithmetic per element (GB300's FP64 pipe bound the earlier version).  Energy and stress use
-// the small-strain forms (snh_eval_small / linear_eval); energies are summed in FP32 within a warp and in
-// FP64 across warps and blocks; forces go to lf32[t][4][3] (FP32).
+// the small-strain forms (snh_eval_small / linear_eval); energies are summed in FP64; forces go to lf32 (FP32, see force_index).
 __global__ void __launch_bounds__(256)
     split32_kernel(int nv, const double* __restrict__ u, const double* __restrict__ xt, float4* __restrict__ uh,
                    float4* __restrict__ ul, float4* __restrict__ w) {
@@ -196,13 +186,10 @@ template <bool FORCES, bool TRIAL, int EB, int MINB = 1>
 __global__ void __launch_bounds__(EB, MINB)
     elem_energy_grad32_kernel(ElemFP64 el, ElemFP32 ef, Split32 sp, const float4* __restrict__ d, float alpha,
                               float dt2, float rho, float* __restrict__ lf32, Reduce red) {
-  __shared__ float stage[FORCES ? EB * 12 : 1];
   __shared__ double shred[EB / 32][2];
-  const int e0 = blockIdx.x * EB;
-  const int e = e0 + threadIdx.x;
-  float part[2] = {0.f, 0.f};
-  float lfv[12];
-  if (e < el.nt) {
+  double v2[2] = {0.0, 0.0};
+  for (int e = blockIdx.x * EB + threadIdx.x; e < el.nt; e += gridDim.x * EB) {
+    float lfv[12];
     const int4 c = el.cells[e];
     const int vid[4] = {c.x, c.y, c.z, c.w};
     float4 hv[4], lv[4], dv[4];
@@ -266,22 +253,14 @@ __global__ void __launch_bounds__(EB, MINB)
         }
 #pragma unroll
       for (int j = 0; j < 3; ++j) lfv[j] = -sV * tot[j] + m * (dd[0][j] + sd[j]);
-    }
-    part[0] = dt2 * V * psi + 0.5f * m * q;
-    part[1] = dt2 * V * sc + 0.5f * m * q;
-  }
-  if (FORCES) {
-    if (e < el.nt) {
+      float4* o = reinterpret_cast<float4*>(lf32) + e;
 #pragma unroll
-      for (int k = 0; k < 12; ++k) stage[threadIdx.x * 12 + k] = lfv[k];
+      for (int i = 0; i < 4; ++i) o[(size_t)i * el.nt] = make_float4(lfv[3 * i], lfv[3 * i + 1], lfv[3 * i + 2], 0.f);
     }
-    __syncthreads();
-    const int nvalid = min(EB, el.nt - e0);
-    float* dst = lf32 + (size_t)e0 * 12;
-    for (int i = threadIdx.x; i < nvalid * 12; i += EB) dst[i] = stage[i];
+    v2[0] += (double)(dt2 * V * psi + 0.5f * m * q);
+    v2[1] += (double)(dt2 * V * sc + 0.5f * m * q);
   }
-  double v2[2];
-  block_sum_s<2, EB, float>(part, v2, shred);
+  block_sum<2, EB>(v2, shred);
   double tot[2];
   if (grid_sum_last<2, EB>(v2, red.partials, red.counter, tot)) {
     if (TRIAL) {
@@ -306,13 +285,10 @@ __global__ void __launch_bounds__(EB)
     elem_delta32_kernel(ElemFP64 el, ElemFP32 ef, Split32 ref, const float4* __restrict__ db,
                         const float4* __restrict__ d, float alpha, float dt2, float rho, double e_ref,
                         double escale_ref, float* __restrict__ lf32, Reduce red) {
-  __shared__ float stage[FORCES ? EB * 12 : 1];
   __shared__ double shred[EB / 32][1];
-  const int e0 = blockIdx.x * EB;
-  const int e = e0 + threadIdx.x;
-  float part[1] = {0.f};
-  float lfv[12];
-  if (e < el.nt) {
+  double v1[1] = {0.0};
+  for (int e = blockIdx.x * EB + threadIdx.x; e < el.nt; e += gridDim.x * EB) {
+    float lfv[12];
     const int4 c = el.cells[e];
     const int vid[4] = {c.x, c.y, c.z, c.w};
     float4 hv[4], lv[4], wv[4];
@@ -383,21 +359,13 @@ __global__ void __launch_bounds__(EB)
         }
 #pragma unroll
       for (int j = 0; j < 3; ++j) lfv[j] = -sV * tot[j] + m * (x[0][j] + sx[j]);
-    }
-    part[0] = dt2 * V * dpsi + m * cross + 0.5f * m * quad;
-  }
-  if (FORCES) {
-    if (e < el.nt) {
+      float4* o = reinterpret_cast<float4*>(lf32) + e;
 #pragma unroll
-      for (int k = 0; k < 12; ++k) stage[threadIdx.x * 12 + k] = lfv[k];
+      for (int i = 0; i < 4; ++i) o[(size_t)i * el.nt] = make_float4(lfv[3 * i], lfv[3 * i + 1], lfv[3 * i + 2], 0.f);
     }
-    __syncthreads();
-    const int nvalid = min(EB, el.nt - e0);
-    float* dst = lf32 + (size_t)e0 * 12;
-    for (int i = threadIdx.x; i < nvalid * 12; i += EB) dst[i] = stage[i];
+    v1[0] += (double)(dt2 * V * dpsi + m * cross + 0.5f * m * quad);
   }
-  double v1[1];
-  block_sum_s<1, EB, float>(part, v1, shred);
+  block_sum<1, EB>(v1, shred);
   double tot[1];
   if (grid_sum_last<1, EB>(v1, red.partials, red.counter, tot)) {
     if (TRIAL) {
@@ -420,79 +388,78 @@ __global__ void __launch_bounds__(256)
 }
 
 constexpr int GB = 256;
-constexpr int GL = 4;  // lanes of a vertex in the force gathers
 
-// the sums of a, b, c over a vertex's GL = 4 lanes: lane q of them ends with component q (lane 3 with nothing); the
-// first exchange splits the values over the lanes, 3 additions instead of 6
-template <typename S>
-__device__ __forceinline__ S quad_sum(S a, S b, S c, int q) {
-  const bool hi = q & 2;
-  S u = hi ? c : a, v = hi ? S(0) : b;
-  u += __shfl_xor_sync(0xffffffffu, hi ? a : c, 2);
-  v += __shfl_xor_sync(0xffffffffu, hi ? b : S(0), 2);
-  const bool odd = q & 1;
-  const S t = odd ? v : u;
-  return t + __shfl_xor_sync(0xffffffffu, odd ? u : v, 1);
+// Local forces are 4-wide vectors, so an incidence is one load (three scalars each touch their own line of the 32 lanes'
+// scattered ones): with soa > 0 (tets, soa = their number) vertex i of element e at i * soa + e, so the element pass
+// writes four coalesced vectors a thread; with soa = 0 (triangles) in the order of the incidence codes.
+__device__ __forceinline__ size_t force_index(int code, int soa) {
+  return soa > 0 ? (size_t)(code & 3) * soa + (code >> 2) : (size_t)code;
 }
 
-// forces from FP32 local forces lf32[(e, i)][3], summed per vertex in FP32 (four lanes a vertex), Dirichlet dofs zeroed;
+// forces from FP32 local forces lf32 (force_index), summed per vertex in FP32 (four lanes a vertex), Dirichlet dofs zeroed;
 // |g|^2
 template <int B>
 __global__ void __launch_bounds__(B)
-    vertex_gather32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
+    vertex_gather32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc, int soa,
                            const float* __restrict__ lf32, const uint8_t* __restrict__ mask, double* __restrict__ g,
                            Reduce red) {
   __shared__ double shred[B / 32][1];
-  const int i = blockIdx.x * B + threadIdx.x, v = i / GL, q = i % GL;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f, part[1] = {0.f};
-  if (v < nv) {
-    const int k1 = vptr[v + 1];
+  double v1[1] = {0.0};
+  const int q = threadIdx.x % GL;
+  for (int v0 = blockIdx.x * (B / GL); v0 < nv; v0 += gridDim.x * (B / GL)) {
+    const int v = v0 + threadIdx.x / GL;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+    if (v < nv) {
+      const int k1 = vptr[v + 1];
 #pragma unroll 2
-    for (int k = vptr[v] + q; k < k1; k += GL) {
-      const float* s = lf32 + (size_t)vinc[k] * 3;
-      a0 += s[0];
-      a1 += s[1];
-      a2 += s[2];
+      for (int k = vptr[v] + q; k < k1; k += GL) {
+        const V4<float> f = reinterpret_cast<const V4<float>*>(lf32)[force_index(vinc[k], soa)];
+        a0 += f.x;
+        a1 += f.y;
+        a2 += f.z;
+      }
+    }
+    float t = quad_sum<float>(a0, a1, a2, q);
+    if (v < nv && q < 3) {
+      if ((mask[v] >> q) & 1) t = 0.f;
+      g[(size_t)v * 3 + q] = t;
+      v1[0] += (double)(t * t);
     }
   }
-  float t = quad_sum<float>(a0, a1, a2, q);
-  if (v < nv && q < 3) {
-    if ((mask[v] >> q) & 1) t = 0.f;
-    g[(size_t)v * 3 + q] = t;
-    part[0] = t * t;
-  }
-  double v1[1];
-  block_sum_s<1, B, float>(part, v1, shred);
+  block_sum<1, B>(v1, shred);
   double tot[1];
   if (grid_sum_last<1, B>(v1, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
 }
 
-// forces as the reference's FP64 forces plus the FP32 local force increments lf32[(e, i)][3] summed per
+// forces as the reference's FP64 forces plus the FP32 local force increments lf32 (force_index) summed per
 // vertex (four lanes a vertex), Dirichlet dofs zeroed; |g|^2 in FP64
 template <int B>
 __global__ void __launch_bounds__(B)
-    vertex_gather_delta32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
+    vertex_gather_delta32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc, int soa,
                                  const float* __restrict__ lf32, const uint8_t* __restrict__ mask,
                                  const double* __restrict__ gref, double* __restrict__ g, Reduce red) {
   __shared__ double shred[B / 32][1];
-  const int i = blockIdx.x * B + threadIdx.x, v = i / GL, q = i % GL;
-  float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+  const int q = threadIdx.x % GL;
   double part[1] = {0.0};
-  if (v < nv) {
-    const int k1 = vptr[v + 1];
+  for (int v0 = blockIdx.x * (B / GL); v0 < nv; v0 += gridDim.x * (B / GL)) {
+    const int v = v0 + threadIdx.x / GL;
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f;
+    if (v < nv) {
+      const int k1 = vptr[v + 1];
 #pragma unroll 2
-    for (int k = vptr[v] + q; k < k1; k += GL) {
-      const float* s = lf32 + (size_t)vinc[k] * 3;
-      a0 += s[0];
-      a1 += s[1];
-      a2 += s[2];
+      for (int k = vptr[v] + q; k < k1; k += GL) {
+        const V4<float> f = reinterpret_cast<const V4<float>*>(lf32)[force_index(vinc[k], soa)];
+        a0 += f.x;
+        a1 += f.y;
+        a2 += f.z;
+      }
     }
-  }
-  const float t = quad_sum<float>(a0, a1, a2, q);
-  if (v < nv && q < 3) {
-    const double gq = ((mask[v] >> q) & 1) ? 0.0 : gref[(size_t)v * 3 + q] + (double)t;
-    g[(size_t)v * 3 + q] = gq;
-    part[0] = gq * gq;
+    const float t = quad_sum<float>(a0, a1, a2, q);
+    if (v < nv && q < 3) {
+      const double gq = ((mask[v] >> q) & 1) ? 0.0 : gref[(size_t)v * 3 + q] + (double)t;
+      g[(size_t)v * 3 + q] = gq;
+      part[0] += gq * gq;
+    }
   }
   block_sum<1, B>(part, shred);
   double tot[1];
@@ -500,37 +467,41 @@ __global__ void __launch_bounds__(B)
 }
 
 // Four lanes share a vertex: one lane a vertex walked its 24 incidences as a chain of dependent loads (62 us at 180,285
-// vertices, 12.7 us at 1,331, where nothing else was in flight).  mnode (tets): the force M_i (u_i (+ alpha d_i) - x~_i)
+// vertices, 12.7 us at 1,331, where nothing else was in flight; now 51 and 7.6).  mnode (tets): the force M_i (u_i (+ alpha d_i) - x~_i)
 // that the element pass leaves to the vertices, nullptr otherwise.
 template <typename SD>
 __global__ void __launch_bounds__(GB)
-    vertex_gather_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
+    vertex_gather_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc, int soa,
                          const double* __restrict__ lf, const uint8_t* __restrict__ mask, const double* __restrict__ mnode, double rho,
                          const double* __restrict__ u, const double* __restrict__ xt, const V4<SD>* __restrict__ d,
                          double alpha, double* __restrict__ g, Reduce red) {
   __shared__ double shred[GB / 32][1];
-  const int i = blockIdx.x * GB + threadIdx.x, v = i / GL, q = i % GL;
-  double a0 = 0, a1 = 0, a2 = 0, part = 0;
-  if (v < nv) {
-    const int k1 = vptr[v + 1];
+  const int q = threadIdx.x % GL;
+  double part = 0;
+  for (int v0 = blockIdx.x * (GB / GL); v0 < nv; v0 += gridDim.x * (GB / GL)) {
+    const int v = v0 + threadIdx.x / GL;
+    double a0 = 0, a1 = 0, a2 = 0;
+    if (v < nv) {
+      const int k1 = vptr[v + 1];
 #pragma unroll 2
-    for (int k = vptr[v] + q; k < k1; k += GL) {
-      const double* s = lf + (size_t)vinc[k] * 3;
-      a0 += s[0];
-      a1 += s[1];
-      a2 += s[2];
+      for (int k = vptr[v] + q; k < k1; k += GL) {
+        const V4<double> f = reinterpret_cast<const V4<double>*>(lf)[force_index(vinc[k], soa)];
+        a0 += f.x;
+        a1 += f.y;
+        a2 += f.z;
+      }
     }
-  }
-  double t = quad_sum<double>(a0, a1, a2, q);
-  if (v < nv && q < 3) {
-    if (mnode != nullptr) {
-      double x = u[(size_t)v * 3 + q];
-      if (d != nullptr) x += alpha * (double)reinterpret_cast<const SD*>(d + v)[q];
-      t += (rho * mnode[v]) * (x - xt[(size_t)v * 3 + q]);
+    double t = quad_sum<double>(a0, a1, a2, q);
+    if (v < nv && q < 3) {
+      if (mnode != nullptr) {
+        double x = u[(size_t)v * 3 + q];
+        if (d != nullptr) x += alpha * (double)reinterpret_cast<const SD*>(d + v)[q];
+        t += (rho * mnode[v]) * (x - xt[(size_t)v * 3 + q]);
+      }
+      if ((mask[v] >> q) & 1) t = 0;  // boundary_condition::grads (boundary.hpp:45-51)
+      g[(size_t)v * 3 + q] = t;
+      part += t * t;
     }
-    if ((mask[v] >> q) & 1) t = 0;  // boundary_condition::grads (boundary.hpp:45-51)
-    g[(size_t)v * 3 + q] = t;
-    part = t * t;
   }
   double v1[1] = {part};
   block_sum<1, GB>(v1, shred);
@@ -606,7 +577,7 @@ void launch_elem_energy_grad(const ElemFP64& el, const double* u, const double* 
                              double dt2, double rho, int nv, const double* mnode, double* lf, bool with_forces,
                              bool trial, const Reduce& red, cudaStream_t st) {
   if (el.nt <= 0) return;
-  const int grid = div_up(el.nt, EB);
+  const int grid = wave_grid(el.nt, EB, 768);
   auto go = [&](auto fn) { fn<<<grid, EB, 0, st>>>(el, u, xt, d, alpha, dt2, rho, nv, mnode, lf, red); };
   if (trial && with_forces)
     go(elem_energy_grad_kernel<SD, true, true>);
@@ -640,7 +611,7 @@ void launch_elem_energy_grad32(const ElemFP64& el, const ElemFP32& ef, const Spl
   // in flight for the dependent vertex gathers, a few bytes of spill)
   auto launch = [&](auto B, auto M) {
     constexpr int b = decltype(B)::value, m = decltype(M)::value;
-    const int grid = div_up(el.nt, b);
+    const int grid = wave_grid(el.nt, b, m > 1 ? 1024 : 768);
     if (trial && with_forces)
       elem_energy_grad32_kernel<true, true, b, m><<<grid, b, 0, st>>>(el, ef, sp, d, a, f_dt2, f_rho, lf32, red);
     else if (trial)
@@ -667,7 +638,7 @@ void launch_elem_delta32(const ElemFP64& el, const ElemFP32& ef, const Split32& 
   const float f_dt2 = (float)dt2, f_rho = (float)rho, a = (float)alpha;
   auto go = [&](auto B) {
     constexpr int b = decltype(B)::value;
-    const int grid = div_up(el.nt, b);
+    const int grid = wave_grid(el.nt, b, 640);
     if (trial && with_forces)
       elem_delta32_kernel<true, true, b><<<grid, b, 0, st>>>(el, ef, ref, db, d, a, f_dt2, f_rho, e_ref, escale_ref, lf32, red);
     else if (trial)
@@ -680,12 +651,12 @@ void launch_elem_delta32(const ElemFP64& el, const ElemFP32& ef, const Split32& 
   dispatch_block<64, 128, 256>(block == 0 ? EB : block, go);
   after_launch("elem_delta32");
 }
-void launch_vertex_gather_delta32(int nv, const int* vptr, const int* vinc, const float* lf32, const uint8_t* mask,
+void launch_vertex_gather_delta32(int nv, const int* vptr, const int* vinc, int soa, const float* lf32, const uint8_t* mask,
                                   const double* gref, double* g, const Reduce& red, cudaStream_t st, int block) {
   if (nv <= 0) return;
   auto go = [&](auto B) {
     constexpr int b = decltype(B)::value;
-    vertex_gather_delta32_kernel<b><<<div_up((long long)GL * nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, gref, g, red);
+    vertex_gather_delta32_kernel<b><<<wave_grid((long long)GL * nv, b, 2048), b, 0, st>>>(nv, vptr, vinc, soa, lf32, mask, gref, g, red);
   };
   dispatch_block<128, 256, 512>(block == 0 ? 256 : block, go);
   after_launch("vertex_gather_delta32");
@@ -696,29 +667,29 @@ void launch_delta_base(int nv, const double* u, const double* uref, float4* db, 
   after_launch("delta_base");
 }
 
-void launch_vertex_gather32(int nv, const int* vptr, const int* vinc, const float* lf32, const uint8_t* mask,
+void launch_vertex_gather32(int nv, const int* vptr, const int* vinc, int soa, const float* lf32, const uint8_t* mask,
                             double* g, const Reduce& red, cudaStream_t st, int block) {
   if (nv <= 0) return;
   auto go = [&](auto B) {
     constexpr int b = decltype(B)::value;
-    vertex_gather32_kernel<b><<<div_up((long long)GL * nv, b), b, 0, st>>>(nv, vptr, vinc, lf32, mask, g, red);
+    vertex_gather32_kernel<b><<<wave_grid((long long)GL * nv, b, 2048), b, 0, st>>>(nv, vptr, vinc, soa, lf32, mask, g, red);
   };
   dispatch_block<128, 256, 512>(block == 0 ? 256 : block, go);
   after_launch("vertex_gather32");
 }
 template <typename SD>
-void launch_vertex_gather(int nv, const int* vptr, const int* vinc, const double* lf, const uint8_t* mask,
+void launch_vertex_gather(int nv, const int* vptr, const int* vinc, int soa, const double* lf, const uint8_t* mask,
                           const double* mnode, double rho, const double* u, const double* xt, const V4<SD>* d,
                           double alpha, double* g, const Reduce& red, cudaStream_t st) {
   if (nv <= 0) return;
-  vertex_gather_kernel<SD><<<div_up((long long)GL * nv, GB), GB, 0, st>>>(nv, vptr, vinc, lf, mask, mnode, rho, u, xt, d,
+  vertex_gather_kernel<SD><<<wave_grid((long long)GL * nv, GB, 2048), GB, 0, st>>>(nv, vptr, vinc, soa, lf, mask, mnode, rho, u, xt, d,
                                                                          alpha, g, red);
   after_launch("vertex_gather");
 }
-template void launch_vertex_gather<float>(int, const int*, const int*, const double*, const uint8_t*, const double*, double,
+template void launch_vertex_gather<float>(int, const int*, const int*, int, const double*, const uint8_t*, const double*, double,
                                           const double*, const double*, const float4*, double, double*, const Reduce&,
                                           cudaStream_t);
-template void launch_vertex_gather<double>(int, const int*, const int*, const double*, const uint8_t*, const double*, double,
+template void launch_vertex_gather<double>(int, const int*, const int*, int, const double*, const uint8_t*, const double*, double,
                                            const double*, const double*, const double4_32a*, double, double*,
                                            const Reduce&, cudaStream_t);
 void launch_node_mass(int nv, const int* vptr, const int* vinc, const double* vol, double* mnode, cudaStream_t st) {

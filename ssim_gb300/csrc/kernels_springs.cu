@@ -4,7 +4,7 @@
 // literature uses (Liu et al., "Fast Simulation of Mass-Spring Systems", SIGGRAPH Asia 2013).
 //
 // Springs are 2-vertex cells: the vertex gather, the block pattern, the atomic-free assembly and the
-// PCG are the tet ones; the spring forces go to lf[s][2][3], the Hessian blocks to Kbuf[s][3][9] (upper
+// PCG are the tet ones; the spring forces go to one 4-wide vector a spring, the Hessian blocks to Kbuf[s][3][9] (upper
 // vertex blocks (0,0), (0,1), (1,1)).
 #include "kernels.cuh"
 
@@ -39,25 +39,43 @@ __device__ __forceinline__ void edge_vec(const SpringData& sp, const double* __r
   }
 }
 
-// FP64 spring pass.  FP64 arithmetic is scarce on GB300, so the pass spends it where the digits matter:
-// the edge vector, |e|, l - L, the energy and the forces (one rsqrt gives both l = |e|^2 rsqrt and the
-// force factor's 1/l); the trial direction's difference d_i - d_j is formed in the direction's own type,
-// and the energy's term magnitude (used only as the round-off scale of the line search) in FP32.
+// energy share of vertex v's lumped inertia: 1/2 m_v |u_v (+ alpha d_v) - x~_v|^2
+template <typename SD, bool TRIAL>
+__device__ __forceinline__ double lumped_energy(int v, const double* __restrict__ m, const double* __restrict__ u,
+                                                const double* __restrict__ xt, const V4<SD>* __restrict__ d,
+                                                double alpha) {
+  V4<SD> dv;
+  if (TRIAL) dv = d[v];
+  double part = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    double w = u[3 * (size_t)v + k] - xt[3 * (size_t)v + k];
+    if (TRIAL) w += alpha * (double)comp4<SD>(dv, k);
+    part += w * w;
+  }
+  return 0.5 * m[v] * part;
+}
+
+// FP64 spring pass.  FP64 arithmetic is scarce on GB300 (about 40 operations a spring bound the pass), so it spends it
+// where the digits matter: the edge vector from the stored rest edge, |e|, l - L, the energy and the force (one rsqrt
+// gives both l = |e|^2 rsqrt and the force factor's 1/l); the trial direction's difference d_i - d_j is formed in the
+// direction's own type, and the energy's term magnitude (used only as the round-off scale of the line search) in FP32.
+// One force a spring, a 4-wide vector (vertex i gets +f, j -f: one load an incidence); the threads add their
+// vertices' inertia energy, a pass of its own before.  512 x 512 cloth: 137 + 12 us before, 94 now.
 template <typename SD, bool FORCES, bool TRIAL>
 __global__ void __launch_bounds__(PB)
-    spring_energy_grad_kernel(SpringData sp, const double* __restrict__ u, const V4<SD>* __restrict__ d,
-                              double alpha, double dt2, double* __restrict__ lf, Reduce red) {
-  __shared__ double shred[PB / 32][1];
-  __shared__ double shred2[PB / 32][1];
-  const int s = blockIdx.x * PB + threadIdx.x;
-  double energy[1] = {0.0};
-  float escale[1] = {0.f};
-  if (s < sp.ns) {
+    spring_energy_grad_kernel(SpringData sp, const double* __restrict__ u, const double* __restrict__ xt,
+                              const double* __restrict__ m, int nv, const V4<SD>* __restrict__ d, double alpha, double dt2,
+                              double* __restrict__ lf, Reduce red) {
+  __shared__ double shred[PB / 32][2];
+  const int stride = gridDim.x * PB, first = blockIdx.x * PB + threadIdx.x;
+  double v2[2] = {0.0, 0.0};
+  for (int s = first; s < sp.ns; s += stride) {
     const int2 c = sp.ends[s];
     const int i = c.x, j = c.y;
     double e[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) e[k] = (sp.X[3 * i + k] - sp.X[3 * j + k]) + (u[3 * i + k] - u[3 * j + k]);
+    for (int k = 0; k < 3; ++k) e[k] = sp.e64[(size_t)k * sp.ns + s] + (u[3 * (size_t)i + k] - u[3 * (size_t)j + k]);
     if (TRIAL) {
       const V4<SD> di = d[i], dj = d[j];
       e[0] += alpha * (double)(di.x - dj.x);
@@ -65,25 +83,22 @@ __global__ void __launch_bounds__(PB)
       e[2] += alpha * (double)(di.z - dj.z);
     }
     const double l2 = e[0] * e[0] + e[1] * e[1] + e[2] * e[2];
-    const double rl = l2 > 0.0 ? rsqrt(l2) : 0.0;
+    const double rl = __double_as_longlong(l2) > 0 ? rsqrt(l2) : 0.0;  // l2 > 0 without an FP64 comparison
     const double l = l2 * rl;
     const double L = sp.rest[s], kk = dt2 * sp.k[s];
-    const double dl = l - L;
-    energy[0] = 0.5 * kk * dl * dl;
-    escale[0] = 0.5f * (float)kk * ((float)l2 + (float)L * (float)L);
+    const double dl = l - L, kd = kk * dl;
+    v2[0] += kd * dl;
+    v2[1] += (double)(0.5f * (float)kk * ((float)l2 + (float)L * (float)L));
     if (FORCES) {
-      const double cf = kk * dl * rl;
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        lf[(size_t)s * 6 + q] = cf * e[q];
-        lf[(size_t)s * 6 + 3 + q] = -cf * e[q];
-      }
+      const double cf = kd * rl;
+      reinterpret_cast<double4_32a*>(lf)[s] = mk4<double>(cf * e[0], cf * e[1], cf * e[2]);
     }
   }
-  block_sum<1, PB>(energy, shred);
-  double sc1[1];
-  block_sum_s<1, PB, float>(escale, sc1, shred2);
-  double v2[2] = {energy[0], sc1[0]};
+  double inert = 0.0;
+  for (int v = first; v < nv; v += stride) inert += lumped_energy<SD, TRIAL>(v, m, u, xt, d, alpha);
+  v2[0] = 0.5 * v2[0] + inert;
+  v2[1] += inert;
+  block_sum<2, PB>(v2, shred);
   double tot[2];
   if (grid_sum_last<2, PB>(v2, red.partials, red.counter, tot)) {
     if (TRIAL) {
@@ -104,12 +119,13 @@ __global__ void __launch_bounds__(PB)
 // lf32[s] (vertex i gets +f_s, vertex j -f_s).
 template <typename SD, bool FORCES, bool TRIAL>
 __global__ void __launch_bounds__(PB)
-    spring_energy_grad32_kernel(SpringData sp, Split32 s3, const V4<SD>* __restrict__ d, double alpha, float dt2,
-                                float4* __restrict__ lf32, Reduce red) {
+    spring_energy_grad32_kernel(SpringData sp, Split32 s3, const double* __restrict__ u, const double* __restrict__ xt,
+                                const double* __restrict__ m, int nv, const V4<SD>* __restrict__ d, double alpha,
+                                float dt2, float4* __restrict__ lf32, Reduce red) {
   __shared__ double shred[PB / 32][2];
-  const int s = blockIdx.x * PB + threadIdx.x;
-  float part[2] = {0.f, 0.f};
-  if (s < sp.ns) {
+  const int stride = gridDim.x * PB, first = blockIdx.x * PB + threadIdx.x;
+  double v2[2] = {0.0, 0.0};
+  for (int s = first; s < sp.ns; s += stride) {
     const int2 c = sp.ends[s];
     const float4 e0 = sp.e0[s];
     const float4 hi = s3.uh[c.x], hj = s3.uh[c.y], li = s3.ul[c.x], lj = s3.ul[c.y];
@@ -127,15 +143,18 @@ __global__ void __launch_bounds__(PB)
     const float dl2 = 2.f * (e0.x * D[0] + e0.y * D[1] + e0.z * D[2]) + (D[0] * D[0] + D[1] * D[1] + D[2] * D[2]);
     const float dl = dl2 / (l + L);
     const float kk = dt2 * sp.k32[s];
-    part[0] = 0.5f * kk * dl * dl;
-    part[1] = 0.5f * kk * (l2 + L * L);
+    v2[0] += (double)(0.5f * kk * dl * dl);
+    v2[1] += (double)(0.5f * kk * (l2 + L * L));
     if (FORCES) {
       const float cf = l > 0.f ? kk * dl / l : 0.f;
       lf32[s] = make_float4(cf * ex, cf * ey, cf * ez, 0.f);
     }
   }
-  double v2[2];
-  block_sum_s<2, PB, float>(part, v2, shred);
+  double inert = 0.0;  // the vertices' inertia energy
+  for (int v = first; v < nv; v += stride) inert += lumped_energy<SD, TRIAL>(v, m, u, xt, d, alpha);
+  v2[0] += inert;
+  v2[1] += inert;
+  block_sum<2, PB>(v2, shred);
   double tot[2];
   if (grid_sum_last<2, PB>(v2, red.partials, red.counter, tot)) {
     if (TRIAL) {
@@ -148,8 +167,24 @@ __global__ void __launch_bounds__(PB)
   }
 }
 
+// dof q of vertex v: g = t + m (u (+ alpha d) - x~), zeroed on a Dirichlet dof; returns its square
+template <typename SD>
+__device__ __forceinline__ double spring_dof(double t, bool in, int v, int q, const double* __restrict__ m,
+                                             const double* __restrict__ u, const V4<SD>* __restrict__ d, double alpha,
+                                             const double* __restrict__ xt, const uint8_t* __restrict__ mask,
+                                             double* __restrict__ g) {
+  if (!in) return 0.0;
+  const size_t k = 3 * (size_t)v + q;
+  double w = u[k] - xt[k];
+  if (d != nullptr) w += alpha * (double)reinterpret_cast<const SD*>(d + v)[q];
+  double x = t + m[v] * w;
+  if ((mask[v] >> q) & 1) x = 0;
+  g[k] = x;
+  return x * x;
+}
+
 // g_v from the FP32 spring forces (summed in FP32 over the incident springs) + m_v (u_v (+ alpha d_v) - x~_v)
-// in FP64, Dirichlet dofs zeroed; |g|^2
+// in FP64, four lanes a vertex, Dirichlet dofs zeroed; |g|^2
 template <typename SD>
 __global__ void __launch_bounds__(PB)
     spring_gather32_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
@@ -157,77 +192,36 @@ __global__ void __launch_bounds__(PB)
                            const V4<SD>* __restrict__ d, double alpha, const double* __restrict__ xt,
                            const uint8_t* __restrict__ mask, double* __restrict__ g, Reduce red) {
   __shared__ double shred[PB / 32][1];
-  const int v = blockIdx.x * PB + threadIdx.x;
-  double part = 0;
-  if (v < nv) {
+  double v1[1] = {0.0};
+  const int q = threadIdx.x % GL;
+  for (int v0 = blockIdx.x * (PB / GL); v0 < nv; v0 += gridDim.x * (PB / GL)) {
+    const int v = v0 + threadIdx.x / GL;
     float a[3] = {0.f, 0.f, 0.f};
-    const int k1 = vptr[v + 1];
-    for (int k = vptr[v]; k < k1; ++k) {
-      const int code = vinc[k];
-      const float4 f = lf32[code >> 1];
-      const float sg = (code & 1) ? -1.f : 1.f;
-      a[0] += sg * f.x;
-      a[1] += sg * f.y;
-      a[2] += sg * f.z;
+    if (v < nv) {
+      const int k1 = vptr[v + 1];
+#pragma unroll 2
+      for (int k = vptr[v] + q; k < k1; k += GL) {
+        const int code = vinc[k];
+        const float4 f = lf32[code >> 1];
+        const float sg = (code & 1) ? -1.f : 1.f;
+        a[0] += sg * f.x;
+        a[1] += sg * f.y;
+        a[2] += sg * f.z;
+      }
     }
-    double dv[3] = {0, 0, 0};
-    if (d != nullptr) {
-      const V4<SD> t = d[v];
-      dv[0] = alpha * (double)t.x;
-      dv[1] = alpha * (double)t.y;
-      dv[2] = alpha * (double)t.z;
-    }
-    const uint8_t mk = mask[v];
-#pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      double gq = (double)a[q] + m[v] * ((u[3 * v + q] - xt[3 * v + q]) + dv[q]);
-      if ((mk >> q) & 1) gq = 0;
-      g[3 * v + q] = gq;
-      part += gq * gq;
-    }
+    const float t = quad_sum<float>(a[0], a[1], a[2], q);
+    v1[0] += spring_dof<SD>((double)t, v < nv && q < 3, v, q, m, u, d, alpha, xt, mask, g);
   }
-  double v1[1] = {part};
   block_sum<1, PB>(v1, shred);
   double tot[1];
   if (grid_sum_last<1, PB>(v1, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
 }
 
-// lumped inertia 1/2 sum_v m_v |u_v (+ alpha d_v) - x~_v|^2, added to the (trial) energy and its scale
-template <typename SD, bool TRIAL>
-__global__ void __launch_bounds__(PB)
-    lumped_inertia_energy_kernel(int nv, const double* __restrict__ m, const double* __restrict__ u,
-                                 const double* __restrict__ xt, const V4<SD>* __restrict__ d, double alpha,
-                                 Reduce red) {
-  __shared__ double shred[PB / 32][1];
-  const int v = blockIdx.x * PB + threadIdx.x;
-  double part = 0;
-  if (v < nv) {
-    V4<SD> dv;
-    if (TRIAL) dv = d[v];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      double w = u[3 * v + k] - xt[3 * v + k];
-      if (TRIAL) w += alpha * (double)comp4<SD>(dv, k);
-      part += w * w;
-    }
-    part *= 0.5 * m[v];
-  }
-  double v1[1] = {part};
-  block_sum<1, PB>(v1, shred);
-  double tot[1];
-  if (grid_sum_last<1, PB>(v1, red.partials, red.counter, tot)) {
-    if (TRIAL) {
-      red.sc->trial_energy += tot[0];
-      red.sc->trial_energy_scale += tot[0];
-    } else {
-      red.sc->energy += tot[0];
-      red.sc->energy_scale += tot[0];
-    }
-  }
-}
-
-// g_v = sum of the incident spring forces + m_v (u_v (+ alpha d_v) - x~_v), Dirichlet dofs zeroed; |g|^2.
-// With d the springs' forces must be those of the same trial point u + alpha d.
+// g_v = sum of the incident spring forces (vertex i of a spring receives +f, vertex j -f) + m_v (u_v (+ alpha
+// d_v) - x~_v), Dirichlet dofs zeroed; |g|^2.  With d the springs' forces must be those of the same trial point
+// u + alpha d.  One lane a vertex: an FP64 operation costs a warp the same for any number of active lanes, so the 36
+// additions of 12 incidences serve 32 vertices (512 x 512 cloth: 64 us with four lanes a vertex, 30 so; 52 where the sign
+// was a selected negation instead of a factor, 39 with two stored forces a spring).
 template <typename SD>
 __global__ void __launch_bounds__(PB)
     spring_gather_kernel(int nv, const int* __restrict__ vptr, const int* __restrict__ vinc,
@@ -235,34 +229,22 @@ __global__ void __launch_bounds__(PB)
                          const V4<SD>* __restrict__ d, double alpha, const double* __restrict__ xt,
                          const uint8_t* __restrict__ mask, double* __restrict__ g, Reduce red) {
   __shared__ double shred[PB / 32][1];
-  const int v = blockIdx.x * PB + threadIdx.x;
-  double part = 0;
-  if (v < nv) {
+  double v1[1] = {0.0};
+  for (int v = blockIdx.x * PB + threadIdx.x; v < nv; v += gridDim.x * PB) {
     double a[3] = {0, 0, 0};
     const int k1 = vptr[v + 1];
+#pragma unroll 4
     for (int k = vptr[v]; k < k1; ++k) {
-      const double* s = lf + (size_t)vinc[k] * 3;
-      a[0] += s[0];
-      a[1] += s[1];
-      a[2] += s[2];
-    }
-    const uint8_t mk = mask[v];
-    double dv[3] = {0, 0, 0};
-    if (d != nullptr) {
-      const V4<SD> t = d[v];
-      dv[0] = alpha * (double)t.x;
-      dv[1] = alpha * (double)t.y;
-      dv[2] = alpha * (double)t.z;
+      const int code = vinc[k];
+      const double4_32a f = reinterpret_cast<const double4_32a*>(lf)[code >> 1];
+      const double sg = __hiloint2double((code & 1) ? 0xBFF00000 : 0x3FF00000, 0);  // +-1
+      a[0] = fma(sg, f.x, a[0]);
+      a[1] = fma(sg, f.y, a[1]);
+      a[2] = fma(sg, f.z, a[2]);
     }
 #pragma unroll
-    for (int q = 0; q < 3; ++q) {
-      a[q] += m[v] * ((u[3 * v + q] - xt[3 * v + q]) + dv[q]);
-      if ((mk >> q) & 1) a[q] = 0;
-      g[3 * v + q] = a[q];
-      part += a[q] * a[q];
-    }
+    for (int q = 0; q < 3; ++q) v1[0] += spring_dof<SD>(a[q], true, v, q, m, u, d, alpha, xt, mask, g);
   }
-  double v1[1] = {part};
   block_sum<1, PB>(v1, shred);
   double tot[1];
   if (grid_sum_last<1, PB>(v1, red.partials, red.counter, tot)) red.sc->gnorm2 = tot[0];
@@ -308,30 +290,24 @@ template <typename SD>
 void launch_spring_energy_grad(const SpringData& sp, const double* u, const double* xt, const double* m, int nv,
                                const V4<SD>* d, double alpha, double dt2, double* lf, bool with_forces, bool trial,
                                const Reduce& red, cudaStream_t st) {
-  if (sp.ns > 0) {
-    const int grid = div_up(sp.ns, PB);
-    if (trial && with_forces)
-      spring_energy_grad_kernel<SD, true, true><<<grid, PB, 0, st>>>(sp, u, d, alpha, dt2, lf, red);
-    else if (trial)
-      spring_energy_grad_kernel<SD, false, true><<<grid, PB, 0, st>>>(sp, u, d, alpha, dt2, lf, red);
-    else if (with_forces)
-      spring_energy_grad_kernel<SD, true, false><<<grid, PB, 0, st>>>(sp, u, d, alpha, dt2, lf, red);
-    else
-      spring_energy_grad_kernel<SD, false, false><<<grid, PB, 0, st>>>(sp, u, d, alpha, dt2, lf, red);
-    after_launch("spring_energy_grad");
-  }
-  if (trial)
-    lumped_inertia_energy_kernel<SD, true><<<div_up(nv, PB), PB, 0, st>>>(nv, m, u, xt, d, alpha, red);
+  if (sp.ns <= 0) return;
+  auto go = [&](auto fn) { fn<<<wave_grid(sp.ns, PB, 2048), PB, 0, st>>>(sp, u, xt, m, nv, d, alpha, dt2, lf, red); };
+  if (trial && with_forces)
+    go(spring_energy_grad_kernel<SD, true, true>);
+  else if (trial)
+    go(spring_energy_grad_kernel<SD, false, true>);
+  else if (with_forces)
+    go(spring_energy_grad_kernel<SD, true, false>);
   else
-    lumped_inertia_energy_kernel<SD, false><<<div_up(nv, PB), PB, 0, st>>>(nv, m, u, xt, d, alpha, red);
-  after_launch("lumped_inertia_energy");
+    go(spring_energy_grad_kernel<SD, false, false>);
+  after_launch("spring_energy_grad");
 }
 
 template <typename SD>
 void launch_spring_gather(int nv, const int* vptr, const int* vinc, const double* lf, const double* m,
                           const double* u, const V4<SD>* d, double alpha, const double* xt, const uint8_t* mask,
                           double* g, const Reduce& red, cudaStream_t st) {
-  spring_gather_kernel<SD><<<div_up(nv, PB), PB, 0, st>>>(nv, vptr, vinc, lf, m, u, d, alpha, xt, mask, g, red);
+  spring_gather_kernel<SD><<<wave_grid(nv, PB, 2048), PB, 0, st>>>(nv, vptr, vinc, lf, m, u, d, alpha, xt, mask, g, red);
   after_launch("spring_gather");
 }
 
@@ -339,31 +315,25 @@ template <typename SD>
 void launch_spring_energy_grad32(const SpringData& sp, const Split32& s3, const double* u, const double* xt,
                                  const double* m, int nv, const V4<SD>* d, double alpha, double dt2, float4* lf32,
                                  bool with_forces, bool trial, const Reduce& red, cudaStream_t st) {
-  if (sp.ns > 0) {
-    const int grid = div_up(sp.ns, PB);
-    const float f2 = (float)dt2;
-    if (trial && with_forces)
-      spring_energy_grad32_kernel<SD, true, true><<<grid, PB, 0, st>>>(sp, s3, d, alpha, f2, lf32, red);
-    else if (trial)
-      spring_energy_grad32_kernel<SD, false, true><<<grid, PB, 0, st>>>(sp, s3, d, alpha, f2, lf32, red);
-    else if (with_forces)
-      spring_energy_grad32_kernel<SD, true, false><<<grid, PB, 0, st>>>(sp, s3, d, alpha, f2, lf32, red);
-    else
-      spring_energy_grad32_kernel<SD, false, false><<<grid, PB, 0, st>>>(sp, s3, d, alpha, f2, lf32, red);
-    after_launch("spring_energy_grad32");
-  }
-  if (trial)
-    lumped_inertia_energy_kernel<SD, true><<<div_up(nv, PB), PB, 0, st>>>(nv, m, u, xt, d, alpha, red);
+  if (sp.ns <= 0) return;
+  const float f2 = (float)dt2;
+  auto go = [&](auto fn) { fn<<<wave_grid(sp.ns, PB, 2048), PB, 0, st>>>(sp, s3, u, xt, m, nv, d, alpha, f2, lf32, red); };
+  if (trial && with_forces)
+    go(spring_energy_grad32_kernel<SD, true, true>);
+  else if (trial)
+    go(spring_energy_grad32_kernel<SD, false, true>);
+  else if (with_forces)
+    go(spring_energy_grad32_kernel<SD, true, false>);
   else
-    lumped_inertia_energy_kernel<SD, false><<<div_up(nv, PB), PB, 0, st>>>(nv, m, u, xt, d, alpha, red);
-  after_launch("lumped_inertia_energy");
+    go(spring_energy_grad32_kernel<SD, false, false>);
+  after_launch("spring_energy_grad32");
 }
 
 template <typename SD>
 void launch_spring_gather32(int nv, const int* vptr, const int* vinc, const float4* lf32, const double* m,
                             const double* u, const V4<SD>* d, double alpha, const double* xt, const uint8_t* mask,
                             double* g, const Reduce& red, cudaStream_t st) {
-  spring_gather32_kernel<SD><<<div_up(nv, PB), PB, 0, st>>>(nv, vptr, vinc, lf32, m, u, d, alpha, xt, mask, g, red);
+  spring_gather32_kernel<SD><<<wave_grid((long long)GL * nv, PB, 2048), PB, 0, st>>>(nv, vptr, vinc, lf32, m, u, d, alpha, xt, mask, g, red);
   after_launch("spring_gather32");
 }
 

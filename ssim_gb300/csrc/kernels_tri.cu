@@ -98,7 +98,7 @@ __device__ __forceinline__ void jacobi4(S (&A)[16], S (&V)[16]) {
   }
 }
 
-// one element pass: energy (+ scale), and with FORCES the local forces lf[t][3][3]; inertia from the
+// one element pass: energy (+ scale), and with FORCES the local forces lf[t][3] (4-wide); inertia from the
 // consistent P1 mass rho A / 12 (1 + delta_ij) of the triangle
 template <typename SD, bool FORCES, bool TRIAL>
 __global__ void __launch_bounds__(TB)
@@ -161,9 +161,9 @@ __global__ void __launch_bounds__(TB)
 #pragma unroll
       for (int j = 0; j < 2; ++j) out[j] = -s * tot[j] + m * (dd[0][j] + sd[j]);
       out[2] = out[5] = out[8] = 0.0;
-      double* dst = lf + (size_t)e * 9;
+      double4_32a* dst = reinterpret_cast<double4_32a*>(lf) + 3 * (size_t)e;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) dst[k] = out[k];
+      for (int i = 0; i < 3; ++i) dst[i] = mk4<double>(out[3 * i], out[3 * i + 1], out[3 * i + 2]);
     }
     energy = dt2 * A * psi + 0.5 * m * q;
     escale = dt2 * A * sc + 0.5 * m * q;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(TB)
 // FP32 element pass of the mixed path (the triangle analogue of elem_energy_grad32_kernel): displacement
 // differences from the per-vertex FP32 split ((hi_j - hi_i) + (lo_j - lo_i) + alpha (d_j - d_i)), inertia
 // offsets from w = u - x~ rounded once per vertex, the strain-relative 2D stable Neo-Hookean
-// (snh2_eval_small) or the linear model, FP32 forces lf32[t][3][3] (z = 0) for vertex_gather32; energy
+// (snh2_eval_small) or the linear model, FP32 forces lf32[t][3] (4-wide, z = 0) for vertex_gather32; energy
 // and its magnitude sum summed in FP64 across warps, blocks and the grid.
 template <bool FORCES, bool TRIAL>
 __global__ void __launch_bounds__(TB)
@@ -354,9 +354,9 @@ __global__ void __launch_bounds__(TB)
 #pragma unroll
       for (int j = 0; j < 2; ++j) out[j] = -sA * tot[j] + m * (dd[0][j] + sd[j]);
       out[2] = out[5] = out[8] = 0.f;
-      float* dst = lf32 + (size_t)e * 9;
+      float4* dst = reinterpret_cast<float4*>(lf32) + 3 * (size_t)e;
 #pragma unroll
-      for (int k = 0; k < 9; ++k) dst[k] = out[k];
+      for (int i = 0; i < 3; ++i) dst[i] = make_float4(out[3 * i], out[3 * i + 1], out[3 * i + 2], 0.f);
     }
     part[0] = dt2 * A * psi + 0.5f * m * q;
     part[1] = dt2 * A * sc + 0.5f * m * q;

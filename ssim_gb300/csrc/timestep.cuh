@@ -217,11 +217,11 @@ struct TimeStep {
   // 2D triangles in the plane (cells are triangles; the z dof of every vertex carries no force)
   bool tri2d = false;
   DBuf<int2> sp_ends;
-  DBuf<double> sp_rest, sp_k, vmass;
+  DBuf<double> sp_rest, sp_k, sp_e64, vmass;
   DBuf<float4> sp_e0, sp_lf32;
   DBuf<float> sp_k32;
   std::vector<double> vmass_h, sp_k_h;
-  SpringData spd() const { return SpringData{nt, sp_ends.p, dX.p, sp_rest.p, sp_k.p, sp_e0.p, sp_k32.p}; }
+  SpringData spd() const { return SpringData{nt, sp_ends.p, dX.p, sp_rest.p, sp_k.p, sp_e64.p, sp_e0.p, sp_k32.p}; }
   // the FP32 passes' per-vertex split of next (hi + lo) and of next - x~; split32() refreshes it for the
   // current next (once per base point: every trial of a line search shares it), lf32t holds the tets'
   // FP32 local forces
@@ -259,13 +259,13 @@ struct TimeStep {
                         red(), stream, shapes.elem);
   }
   void delta_gather() {
-    launch_vertex_gather_delta32(nv, vptr.p, vinc.p, lf32t.p, mask.p, gref.p, forces.p, red(), stream, shapes.gather);
+    launch_vertex_gather_delta32(nv, vptr.p, vinc.p, nt, lf32t.p, mask.p, gref.p, forces.p, red(), stream, shapes.gather);
   }
   void split32() {
     uh32.alloc(nv);
     ul32.alloc(nv);
     w32.alloc(nv);
-    if (!springs) lf32t.alloc((tri2d ? 9 : 12) * (size_t)nt);
+    if (!springs) lf32t.alloc((tri2d ? 12 : 16) * (size_t)nt);
     launch_split32(nv, next.p, inertia.p, uh32.p, ul32.p, w32.p, stream);
   }
 
@@ -319,9 +319,9 @@ struct TimeStep {
       launch_spring_gather<S>(nv, vptr.p, vinc.p, lf.p, vmass.p, next.p, d, alpha, inertia.p, mask.p, forces.p, red(),
                               stream);
     else if (fp32)
-      launch_vertex_gather32(nv, vptr.p, vinc.p, lf32t.p, mask.p, forces.p, red(), stream, shapes.gather);
+      launch_vertex_gather32(nv, vptr.p, vinc.p, tri2d ? 0 : nt, lf32t.p, mask.p, forces.p, red(), stream, shapes.gather);
     else
-      launch_vertex_gather<S>(nv, vptr.p, vinc.p, lf.p, mask.p, tri2d ? nullptr : mnode.p, rho, next.p, inertia.p, d,
+      launch_vertex_gather<S>(nv, vptr.p, vinc.p, tri2d ? 0 : nt, lf.p, mask.p, tri2d ? nullptr : mnode.p, rho, next.p, inertia.p, d,
                               alpha, forces.p, red(), stream);
   }
   // mass per upper slot: consistent (tets) or lumped on the diagonal (springs)
@@ -476,6 +476,10 @@ struct TimeStep {
                           (float)(X[3 * i + 2] - X[3 * j + 2]), (float)rest[e]);
     }
     sp_e0.upload(e0, stream);
+    std::vector<double> e64(3 * (size_t)nt);
+    for (int e = 0; e < nt; ++e)
+      for (int q = 0; q < 3; ++q) e64[(size_t)q * nt + e] = X[3 * cells[2 * e] + q] - X[3 * cells[2 * e + 1] + q];
+    sp_e64.upload(e64, stream);
     std::vector<float> k32(sp_k_h.begin(), sp_k_h.end());
     sp_k32.upload(k32, stream);
     sp_lf32.alloc(nt);
@@ -581,7 +585,7 @@ struct TimeStep {
     lo_off.upload(topo.lo_off, stream);
     lo_src.upload(topo.lo_src, stream);
     lo_col.upload(topo.lo_col, stream);
-    lf.alloc((size_t)3 * cv * nt);
+    lf.alloc((size_t)4 * (cv == 2 ? 1 : cv) * nt);  // a 4-wide vector per local force (springs: one a spring)
   }
 
   // the fused kernel's lists, built on its first use (4 slices = 128 block rows per CTA); false if the mesh
@@ -1902,7 +1906,7 @@ struct TimeStep {
         best = 1e300;
         for (int b : {128, 256, 512}) {
           const double ms = time_launches(
-              [&] { launch_vertex_gather32(nv, vptr.p, vinc.p, lf32t.p, mask.p, forces.p, red(), stream, b); });
+              [&] { launch_vertex_gather32(nv, vptr.p, vinc.p, tri2d ? 0 : nt, lf32t.p, mask.p, forces.p, red(), stream, b); });
           ++count;
           if (ms < best) best = ms, t.gather_block = b;
         }
