@@ -10,7 +10,8 @@
 //                sits at vals[9*(q & ~31) + 32*c + (q & 31)] so that every component load of a warp is one
 //                128-byte (FP32) or 256-byte (FP64) line; lower blocks are transposed upper slots
 //   dinv         vec4<S>[3V]  rows of the inverse 3x3 diagonal block (block-Jacobi preconditioner)
-//   Kbuf         S[T][10][9]  scaled element stiffness blocks (v <= w) awaiting assembly
+//   Kbuf         10 T scaled element stiffness blocks (v <= w) awaiting assembly, block b of element e at b T + e: a
+//                V4<S> with values 0-3, one with 4-7 and a scalar per block, in three planes (store_kblock)
 //   lf           double[4][T][4] scaled element forces (xyz0) awaiting the vertex gather; triangles [T][3][4], springs [T][4]
 //   vectors      vec4<S>[V]  CG vectors, one padded xyz triple per vertex
 #pragma once
@@ -24,6 +25,27 @@ namespace ssim_gb {
 
 template <typename S>
 using V4 = typename vec4<S>::type;
+
+// Element blocks of the assembly: n of them, block b of element e at index b n_e + e, as planes of V4<S> (values 0-3, 4-7)
+// and S (value 8).  Elements of one mesh cell are neighbours in memory and their same blocks belong to neighbouring
+// rows, so a warp that gathers one contribution for 32 rows finds its blocks close together: three loads of about 24
+// lines each, where element-major records took nine of 32 lines.
+template <typename S>
+__device__ __forceinline__ void store_kblock(S* K, size_t n, size_t i, const S* v) {
+  V4<S> a, b;
+  a.x = v[0], a.y = v[1], a.z = v[2], a.w = v[3];
+  b.x = v[4], b.y = v[5], b.z = v[6], b.w = v[7];
+  reinterpret_cast<V4<S>*>(K)[i] = a;
+  reinterpret_cast<V4<S>*>(K)[n + i] = b;
+  K[8 * n + i] = v[8];
+}
+template <typename S>
+__device__ __forceinline__ void load_kblock(const S* __restrict__ K, size_t n, size_t i, S (&v)[9]) {
+  const V4<S> a = reinterpret_cast<const V4<S>*>(K)[i], b = reinterpret_cast<const V4<S>*>(K)[n + i];
+  v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+  v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  v[8] = K[8 * n + i];
+}
 
 // a 4-wide vector with w = 0
 template <typename S>
@@ -201,7 +223,7 @@ template <typename SD>
 void launch_spring_gather32(int nv, const int* vptr, const int* vinc, const float4* lf32, const double* m,
                             const double* u, const V4<SD>* d, double alpha, const double* xt, const uint8_t* mask,
                             double* g, const Reduce& red, cudaStream_t st);
-// spring Hessian blocks Kbuf[s][3][9] (scaled by dt^2), the compressed transverse part dropped when spsd
+// spring Hessian blocks (3 a spring, store_kblock; scaled by dt^2), the compressed transverse part dropped when spsd
 template <typename S>
 void launch_spring_hessian(const SpringData& sp, const double* u, double dt2, bool spsd, S* Kbuf, cudaStream_t st);
 // Local forces are 4-wide vectors: [4][t] for tets (soa = t), [t][3] for triangles (soa = 0).
@@ -214,7 +236,7 @@ void launch_vertex_gather(int nv, const int* vptr, const int* vinc, int soa, con
 
 // ---------------- 2D triangles (kernels_tri.cu) ----------------
 // cells int4 (x, y, z = the triangle), dminv rows 0..3 = the row-major 2x2 Dm^-1, vol = area; local forces
-// lf[t][3] (4-wide, z = 0), element blocks Kbuf[t][6][9] (the 6 upper 3x3 vertex blocks, z rows/columns 0)
+// lf[t][3] (4-wide, z = 0), element blocks (store_kblock; the 6 upper 3x3 vertex blocks, z rows/columns 0)
 template <typename SD>
 void launch_tri_energy_grad(const ElemFP64& el, const double* u, const double* xt, const V4<SD>* d, double alpha,
                             double dt2, double rho, double* lf, bool with_forces, bool trial, const Reduce& red,
@@ -247,13 +269,13 @@ void launch_fused_hessian(const ElemFP64& e64, const ElemFP32& e32, const double
 int fused_chunk();
 
 template <typename S>
-void launch_assemble(const SellMatrix& A, const int* cptr, const int* csrc, const S* Kbuf, const S* slot_mass,
+void launch_assemble(const SellMatrix& A, const int* cptr, const int* csrc, const S* Kbuf, size_t nb, const S* slot_mass,
                      const uint8_t* mask, bool filter, S* vals, V4<S>* dinv, int precond, cudaStream_t st, int block = 0);
-// the element Hessian blocks in FP16 (per block a power-of-two scale; 24 bytes a block instead of 36) and the
+// the element Hessian blocks in FP16 (per block a power-of-two scale; 20 bytes a block instead of 36, two planes: uint4[nb], then a word each) and the
 // assembly that reads them (FP32 sums): the mixed Newton's assemblies whose solve runs on the FP16 matrix copy
 void launch_elem_hessian16(const ElemFP64& e64, const ElemFP32& e32, const double* X, const double* u,
-                           const float4* xf, double dt2, bool spsd, uint2* K16, cudaStream_t st, int block = 0);
-void launch_assemble16(const SellMatrix& A, const int* cptr, const int* csrc, const uint2* K16, const float* slot_mass,
+                           const float4* xf, double dt2, bool spsd, uint4* K16, cudaStream_t st, int block = 0);
+void launch_assemble16(const SellMatrix& A, const int* cptr, const int* csrc, const uint4* K16, size_t nb, const float* slot_mass,
                        const uint8_t* mask, bool filter, float* vals, float4* dinv, int precond, cudaStream_t st,
                        int block = 0);
 template <typename S>

@@ -511,15 +511,16 @@ __global__ void __launch_bounds__(GB)
 
 // ------------------------------------------------------------------ element Hessian
 // One thread per tet: K_e = dt^2 V_e pfpx^T H+ pfpx (the gather weight V_e and alpha = dt^2 of
-// time_step.hpp:646-651 folded in), written as the 10 upper 3x3 vertex blocks, staged through shared
-// memory so the global writes are contiguous.  Bound by FP32 arithmetic (FP64: by the FP64 units).  The blocks leave
-// as they are formed (element_stiffness_blocks): 96 registers in FP32, 119 with FP16 blocks, 190 in FP64, no spills;
-// with 78 sums held to the end it was 128 and 176 bytes of spills.  1.02M tets, FP16 blocks: 102 us (169 before); 192k
-// tets, FP32 blocks: 21 us (37); FP64, 84,474 tets: 223 us (531), 30,498 tets: 92 us (195).
-// H16 (FP32 arithmetic only): each block written as twelve FP16 words, the nine values scaled by 2^-k and
-// k (the power of two that puts the block's largest magnitude in [2^14, 2^15)) in word 9: 24 bytes a block
-// instead of 36, read back with three 8-byte loads (kernels_sparse.cu assemble_kernel).
-__device__ __forceinline__ void pack_block16(const float* v, uint2* out) {
+// time_step.hpp:646-651 folded in), written as the 10 upper 3x3 vertex blocks, each a coalesced store
+// into its planes (store_kblock).  Bound by FP32 arithmetic (FP64: by the FP64 units).  The blocks leave
+// as they are formed (element_stiffness_blocks): 110 registers in FP32, 120 with FP16 blocks, 196 in FP64, no spills;
+// with 78 sums held to the end it was 128 and 176 bytes of spills.  1.02M tets, FP16 blocks: 94 us (169 at first, 102 with
+// the blocks staged through shared memory into element-major records); 192k tets, FP32 blocks: 20 us (37); FP64, 84,474
+// tets: 223 us (531), 30,498 tets: 92 us (195).
+// H16 (FP32 arithmetic only): a block is nine FP16 values scaled by 2^-k and k (the power of two that puts the block's
+// largest magnitude in [2^14, 2^15)): the first eight values in a 16-byte vector, the ninth and k in a word of a second
+// plane, 20 bytes a block instead of 36, read back with two loads (kernels_sparse.cu assemble_kernel).
+__device__ __forceinline__ void pack_block16(const float* v, uint4& lo, unsigned int& hi) {
   float m = 0.f;
 #pragma unroll
   for (int i = 0; i < 9; ++i) m = fmaxf(m, fabsf(v[i]));
@@ -527,47 +528,28 @@ __device__ __forceinline__ void pack_block16(const float* v, uint2* out) {
   if (m > 0.f && m <= FLT_MAX) k = ((__float_as_int(m) >> 23) & 0xff) - 127 - 14;  // floor(log2 m) - 14
   k = max(-100, min(100, k));
   const float inv = __int_as_float((127 - k) << 23);  // 2^-k, exact
-  unsigned short h[12];
+  unsigned int h[10];
 #pragma unroll
   for (int i = 0; i < 9; ++i) h[i] = __half_as_ushort(__float2half_rn(v[i] * inv));
-  h[9] = (unsigned short)(short)k;
-  h[10] = h[11] = 0;
-#pragma unroll
-  for (int j = 0; j < 3; ++j)
-    out[j] = make_uint2((unsigned int)h[4 * j] | ((unsigned int)h[4 * j + 1] << 16),
-                        (unsigned int)h[4 * j + 2] | ((unsigned int)h[4 * j + 3] << 16));
+  h[9] = (unsigned int)k & 0xffffu;
+  lo = make_uint4(h[0] | (h[1] << 16), h[2] | (h[3] << 16), h[4] | (h[5] << 16), h[6] | (h[7] << 16));
+  hi = h[8] | (h[9] << 16);
 }
 
 template <typename S, bool XF, int HB, bool H16 = false>
 __global__ void __launch_bounds__(HB, (sizeof(S) == 8 ? 256 : 512) / HB)
     elem_hessian_kernel(ElemFP64 e64, ElemFP32 e32, const double* __restrict__ X, const double* __restrict__ u,
                         const float4* __restrict__ xf, S dt2, int spsd, S* __restrict__ Kbuf) {
-  __shared__ S stage[HB * (H16 ? 60 : 90)];
-  const int nt = e64.nt;
-  const int e0 = blockIdx.x * HB;
-  const int e = e0 + threadIdx.x;
-  if (e < nt) {
-    element_hessian_blocks<S, XF>(e64, e32, X, u, xf, dt2, spsd, e, [&](int v, int w, const S* bv) {
-      const int blk = upper_block_id(v, w);
-      if constexpr (H16) {
-        // packed straight from registers: thread t's 30 words at 30 t (the element's global order)
-        pack_block16(bv, reinterpret_cast<uint2*>(stage) + threadIdx.x * 30 + 3 * blk);
-      } else {
-#pragma unroll
-        for (int c = 0; c < 9; ++c) stage[threadIdx.x * 90 + blk * 9 + c] = bv[c];
-      }
-    });
-  }
-  __syncthreads();
-  const int nvalid = min(HB, nt - e0);
-  if constexpr (H16) {
-    const uint2* src = reinterpret_cast<const uint2*>(stage);
-    uint2* dst = reinterpret_cast<uint2*>(Kbuf) + (size_t)e0 * 30;
-    for (int i = threadIdx.x; i < nvalid * 30; i += HB) dst[i] = src[i];
-  } else {
-    S* dst = Kbuf + (size_t)e0 * 90;
-    for (int i = threadIdx.x; i < nvalid * 90; i += HB) dst[i] = stage[i];
-  }
+  const int nt = e64.nt, e = blockIdx.x * HB + threadIdx.x;
+  if (e >= nt) return;
+  const size_t n = (size_t)nt * 10;
+  element_hessian_blocks<S, XF>(e64, e32, X, u, xf, dt2, spsd, e, [&](int v, int w, const S* bv) {
+    const size_t i = (size_t)upper_block_id(v, w) * nt + e;
+    if constexpr (H16)
+      pack_block16(bv, reinterpret_cast<uint4*>(Kbuf)[i], reinterpret_cast<unsigned int*>(reinterpret_cast<uint4*>(Kbuf) + n)[i]);
+    else
+      store_kblock<S>(Kbuf, n, i, bv);
+  });
 }
 
 }  // namespace
@@ -714,7 +696,7 @@ void launch_elem_hessian(const ElemFP64& e64, const ElemFP32& e32, const double*
   after_launch("elem_hessian");
 }
 void launch_elem_hessian16(const ElemFP64& e64, const ElemFP32& e32, const double* X, const double* u,
-                           const float4* xf, double dt2, bool spsd, uint2* K16, cudaStream_t st, int block) {
+                           const float4* xf, double dt2, bool spsd, uint4* K16, cudaStream_t st, int block) {
   if (e64.nt <= 0) return;
   float* kb = reinterpret_cast<float*>(K16);
   auto go = [&](auto B) {
@@ -727,7 +709,8 @@ void launch_elem_hessian16(const ElemFP64& e64, const ElemFP32& e32, const doubl
   };
   dispatch_block<32, 64, 128>(block == 0 ? HB : block, go);
   after_launch("elem_hessian16");
-}template void launch_elem_hessian<float>(const ElemFP64&, const ElemFP32&, const double*, const double*,
+}
+template void launch_elem_hessian<float>(const ElemFP64&, const ElemFP32&, const double*, const double*,
                                          const float4*, double, bool, float*, cudaStream_t, int);
 template void launch_elem_hessian<double>(const ElemFP64&, const ElemFP32&, const double*, const double*,
                                           const float4*, double, bool, double*, cudaStream_t, int);

@@ -14,13 +14,17 @@ constexpr int SB = 256;  // block of the slot / row / dof kernels (a multiple of
 // Assembly (update_hessian, time_step.hpp:631-657): each upper slot (one 3x3 vertex-pair block of the
 // symmetric matrix) adds its precomputed list of element blocks (global_composer.hpp:103-119 builds the
 // same map entry by entry) to the consistent-mass block, then applies the Dirichlet identity filter
-// (boundary.hpp:53-67).  One thread per slot, no atomics: deterministic.
-// one element block in the FP16 form of launch_elem_hessian16: three 8-byte words, nine FP16 values and the
-// power-of-two exponent k in word 9; value = half * 2^k (exact in FP32)
-__device__ __forceinline__ void load_block16(const uint2* __restrict__ K16, int blk, float (&kv)[9]) {
-  const uint2* p = K16 + 3 * (size_t)blk;
-  const uint2 w0 = p[0], w1 = p[1], w2 = p[2];
-  const unsigned int u[6] = {w0.x, w0.y, w1.x, w1.y, w2.x, w2.y};
+// (boundary.hpp:53-67).  One thread per slot, no atomics: deterministic.  Bound by the scattered loads of the
+// contributions (24 on the diagonal, about 6 elsewhere): the planes of store_kblock keep a warp's loads close together, and
+// the next two codes are fetched while two blocks are on their way.  1.02M tets, FP16 blocks: 111 us with element-major
+// 24-byte records, 96 with 16 + 4 bytes in that order, 70 as planes by block; 192k tets, FP16 24 -> 15 us, FP32 38 us with
+// a lane a slot on element-major records, 28 with four, 26 now; FP64, 84,474 tets 35 -> 33 (bound by its additions).
+
+// one element block in the FP16 form of launch_elem_hessian16: eight FP16 values, and the ninth with the power-of-two
+// exponent k in the plane after the nb blocks; value = half * 2^k (exact in FP32)
+__device__ __forceinline__ void load_block16(const uint4* __restrict__ K16, size_t nb, int blk, float (&kv)[9]) {
+  const uint4 w = K16[blk];
+  const unsigned int u[5] = {w.x, w.y, w.z, w.w, reinterpret_cast<const unsigned int*>(K16 + nb)[blk]};
   const int k = (int)(short)(unsigned short)(u[4] >> 16);
   const float sc = __int_as_float((127 + k) << 23);
 #pragma unroll
@@ -34,14 +38,14 @@ template <typename S, int B, bool H16 = false>
 __global__ void __launch_bounds__(B)
     assemble_kernel(SellMatrix A, const int* __restrict__ cptr, const int* __restrict__ csrc,
                     const S* __restrict__ Kbuf, const S* __restrict__ slot_mass, const uint8_t* __restrict__ mask,
-                    int filter, S* __restrict__ vals, V4<S>* __restrict__ dinv, int precond) {
+                    int filter, S* __restrict__ vals, V4<S>* __restrict__ dinv, int precond, size_t nb) {
   const int q = blockIdx.x * B + threadIdx.x;
   if (q >= A.nslots) return;
   S acc[9];
 #pragma unroll
   for (int i = 0; i < 9; ++i) acc[i] = S(0);
   if constexpr (H16) {
-    const uint2* K16 = reinterpret_cast<const uint2*>(Kbuf);
+    const uint4* K16 = reinterpret_cast<const uint4*>(Kbuf);
     const int c1 = cptr[q + 1];
     int c = cptr[q];
     auto add16 = [&](int code, const float (&kv)[9]) {
@@ -55,18 +59,21 @@ __global__ void __launch_bounds__(B)
           for (int b = 0; b < 3; ++b) acc[a * 3 + b] += kv[b * 3 + a];
       }
     };
+    int n0 = c < c1 ? csrc[c] : 0, n1 = c + 1 < c1 ? csrc[c + 1] : 0;
     for (; c + 2 <= c1; c += 2) {
-      const int code0 = csrc[c], code1 = csrc[c + 1];
+      const int code0 = n0, code1 = n1;
       float kv0[9], kv1[9];
-      load_block16(K16, code0 & 0x7fffffff, kv0);
-      load_block16(K16, code1 & 0x7fffffff, kv1);
+      n0 = c + 2 < c1 ? csrc[c + 2] : 0;
+      n1 = c + 3 < c1 ? csrc[c + 3] : 0;
+      load_block16(K16, nb, code0 & 0x7fffffff, kv0);
+      load_block16(K16, nb, code1 & 0x7fffffff, kv1);
       add16(code0, kv0);
       add16(code1, kv1);
     }
     if (c < c1) {
-      const int code = csrc[c];
+      const int code = n0;
       float kv[9];
-      load_block16(K16, code & 0x7fffffff, kv);
+      load_block16(K16, nb, code & 0x7fffffff, kv);
       add16(code, kv);
     }
   } else if (Kbuf != nullptr) {
@@ -84,25 +91,21 @@ __global__ void __launch_bounds__(B)
     };
     const int c1 = cptr[q + 1];
     int c = cptr[q];
+    int n0 = c < c1 ? csrc[c] : 0, n1 = c + 1 < c1 ? csrc[c + 1] : 0;
     for (; c + 2 <= c1; c += 2) {
-      const int code0 = csrc[c], code1 = csrc[c + 1];
-      const S* k0 = Kbuf + (size_t)(code0 & 0x7fffffff) * 9;
-      const S* k1 = Kbuf + (size_t)(code1 & 0x7fffffff) * 9;
+      const int code0 = n0, code1 = n1;
+      n0 = c + 2 < c1 ? csrc[c + 2] : 0;
+      n1 = c + 3 < c1 ? csrc[c + 3] : 0;
       S kv0[9], kv1[9];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) {
-        kv0[i] = k0[i];
-        kv1[i] = k1[i];
-      }
+      load_kblock<S>(Kbuf, nb, code0 & 0x7fffffff, kv0);
+      load_kblock<S>(Kbuf, nb, code1 & 0x7fffffff, kv1);
       add(code0, kv0);
       add(code1, kv1);
     }
     if (c < c1) {
-      const int code = csrc[c];
-      const S* k = Kbuf + (size_t)(code & 0x7fffffff) * 9;
+      const int code = n0;
       S kv[9];
-#pragma unroll
-      for (int i = 0; i < 9; ++i) kv[i] = k[i];
+      load_kblock<S>(Kbuf, nb, code & 0x7fffffff, kv);
       add(code, kv);
     }
   }
@@ -128,74 +131,6 @@ __global__ void __launch_bounds__(B)
   const size_t base = sell_base(q);
 #pragma unroll
   for (int c = 0; c < 9; ++c) vals[base + 32 * c] = acc[c];
-}
-
-// The FP32-block assembly with four lanes a slot, three of them a row each.  The element blocks lie anywhere in memory: a
-// lane per slot touches 32 blocks a load and takes nine loads a block, a quad per slot eight and three.  192k tets: 28.6 us
-// against 38.2 with a lane per slot; FP64 blocks (26.1 against 22.2 at 30,498 tets) and FP16 blocks, which a lane reads in
-// three loads (119 against 110 at 1.02M tets), keep the lane.  Each entry adds its blocks in the list's order, as there.
-template <int B>
-__global__ void __launch_bounds__(B)
-    assemble_quad_kernel(SellMatrix A, const int* __restrict__ cptr, const int* __restrict__ csrc,
-                         const float* __restrict__ Kbuf, const float* __restrict__ slot_mass,
-                         const uint8_t* __restrict__ mask, int filter, float* __restrict__ vals, float4* __restrict__ dinv,
-                         int precond) {
-  const long long i = (long long)blockIdx.x * B + threadIdx.x;
-  const int q = (int)(i >> 2), r = (int)(i & 3), rr = min(r, 2), lane = threadIdx.x & 31;
-  if (q >= A.nslots) return;  // whole warps: nslots is a multiple of 32
-  float acc[3] = {0.f, 0.f, 0.f};  // row r of the slot's block
-  const int c1 = cptr[q + 1];
-  auto load = [&](int code, float (&v)[3]) {  // row r of the element's block, or of its transpose
-    const float* k = Kbuf + (size_t)(code & 0x7fffffff) * 9 + (code >= 0 ? 3 * rr : rr);
-    const int step = code >= 0 ? 1 : 3;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) v[j] = k[j * step];
-  };
-  int c = cptr[q];
-  for (; c + 2 <= c1; c += 2) {
-    const int code0 = csrc[c], code1 = csrc[c + 1];
-    float v0[3], v1[3];
-    load(code0, v0);
-    load(code1, v1);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) acc[j] = (acc[j] + v0[j]) + v1[j];
-  }
-  if (c < c1) {
-    float v[3];
-    load(csrc[c], v);
-#pragma unroll
-    for (int j = 0; j < 3; ++j) acc[j] += v[j];
-  }
-  const int u = A.slot_row[q];
-  if (u >= 0) {
-    const float m = slot_mass[q];
-#pragma unroll
-    for (int j = 0; j < 3; ++j)
-      if (j == r) acc[j] += m;
-    const int w = A.sl_col[q];
-    if (filter) {
-      const int mu = mask[u], mw = mask[w];
-      if (mu | mw) {
-#pragma unroll
-        for (int j = 0; j < 3; ++j)
-          if (((mu >> r) & 1) || ((mw >> j) & 1)) acc[j] = (u == w && r == j) ? 1.f : 0.f;
-      }
-    }
-    if (dinv != nullptr && u == w) {
-      const unsigned int quad = 0xfu << (lane & 28);
-      float full[9];
-#pragma unroll
-      for (int k = 0; k < 3; ++k)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) full[3 * k + j] = __shfl_sync(quad, acc[j], (lane & 28) + k);
-      if (r == 0) precond_rows<float>(full, precond, dinv + 3 * (size_t)u);
-    }
-  }
-  if (r < 3) {
-    const size_t base = sell_base(q) + 96 * r;
-#pragma unroll
-    for (int j = 0; j < 3; ++j) vals[base + 32 * j] = acc[j];
-  }
 }
 
 // Symmetric SELL-32 3x3-block SpMV, one thread per block row; a warp walks one slice in lockstep so every
@@ -1485,27 +1420,20 @@ void launch_kron_extract(const SellMatrix& A, const S* vals, S* svals, int* not_
 }
 
 template <typename S>
-void launch_assemble(const SellMatrix& A, const int* cptr, const int* csrc, const S* Kbuf, const S* slot_mass,
+void launch_assemble(const SellMatrix& A, const int* cptr, const int* csrc, const S* Kbuf, size_t nb, const S* slot_mass,
                      const uint8_t* mask, bool filter, S* vals, V4<S>* dinv, int precond, cudaStream_t st,
                      int block) {
   if (A.nslots <= 0) return;
   auto go = [&](auto Bc) {
     constexpr int b = decltype(Bc)::value;
-    if constexpr (sizeof(S) == 4) {
-      if (Kbuf != nullptr) {
-        assemble_quad_kernel<b><<<div_up(4LL * A.nslots, b), b, 0, st>>>(A, cptr, csrc, Kbuf, slot_mass, mask, filter ? 1 : 0,
-                                                                         vals, dinv, precond);
-        return;
-      }
-    }
     assemble_kernel<S, b><<<div_up(A.nslots, b), b, 0, st>>>(A, cptr, csrc, Kbuf, slot_mass, mask, filter ? 1 : 0,
-                                                             vals, dinv, precond);
+                                                             vals, dinv, precond, nb);
   };
   dispatch_block<128, 256, 512>(block == 0 ? SB : block, go);
   after_launch("assemble");
 }
 
-void launch_assemble16(const SellMatrix& A, const int* cptr, const int* csrc, const uint2* K16, const float* slot_mass,
+void launch_assemble16(const SellMatrix& A, const int* cptr, const int* csrc, const uint4* K16, size_t nb, const float* slot_mass,
                        const uint8_t* mask, bool filter, float* vals, float4* dinv, int precond, cudaStream_t st,
                        int block) {
   if (A.nslots <= 0) return;
@@ -1513,7 +1441,7 @@ void launch_assemble16(const SellMatrix& A, const int* cptr, const int* csrc, co
   auto go = [&](auto Bc) {
     constexpr int b = decltype(Bc)::value;
     assemble_kernel<float, b, true><<<div_up(A.nslots, b), b, 0, st>>>(A, cptr, csrc, kb, slot_mass, mask,
-                                                                        filter ? 1 : 0, vals, dinv, precond);
+                                                                        filter ? 1 : 0, vals, dinv, precond, nb);
   };
   dispatch_block<128, 256, 512>(block == 0 ? SB : block, go);
   after_launch("assemble16");
@@ -1797,7 +1725,7 @@ void launch_instance_norms(int ninst, const int* voff, const double* g, double* 
 }
 
 #define SSIM_INST(S)                                                                                              \
-  template void launch_assemble<S>(const SellMatrix&, const int*, const int*, const S*, const S*, const uint8_t*, \
+  template void launch_assemble<S>(const SellMatrix&, const int*, const int*, const S*, size_t, const S*, const uint8_t*, \
                                    bool, S*, V4<S>*, int, cudaStream_t, int);                                     \
   template void launch_spmv<S>(const SellMatrix&, const S*, const V4<S>*, V4<S>*, cudaStream_t);                 \
   template void launch_kron_extract<S>(const SellMatrix&, const S*, S*, int*, cudaStream_t);                     \

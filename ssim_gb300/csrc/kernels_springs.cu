@@ -4,7 +4,7 @@
 // literature uses (Liu et al., "Fast Simulation of Mass-Spring Systems", SIGGRAPH Asia 2013).
 //
 // Springs are 2-vertex cells: the vertex gather, the block pattern, the atomic-free assembly and the
-// PCG are the tet ones; the spring forces go to one 4-wide vector a spring, the Hessian blocks to Kbuf[s][3][9] (upper
+// PCG are the tet ones; the spring forces go to one 4-wide vector a spring, the Hessian blocks to Kbuf (upper
 // vertex blocks (0,0), (0,1), (1,1)).
 #include "kernels.cuh"
 
@@ -275,13 +275,13 @@ __global__ void __launch_bounds__(PB)
 #pragma unroll
     for (int b = 0; b < 3; ++b)
       K[a * 3 + b] = (S)(dt2 * k * ((1.0 - c) * n[a] * n[b] + (a == b ? c : 0.0)));
-  S* o = Kbuf + (size_t)s * 27;
+  S M[9];
 #pragma unroll
-  for (int q = 0; q < 9; ++q) {
-    o[q] = K[q];
-    o[9 + q] = -K[q];
-    o[18 + q] = K[q];
-  }
+  for (int q = 0; q < 9; ++q) M[q] = -K[q];
+  const size_t ns = sp.ns;
+  store_kblock<S>(Kbuf, 3 * ns, s, K);
+  store_kblock<S>(Kbuf, 3 * ns, ns + s, M);
+  store_kblock<S>(Kbuf, 3 * ns, 2 * ns + s, K);
 }
 
 }  // namespace

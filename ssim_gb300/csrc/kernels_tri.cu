@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(TB)
     B[0][cc] = -(B[1][cc] + B[2][cc]);
   }
   const S sc = (S)(dt2 * el.vol[e]);
-  S* out = Kbuf + (size_t)e * 54;
   int blk = 0;
 #pragma unroll
   for (int v = 0; v < 3; ++v)
@@ -276,8 +275,7 @@ __global__ void __launch_bounds__(TB)
           }
           K[a * 3 + b] = sc * t;
         }
-#pragma unroll
-      for (int k = 0; k < 9; ++k) out[blk * 9 + k] = K[k];
+      store_kblock<S>(Kbuf, (size_t)6 * el.nt, (size_t)blk * el.nt + e, K);
       ++blk;
     }
 }

@@ -75,7 +75,7 @@ static void export_values(TimeStep& t, int which, double* out) {
   const S* src = s.vals.p;
   if (which == SSIM_GB_MASS || which == SSIM_GB_MASS_FILTERED) {
     s.mvals.alloc(9 * (size_t)t.topo.nslots);
-    ssim_gb::launch_assemble<S>(t.A(), t.cptr.p, t.csrc.p, nullptr, s.slot_mass.p, t.mask.p,
+    ssim_gb::launch_assemble<S>(t.A(), t.cptr.p, t.csrc.p, nullptr, 0, s.slot_mass.p, t.mask.p,
                                 which == SSIM_GB_MASS_FILTERED, s.mvals.p, nullptr, 0, t.stream);
     src = s.mvals.p;
   }
@@ -91,7 +91,7 @@ static void do_spmv(TimeStep& t, int which, const double* x, double* y) {
   const S* vals = s.vals.p;
   if (which == SSIM_GB_MASS || which == SSIM_GB_MASS_FILTERED) {
     s.mvals.alloc(9 * (size_t)t.topo.nslots);
-    ssim_gb::launch_assemble<S>(t.A(), t.cptr.p, t.csrc.p, nullptr, s.slot_mass.p, t.mask.p,
+    ssim_gb::launch_assemble<S>(t.A(), t.cptr.p, t.csrc.p, nullptr, 0, s.slot_mass.p, t.mask.p,
                                 which == SSIM_GB_MASS_FILTERED, s.mvals.p, nullptr, 0, t.stream);
     vals = s.mvals.p;
   }

@@ -56,7 +56,7 @@ struct DBuf {
 template <typename S>
 struct Solver {
   DBuf<S> K, vals, mvals;  // element blocks, system values, mass values (SELL)
-  DBuf<uint2> K16;         // element blocks in FP16 (launch_elem_hessian16), mixed Newton only
+  DBuf<uint4> K16;         // element blocks in FP16 (launch_elem_hessian16), mixed Newton only
   DBuf<S> slot_mass;
   DBuf<V4<S>> x, r, z, p0, p1, q, dinv, tmp;
   DBuf<V4<S>> pm;  // the pipelined PCG's double-buffered m = M w (2 nv), allocated on first use
@@ -578,7 +578,15 @@ struct TimeStep {
     sl_col.upload(topo.sl_col, stream);
     slot_row.upload(topo.slot_row, stream);
     cptr.upload(topo.cptr, stream);
-    csrc.upload(topo.csrc, stream);
+    {  // element-major codes e nb + b to the planes' b nt + e (store_kblock)
+      const int nb = topo.cv * (topo.cv + 1) / 2;
+      std::vector<int32_t> src(topo.csrc);
+      for (auto& c : src) {
+        const uint32_t i = (uint32_t)c & 0x7fffffffu;
+        c = (int32_t)(((i % nb) * (uint32_t)nt + i / nb) | ((uint32_t)c & 0x80000000u));
+      }
+      csrc.upload(src, stream);
+    }
     bptr.upload(topo.bptr, stream);
     slot_k.upload(topo.slot_k, stream);
     slot_kt.upload(topo.slot_kt, stream);
@@ -752,7 +760,7 @@ struct TimeStep {
       s.slot_pd.upload(pds, stream);
       s.pd_vals.alloc(9 * (size_t)topo.nslots);
       s.pd_dinv.alloc(3 * (size_t)nv);
-      launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, s.slot_pd.p, mask.p, true, s.pd_vals.p, s.pd_dinv.p, 2, stream);
+      launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, 0, s.slot_pd.p, mask.p, true, s.pd_vals.p, s.pd_dinv.p, 2, stream);
       pd_kron_form<S>(s);
       return;
     }
@@ -781,7 +789,7 @@ struct TimeStep {
     s.slot_pd.upload(pds, stream);
     s.pd_vals.alloc(9 * (size_t)topo.nslots);
     s.pd_dinv.alloc(3 * (size_t)nv);
-    launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, s.slot_pd.p, mask.p, true, s.pd_vals.p, s.pd_dinv.p, 2, stream);
+    launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, 0, s.slot_pd.p, mask.p, true, s.pd_vals.p, s.pd_dinv.p, 2, stream);
     pd_kron_form<S>(s);
   }
 
@@ -904,6 +912,7 @@ struct TimeStep {
   template <typename S>
   Solver<S>& solver();
 
+  size_t nkblocks() const { return (size_t)(topo.cv * (topo.cv + 1) / 2) * nt; }  // element blocks of an assembly
   // update_hessian (time_step.hpp:626-658)
   // k16: the element blocks in FP16 (tets, mixed precision; for assemblies whose solve runs on the FP16 copy)
   template <typename S>
@@ -922,18 +931,18 @@ struct TimeStep {
     }
     if constexpr (std::is_same<S, float>::value) {
       if (k16 && !springs && !tri2d) {
-        s.K16.alloc((size_t)30 * nt);
+        s.K16.alloc(nkblocks() + div_up((long long)nkblocks(), 4));
         launch_elem_hessian16(e64(), e32(), dX.p, next.p, xfp, dt * dt, spsd, s.K16.p, stream, shapes.hess);
         if (profiling) prof_end(e0, e1, PK_HESS, 0);
         if (profiling) prof_begin(e0, e1);
-        launch_assemble16(A(), cptr.p, csrc.p, s.K16.p, s.slot_mass.p, mask.p, filter, s.vals.p, s.dinv.p,
+        launch_assemble16(A(), cptr.p, csrc.p, s.K16.p, nkblocks(), s.slot_mass.p, mask.p, filter, s.vals.p, s.dinv.p,
                           params.precond, stream, shapes.assem);
         if (profiling) prof_end(e0, e1, PK_ASM, 0);
         return;
       }
     }
     // two kernels through the per-element block buffer (allocated on first use)
-    s.K.alloc((size_t)9 * (topo.cv * (topo.cv + 1) / 2) * nt);
+    s.K.alloc(9 * nkblocks());
     if (springs)
       launch_spring_hessian<S>(spd(), next.p, dt * dt, spsd, s.K.p, stream);
     else if (tri2d)
@@ -943,7 +952,7 @@ struct TimeStep {
                              shapes.hess);
     if (profiling) prof_end(e0, e1, PK_HESS, 0);
     if (profiling) prof_begin(e0, e1);
-    launch_assemble<S>(A(), cptr.p, csrc.p, s.K.p, s.slot_mass.p, mask.p, filter, s.vals.p, s.dinv.p,
+    launch_assemble<S>(A(), cptr.p, csrc.p, s.K.p, nkblocks(), s.slot_mass.p, mask.p, filter, s.vals.p, s.dinv.p,
                        params.precond, stream, shapes.assem);
     if (profiling) prof_end(e0, e1, PK_ASM, 0);
   }
@@ -1450,7 +1459,7 @@ struct TimeStep {
     }
     if (projected) *projected = proj;
     s.mvals.alloc(9 * (size_t)topo.nslots);
-    launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, s.slot_mass.p, mask.p, false, s.mvals.p, nullptr, 0, stream);
+    launch_assemble<S>(A(), cptr.p, csrc.p, nullptr, 0, s.slot_mass.p, mask.p, false, s.mvals.p, nullptr, 0, stream);
     launch_spmv<S>(A(), s.mvals.p, s.x.p, s.q.p, stream);
     launch_adj_finish<S>(nv, dt, s.q.p, dof_type.p, gprev.p, ubar, vbar, stream);
     launch_adj_material<S>(e64(), dX.p, next.p, s.x.p, dt * dt, ebar, stream);
@@ -1918,7 +1927,7 @@ struct TimeStep {
     t.hessian_block = 0;
     t.assembly_block = 0;
     double hbest = 1e300, abest = 1e300;
-    s.K.alloc((size_t)9 * (topo.cv * (topo.cv + 1) / 2) * nt);
+    s.K.alloc(9 * nkblocks());
     if (tets) {
       for (int b : {32, 64, 128}) {
         const double ms = time_launches(
@@ -1932,7 +1941,7 @@ struct TimeStep {
     }
     for (int b : {128, 256, 512}) {
       const double ms = time_launches([&] {
-        launch_assemble<S>(A(), cptr.p, csrc.p, s.K.p, s.slot_mass.p, mask.p, true, s.vals.p, s.dinv.p,
+        launch_assemble<S>(A(), cptr.p, csrc.p, s.K.p, nkblocks(), s.slot_mass.p, mask.p, true, s.vals.p, s.dinv.p,
                            params.precond, stream, b);
       });
       ++count;
