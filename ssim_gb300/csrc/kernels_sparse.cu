@@ -11,6 +11,13 @@ namespace {
 constexpr int SB = 256;  // block of the slot / row / dof kernels (a multiple of the 32-row slice)
 
 
+__global__ void __launch_bounds__(SB) plane_codes_kernel(int n, int nb, int nt, int* __restrict__ codes) {
+  const unsigned int c = (unsigned int)blockIdx.x * SB + threadIdx.x;
+  if (c >= (unsigned int)n) return;
+  const unsigned int w = (unsigned int)codes[c], i = w & 0x7fffffffu, e = i / (unsigned int)nb;
+  codes[c] = (int)(((i - e * nb) * (unsigned int)nt + e) | (w & 0x80000000u));
+}
+
 // Assembly (update_hessian, time_step.hpp:631-657): each upper slot (one 3x3 vertex-pair block of the
 // symmetric matrix) adds its precomputed list of element blocks (global_composer.hpp:103-119 builds the
 // same map entry by entry) to the consistent-mass block, then applies the Dirichlet identity filter
@@ -1417,6 +1424,12 @@ void launch_kron_extract(const SellMatrix& A, const S* vals, S* svals, int* not_
   if (A.nslots <= 0) return;
   kron_extract_kernel<S><<<div_up(A.nslots, SB), SB, 0, st>>>(A.nslots, vals, svals, not_kron);
   after_launch("kron_extract");
+}
+
+void launch_plane_codes(int n, int nb, int nt, int* codes, cudaStream_t st) {
+  if (n <= 0) return;
+  plane_codes_kernel<<<div_up(n, SB), SB, 0, st>>>(n, nb, nt, codes);
+  after_launch("plane_codes");
 }
 
 template <typename S>

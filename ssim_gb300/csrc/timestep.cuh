@@ -578,15 +578,8 @@ struct TimeStep {
     sl_col.upload(topo.sl_col, stream);
     slot_row.upload(topo.slot_row, stream);
     cptr.upload(topo.cptr, stream);
-    {  // element-major codes e nb + b to the planes' b nt + e (store_kblock)
-      const int nb = topo.cv * (topo.cv + 1) / 2;
-      std::vector<int32_t> src(topo.csrc);
-      for (auto& c : src) {
-        const uint32_t i = (uint32_t)c & 0x7fffffffu;
-        c = (int32_t)(((i % nb) * (uint32_t)nt + i / nb) | ((uint32_t)c & 0x80000000u));
-      }
-      csrc.upload(src, stream);
-    }
+    csrc.upload(topo.csrc, stream);
+    launch_plane_codes((int)topo.csrc.size(), topo.cv * (topo.cv + 1) / 2, nt, csrc.p, stream);
     bptr.upload(topo.bptr, stream);
     slot_k.upload(topo.slot_k, stream);
     slot_kt.upload(topo.slot_kt, stream);
