@@ -316,17 +316,18 @@ struct HalfMatrix {
   const int* off;       // [nslices + 1] entry offset of each slice (multiple of 32)
   const int* col;       // [nfs] block column, own row for padding
   const uint4* v8;      // [nfs] values 0..7 of the scaled block (row-major), FP16
-  const uint16_t* v1;   // [nfs] value 8, FP16 bits
+  const uint16_t* v1;   // [nfs][vs] value 8, FP16 bits, then (vs = 2) the column less the slice's first row, 16 bits signed
   const float4* scale;  // [nv] s_a
   const float4* iscale; // [nv] 1 / s_a
+  int vs;               // 16-bit words an entry in v1: 2 where every column lies within 2^15 rows of its slice, else 1
 };
 // scale, inverse scale and the scaled block-Jacobi rows (precond 0 / 1 / 2 on S B S) from the diagonal blocks
 // of the FP32 symmetric values
 void launch_half_prepare(const SellMatrix& A, const float* vals, int precond, float4* scale, float4* iscale,
                          float4* dinv16, cudaStream_t st);
-// the FP16 values of every full entry from the FP32 symmetric values (src: build_full_sell's sources)
+// the FP16 values (and packed columns, vs = 2) of every full entry from the FP32 symmetric values (src: build_full_sell's sources)
 void launch_half_convert(const SellMatrix& A, const int* off, const int* col, const int* src, const float* vals,
-                         const float4* scale, uint4* v8, uint16_t* v1, cudaStream_t st);
+                         const float4* scale, uint4* v8, uint16_t* v1, int vs, cudaStream_t st);
 // PCG setup in the scaled space: r~ = S (negate ? -b : b), z~ = M~ r~, x = p0 = 0; partials (r~, z~) and
 // (r, r) of the unscaled residual
 void launch_pcg_setup_half(const HalfMatrix& H, const double* b, const float4* dinv16, float4* x, float4* r, float4* z,

@@ -280,6 +280,7 @@ __device__ __forceinline__ void sym_unit(const SellMatrix& A, const S* __restric
 struct HalfPlan {
   int grid, T, spc, res, tile, cached;  // spc: most slices of a block; res, tile in slices
   int cache_entries;                    // most entries of a block (when cached)
+  int packed;                           // 16-bit columns (HalfMatrix vs = 2)
   int keep;                             // slices whose entries L2 is asked to keep; -1: no hints
   size_t smem;
 };
@@ -334,13 +335,30 @@ __device__ __forceinline__ int ld_hint(const int* p, unsigned long long pol) {
 // Entries k0, k0 + T, ... of a slice of width W (col / v8 / v1: its first entry, this lane): four at a time with all
 // their loads in flight.  The kernel is bound by the instructions it issues (59% of the issue slots in a first
 // version with run-time strides and a predicate per entry), so T is a compile-time stride (immediate offsets) and
-// only a unit's ragged end tests the width.
-template <int T, bool HINT>
-__device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const uint16_t* v1, int W, int k0,
+// only a unit's ragged end tests the width.  PACKED: the ninth value and the column's distance from the slice's first row
+// share a word, 20 bytes and two loads an entry instead of 22 and three (32-bit columns are kept for patterns that reach
+// further than 2^15 rows).  Whole solves: 1.02M-tet beam 662 -> 652 us, 192k-tet bar 283 -> 279, 64-cube batch 1,734 ->
+// 1,648, where the entries come from DRAM.
+template <int T, bool HINT, bool PACKED>
+__device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const uint16_t* v1, int W, int k0, int row0,
                                           const float4* x, unsigned long long pol, float& a0, float& a1, float& a2) {
-  col += 32 * k0;
+  const int* words = PACKED ? reinterpret_cast<const int*>(v1) + 32 * k0 : nullptr;
   v8 += 32 * k0;
-  v1 += 32 * k0;
+  if constexpr (!PACKED) {
+    col += 32 * k0;
+    v1 += 32 * k0;
+  }
+  // column and ninth value of the entry at o
+  auto load_ch = [&](int o, int& c, uint16_t& h) {
+    if constexpr (PACKED) {
+      const int w = ld_hint<HINT>(words + o, pol);
+      c = row0 + (w >> 16);
+      h = (uint16_t)w;
+    } else {
+      c = ld_hint<HINT>(col + o, pol);
+      h = ld_hint<HINT>(v1 + o, pol);
+    }
+  };
   int n = W - k0;  // entries 0, T, ... < n remain
   for (; n > 3 * T; n -= 4 * T) {
     int c[4];
@@ -348,25 +366,29 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
     uint16_t h[4];
     float4 xv[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) c[j] = ld_hint<HINT>(col + 32 * T * j, pol);
+    for (int j = 0; j < 4; ++j) load_ch(32 * T * j, c[j], h[j]);
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      p[j] = ld_hint<HINT>(v8 + 32 * T * j, pol);
-      h[j] = ld_hint<HINT>(v1 + 32 * T * j, pol);
-    }
+    for (int j = 0; j < 4; ++j) p[j] = ld_hint<HINT>(v8 + 32 * T * j, pol);
 #pragma unroll
     for (int j = 0; j < 4; ++j) xv[j] = x[c[j]];
 #pragma unroll
     for (int j = 0; j < 4; ++j) half_fma(p[j], h[j], xv[j], a0, a1, a2);
-    col += 128 * T;
     v8 += 128 * T;
-    v1 += 128 * T;
+    if constexpr (PACKED) {
+      words += 128 * T;
+    } else {
+      col += 128 * T;
+      v1 += 128 * T;
+    }
   }
   if (n > 0) {  // one to three entries: the missing ones repeat the first with a zero vector
     const int o1 = n > T ? 32 * T : 0, o2 = n > 2 * T ? 64 * T : 0;
-    const int c0 = ld_hint<HINT>(col, pol), c1 = ld_hint<HINT>(col + o1, pol), c2 = ld_hint<HINT>(col + o2, pol);
+    int c0, c1, c2;
+    uint16_t h0, h1, h2;
+    load_ch(0, c0, h0);
+    load_ch(o1, c1, h1);
+    load_ch(o2, c2, h2);
     const uint4 p0 = ld_hint<HINT>(v8, pol), p1 = ld_hint<HINT>(v8 + o1, pol), p2 = ld_hint<HINT>(v8 + o2, pol);
-    const uint16_t h0 = ld_hint<HINT>(v1, pol), h1 = ld_hint<HINT>(v1 + o1, pol), h2 = ld_hint<HINT>(v1 + o2, pol);
     const float4 x0 = x[c0];
     float4 x1 = x[c1], x2 = x[c2];
     if (n <= T) x1 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -389,7 +411,7 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
 // drifts from the true one with the iterations and the condition number, so after pipe_iters iterations the
 // solve continues as Chronopoulos-Gear PCG from the same state (w = A u recomputed, two exchanges a round).
 // CACHED: the block's matrix entries are in shared memory too.  HINT: they are loaded with L2 priorities (pl.keep).
-template <bool CACHED, int T, bool HINT = false>
+template <bool CACHED, int T, bool HINT, bool PACKED>
 __global__ void __launch_bounds__(HT, 1)
     resident_half_kernel(HalfMatrix H, const float4* __restrict__ dinv, float4* x, float4* r, float4* z, float4* p,
                          float4* sv, float4* w, float4* m, HalfSolveArgs a, HalfPlan pl, Reduce red, GridExchange gx) {
@@ -401,6 +423,7 @@ __global__ void __launch_bounds__(HT, 1)
   const int nv = H.nv, nsl = (nv + 31) >> 5;
   constexpr int lt = T == 8 ? 3 : 2;
   static_assert(T == 1 << lt, "T is 4 or 8");
+  constexpr int VS = PACKED ? 2 : 1;
   const int s0 = (int)((long long)blockIdx.x * nsl / gridDim.x), ns = (int)((long long)(blockIdx.x + 1) * nsl / gridDim.x) - s0;
   const int RS = 32 * pl.res, PR = 32 * pl.tile;
   // shared memory: cached matrix entries (16-byte values first), row state, unit partials, per-slice dots, offsets
@@ -409,8 +432,9 @@ __global__ void __launch_bounds__(HT, 1)
   float* pb = st + (size_t)kHalfState * RS;
   float* shw = pb + (size_t)3 * T * PR;
   int* off = reinterpret_cast<int*>(shw + 4 * pl.spc);
+  // the cached entries' columns and ninth values: one word (PACKED), or 4-byte columns and then 2-byte values
   int* ccol = off + pl.spc + 1;
-  uint16_t* c1 = reinterpret_cast<uint16_t*>(ccol + pl.cache_entries);
+  uint16_t* c1 = reinterpret_cast<uint16_t*>(PACKED ? ccol : ccol + pl.cache_entries);
   if (tid == 0) xs.fail = 0;
   for (int i = tid; i <= ns; i += HT) off[i] = H.off[s0 + i];
   __syncthreads();
@@ -419,8 +443,12 @@ __global__ void __launch_bounds__(HT, 1)
     const int ne = off[ns] - e0;
     for (int i = tid; i < ne; i += HT) {
       c8[i] = H.v8[e0 + i];
-      ccol[i] = H.col[e0 + i];
-      c1[i] = H.v1[e0 + i];
+      if constexpr (PACKED) {
+        ccol[i] = reinterpret_cast<const int*>(H.v1)[e0 + i];
+      } else {
+        ccol[i] = H.col[e0 + i];
+        c1[i] = H.v1[e0 + i];
+      }
     }
   }
   unsigned long long nx = 0;  // exchanges so far
@@ -438,11 +466,12 @@ __global__ void __launch_bounds__(HT, 1)
       const int b = off[t0 + (i >> lt)], W = (off[t0 + (i >> lt) + 1] - b) >> 5;
       float a0 = 0.f, a1 = 0.f, a2 = 0.f;
       if constexpr (CACHED)
-        half_unit<T, false>(ccol + (b - e0) + lane, c8 + (b - e0) + lane, c1 + (b - e0) + lane, W, i & (T - 1), v, 0, a0, a1,
-                            a2);
+        half_unit<T, false, PACKED>(ccol + (b - e0) + lane, c8 + (b - e0) + lane, c1 + VS * (b - e0 + lane), W, i & (T - 1),
+                                    32 * (s0 + t0 + (i >> lt)), v, 0, a0, a1, a2);
       else
-        half_unit<T, HINT>(H.col + b + lane, H.v8 + b + lane, H.v1 + b + lane, W, i & (T - 1), v,
-                           t0 + (i >> lt) < pl.keep ? pol_keep : pol_pass, a0, a1, a2);
+        half_unit<T, HINT, PACKED>(H.col + b + lane, H.v8 + b + lane, H.v1 + (size_t)VS * (b + lane), W, i & (T - 1),
+                                   32 * (s0 + t0 + (i >> lt)), v, t0 + (i >> lt) < pl.keep ? pol_keep : pol_pass, a0, a1,
+                                   a2);
       float* o = pb + (size_t)3 * (i & (T - 1)) * PR + 32 * (i >> lt) + lane;
       o[0] = a0;
       o[PR] = a1;
@@ -1013,7 +1042,8 @@ constexpr size_t kSmemReserve = 8 * 1024;  // static shared memory and the 1 KB 
 
 size_t half_smem(const HalfPlan& p) {
   const size_t f = (size_t)kHalfState * 32 * p.res + (size_t)3 * p.T * 32 * p.tile + 4 * (size_t)p.spc;
-  return (size_t)16 * p.cache_entries + 4 * f + 4 * ((size_t)p.spc + 1) + 6 * (size_t)p.cache_entries + 64;
+  return (size_t)16 * p.cache_entries + 4 * f + 4 * ((size_t)p.spc + 1) +
+         (p.packed ? 4 : 6) * (size_t)p.cache_entries + 64;
 }
 
 }  // namespace
@@ -1029,9 +1059,9 @@ static GridExchange grid_exchange(const ResidentSync& rs, cudaStream_t st) {
                       (unsigned int)rs.extra, rs.spin_limit > 0 ? rs.spin_limit : (1LL << 21)};
 }
 
-// 22 bytes an entry against the double-buffered m and the vectors of the rows that are not on chip
+// 20 or 22 bytes an entry against the double-buffered m and the vectors of the rows that are not on chip
 static HalfPlan l2_hints(HalfPlan p, int nv, const int32_t* off, size_t l2) {
-  const double matrix = 22.0 * off[div_up(nv, 32)];
+  const double matrix = (p.packed ? 20.0 : 22.0) * off[div_up(nv, 32)];
   const double other = 32.0 * nv + 176.0 * nv * (p.spc - p.res) / std::max(p.spc, 1);
   if (p.grid > 0 && matrix + other > 0.8 * (double)l2)
     p.keep = (int)(p.spc * std::min(1.0, std::max(0.0, 0.6 * (double)l2 - other) / matrix));
@@ -1050,8 +1080,9 @@ static HalfPlan l2_hints(HalfPlan p, int nv, const int32_t* off, size_t l2) {
 //  batches of cubes, 126 MB of L2 (matrix / other bytes, MB; Newton iterations, ms): 77 / 8 6.43 without and 6.77 with
 //  60 MB kept; 92 / 17 10.1, 8.87 with 60; 108 / 28 15.1, 12.9 with 50; 118 / 35 18.0, 15.4 with 40; 157 / 60 22.7, 20.3
 //  with 20; 250 / 122 36.9, 36.6.  So: hints above 0.8 of L2, 0.6 of L2 less the other bytes kept.
-static HalfPlan half_plan(int nv, const int32_t* off, int nsm, size_t smem_max, size_t l2, int max_blocks) {
+static HalfPlan half_plan(int nv, int packed, const int32_t* off, int nsm, size_t smem_max, size_t l2, int max_blocks) {
   HalfPlan p{};
+  p.packed = packed;
   p.keep = -1;
   const int nsl = div_up(nv, 32);
   p.grid = std::max(1, std::min(std::min(nsm, kMaxBlocks), nsl));
@@ -1102,13 +1133,17 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
   int nsm = 0;
   size_t smem_max = 0, l2 = 0;
   if (!resident_device(nsm, smem_max, l2)) return false;
-  HalfPlan pl = half_plan(H.nv, off_host, nsm, smem_max, l2, max_blocks);
+  HalfPlan pl = half_plan(H.nv, H.vs == 2, off_host, nsm, smem_max, l2, max_blocks);
   if (pl.grid < 1) return false;
   pl.smem = half_smem(pl);
-  const void* fn = pl.keep >= 0 ? (const void*)resident_half_kernel<false, 4, true>
-                   : !pl.cached ? (const void*)resident_half_kernel<false, 4>
-                   : pl.T == 4  ? (const void*)resident_half_kernel<true, 4>
-                                : (const void*)resident_half_kernel<true, 8>;
+  auto kernel = [&](auto P) {
+    constexpr bool k = decltype(P)::value;
+    return pl.keep >= 0 ? (const void*)resident_half_kernel<false, 4, true, k>
+           : !pl.cached ? (const void*)resident_half_kernel<false, 4, false, k>
+           : pl.T == 4  ? (const void*)resident_half_kernel<true, 4, false, k>
+                        : (const void*)resident_half_kernel<true, 8, false, k>;
+  };
+  const void* fn = pl.packed ? kernel(std::true_type{}) : kernel(std::false_type{});
   if (!resident_fits(fn, HT, pl.smem)) return false;
   GridExchange gx = grid_exchange(rs, st);
   HalfMatrix h = H;

@@ -711,11 +711,22 @@ constexpr int kConvertParts = 4;
 __global__ void __launch_bounds__(SB)
     half_convert_kernel(int nv, const int* __restrict__ off, const int* __restrict__ col, const int* __restrict__ src,
                         const float* __restrict__ vals, const float4* __restrict__ scale, uint4* __restrict__ v8,
-                        uint16_t* __restrict__ v1) {
+                        uint16_t* __restrict__ v1, int vs) {
   const int unit = blockIdx.x * (SB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int sl = unit / kConvertParts, part = unit % kConvertParts, u = 32 * sl + lane;
-  if (u >= nv) return;
+  if (sl >= (nv + 31) >> 5) return;
   const int b = off[sl], W = (off[sl + 1] - b) >> 5;
+  auto word = [&](int e, float h8) {  // the ninth value, with the column where it is packed
+    const unsigned int h = __half_as_ushort(__float2half_rn(h8));
+    if (vs == 2)
+      reinterpret_cast<unsigned int*>(v1)[e] = h | ((unsigned int)(col[e] - 32 * sl) << 16);
+    else
+      v1[e] = (uint16_t)h;
+  };
+  if (u >= nv) {  // rows past the last vertex: only their columns are ever used
+    for (int k = part; k < W; k += kConvertParts) word(b + 32 * k + lane, 0.f);
+    return;
+  }
   const float4 su = scale[u];
   const float sa[3] = {su.x, su.y, su.z};
 #pragma unroll 2
@@ -736,7 +747,7 @@ __global__ void __launch_bounds__(SB)
       for (int c = 0; c < 3; ++c) h[3 * a + c] = (tr ? v[3 * c + a] : v[3 * a + c]) * sa[a] * sw[c];
     v8[e] = make_uint4(pack_half2(h[0], h[1]), pack_half2(h[2], h[3]), pack_half2(h[4], h[5]),
                        pack_half2(h[6], h[7]));
-    v1[e] = __half_as_ushort(__float2half_rn(h[8]));
+    word(e, h[8]);
   }
 }
 
@@ -768,12 +779,12 @@ __device__ __forceinline__ void half_row_product(const HalfMatrix& H, int u, con
   int k = 0;
   for (; k + 2 <= W; k += 2) {
     const uint4 p0 = H.v8[e0 + 32 * (size_t)k], p1 = H.v8[e0 + 32 * (size_t)(k + 1)];
-    const uint16_t h0 = H.v1[e0 + 32 * (size_t)k], h1 = H.v1[e0 + 32 * (size_t)(k + 1)];
+    const uint16_t h0 = H.v1[(e0 + 32 * (size_t)k) * H.vs], h1 = H.v1[(e0 + 32 * (size_t)(k + 1)) * H.vs];
     const float4 x0 = x[col(k)], x1 = x[col(k + 1)];
     fma_block(p0, h0, x0);
     fma_block(p1, h1, x1);
   }
-  if (k < W) fma_block(H.v8[e0 + 32 * (size_t)k], H.v1[e0 + 32 * (size_t)k], x[col(k)]);
+  if (k < W) fma_block(H.v8[e0 + 32 * (size_t)k], H.v1[(e0 + 32 * (size_t)k) * H.vs], x[col(k)]);
 }
 
 __global__ void __launch_bounds__(SB)
@@ -1548,9 +1559,9 @@ void launch_half_prepare(const SellMatrix& A, const float* vals, int precond, fl
 }
 
 void launch_half_convert(const SellMatrix& A, const int* off, const int* col, const int* src, const float* vals,
-                         const float4* scale, uint4* v8, uint16_t* v1, cudaStream_t st) {
+                         const float4* scale, uint4* v8, uint16_t* v1, int vs, cudaStream_t st) {
   if (A.nv <= 0) return;
-  half_convert_kernel<<<div_up((long long)div_up(A.nv, 32) * kConvertParts, SB / 32), SB, 0, st>>>(A.nv, off, col, src, vals, scale, v8, v1);
+  half_convert_kernel<<<div_up((long long)div_up(A.nv, 32) * kConvertParts, SB / 32), SB, 0, st>>>(A.nv, off, col, src, vals, scale, v8, v1, vs);
   after_launch("half_convert");
 }
 

@@ -159,6 +159,7 @@ struct TimeStep {
   DBuf<uint16_t> h16v1;
   DBuf<float4> h16scale, h16iscale, h16dinv;
   bool h16_ok = false, h16_built = false;
+  int h16vs = 1;
   long long nfs = 0;
   long long asm_count = 0, h16_count = -1;  // assemblies of the FP32 values; the one the copy was made from
   bool last_half = false;  // the last pcg() ran on the FP16 copy
@@ -617,6 +618,7 @@ struct TimeStep {
     if (!h16_ok) return false;
     nfs = (long long)col.size();
     h16off_h = off;
+    h16vs = half_columns_pack(off, col) ? 2 : 1;
     h16off.upload(off, stream);
     h16col.upload(col, stream);
     h16src.upload(src, stream);
@@ -624,18 +626,18 @@ struct TimeStep {
     return true;
   }
   HalfMatrix half_matrix() const {
-    return HalfMatrix{nv, h16off.p, h16col.p, h16v8.p, h16v1.p, h16scale.p, h16iscale.p};
+    return HalfMatrix{nv, h16off.p, h16col.p, h16v8.p, h16v1.p, h16scale.p, h16iscale.p, h16vs};
   }
   // the FP16 copy of the current FP32 system values (remade only after a new assembly)
   void half_refresh() {
     h16v8.alloc((size_t)nfs);
-    h16v1.alloc((size_t)nfs);
+    h16v1.alloc((size_t)nfs * h16vs);
     h16scale.alloc(nv);
     h16iscale.alloc(nv);
     h16dinv.alloc(3 * (size_t)nv);
     if (h16_count == asm_count) return;
     launch_half_prepare(A(), sf.vals.p, params.precond, h16scale.p, h16iscale.p, h16dinv.p, stream);
-    launch_half_convert(A(), h16off.p, h16col.p, h16src.p, sf.vals.p, h16scale.p, h16v8.p, h16v1.p, stream);
+    launch_half_convert(A(), h16off.p, h16col.p, h16src.p, sf.vals.p, h16scale.p, h16v8.p, h16v1.p, h16vs, stream);
     h16_count = asm_count;
   }
   // the FP16 copy serves a solve when it is enabled, the tolerance is loose enough for its rounding, the

@@ -202,11 +202,20 @@ bool build_full_sell(const Topology& t, std::vector<int32_t>& off, std::vector<i
           col[e] = w;
           src[e] = w >= u ? upper_slot(t, u, w) : (int32_t)(0x80000000u | (uint32_t)upper_slot(t, w, u));
         } else {
-          col[e] = u < t.nv ? u : 0;
+          col[e] = std::min(u, t.nv - 1);
         }
       }
     }
   }
+  return true;
+}
+
+bool half_columns_pack(const std::vector<int32_t>& off, const std::vector<int32_t>& col) {
+  for (size_t s = 0; s + 1 < off.size(); ++s)
+    for (int32_t e = off[s]; e < off[s + 1]; ++e) {
+      const long long d = (long long)col[e] - 32LL * (long long)s;
+      if (d < -32768 || d > 32767) return false;
+    }
   return true;
 }
 

@@ -69,6 +69,8 @@ void build_topology(int nv, int nt, const int32_t* cells, Topology& t, int cv = 
 // 31-bit indices.
 bool build_full_sell(const Topology& t, std::vector<int32_t>& off, std::vector<int32_t>& col,
                      std::vector<int32_t>& src);
+// whether every column of that pattern lies within 2^15 rows of its slice's first row (16-bit columns)
+bool half_columns_pack(const std::vector<int32_t>& off, const std::vector<int32_t>& col);
 
 // the upper-triangular block id of the local vertex pair (v <= w) used by the element Hessian kernel
 constexpr int upper_block_id(int v, int w) { return v * 4 - (v * (v - 1)) / 2 + (w - v); }

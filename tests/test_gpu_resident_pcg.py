@@ -146,3 +146,34 @@ def test_half_solve_beyond_l2():
     ts.set_params(pcg_half_matrix=0)
     _, it0, _ = ts.pcg(b, rtol=5e-2)
     assert abs(it - it0) <= 0.1 * it0 + 2, (it, it0)
+
+
+@pytest.mark.parametrize("hexes,swap,blocks", [
+    ((33, 33, 33), 31000, 0),   # columns up to 32,224 rows away: 16-bit offsets near their limit, entries on chip
+    ((33, 33, 33), 31000, 60),  # the same with the entries in global memory
+    ((33, 33, 33), 32700, 0),   # up to 33,924: 4-byte columns, entries on chip
+    ((33, 33, 33), 32700, 60),  # in global memory
+    ((66, 66, 66), 200000, 0),  # with L2 priorities
+])
+def test_half_solve_far_columns(hexes, swap, blocks):
+    """A grid mesh with vertex 0 and a far one's numbers swapped, so that some columns lie near or beyond the 2^15 rows that
+    a packed entry's column can be from its slice.  The true residual on the FP32 values is within 5e-2 plus the copy's
+    rounding (5e-3), the iterations within 10% + 2 of the solve on the FP32 values."""
+    X, T = mesh.kuhn_box(hexes, tuple(0.02 * k for k in hexes))
+    X[[0, swap]] = X[[swap, 0]]
+    T = np.where(T == 0, swap, np.where(T == swap, 0, T)).astype(T.dtype)
+    fixed = np.where(X[:, 0] == 0.0)[0]
+    ts = g.TimeStep(X, T, 1e-2, 1e5, 0.45, 1000.0)
+    ts.set_precision("mixed")
+    ts.set_material(10.0 ** mesh.uniform(52, T.shape[0], 4.0, 6.0), None)
+    ts.mark_dirichlet_batched(fixed, np.zeros((fixed.size, 3)))
+    ts.set_params(g.default_params(precond=2, pcg_max_blocks=blocks))
+    ts.reset("newton")
+    ts.update_hessian(False, True, True)
+    b = np.random.default_rng(53).normal(size=X.shape)
+    x, it, rr = ts.pcg(b, rtol=5e-2)
+    assert rr <= 5e-2
+    assert np.linalg.norm(b.reshape(-1) - ts.spmv(x).reshape(-1)) <= (5e-2 + 5e-3) * np.linalg.norm(b)
+    ts.set_params(pcg_half_matrix=0, pcg_persistent=0)
+    _, it0, _ = ts.pcg(b, rtol=5e-2)
+    assert abs(it - it0) <= 0.1 * it0 + 2, (it, it0)
