@@ -271,6 +271,12 @@ int fused_chunk();
 template <typename S>
 void launch_assemble(const SellMatrix& A, const int* cptr, const int* csrc, const S* Kbuf, size_t nb, const S* slot_mass,
                      const uint8_t* mask, bool filter, S* vals, V4<S>* dinv, int precond, cudaStream_t st, int block = 0);
+// the scalars to the host's pinned copy, then seq to its counter, which the host polls
+struct HostScalars {
+  DevScalars s;
+  unsigned long long seq;
+};
+void launch_publish(const DevScalars* sc, HostScalars* host, unsigned long long seq, cudaStream_t st);
 // assembly codes from the topology's element-major e nb + b to the planes' b nt + e (store_kblock), in place
 void launch_plane_codes(int n, int nb, int nt, int* codes, cudaStream_t st);
 // the element Hessian blocks in FP16 (per block a power-of-two scale; 20 bytes a block instead of 36, two planes: uint4[nb], then a word each) and the

@@ -11,6 +11,18 @@ namespace {
 constexpr int SB = 256;  // block of the slot / row / dof kernels (a multiple of the 32-row slice)
 
 
+// One warp: a word of the scalars a lane into pinned host memory, the counter after them.
+__global__ void publish_kernel(const DevScalars* __restrict__ sc, HostScalars* host, unsigned long long seq) {
+  constexpr int words = sizeof(DevScalars) / 8;
+  static_assert(sizeof(DevScalars) % 8 == 0, "whole words");
+  const unsigned long long* src = reinterpret_cast<const unsigned long long*>(sc);
+  volatile unsigned long long* dst = reinterpret_cast<unsigned long long*>(&host->s);
+  for (int i = threadIdx.x; i < words; i += 32) dst[i] = src[i];
+  __threadfence_system();
+  __syncwarp();
+  if (threadIdx.x == 0) asm volatile("st.release.sys.global.u64 [%0], %1;" ::"l"(&host->seq), "l"(seq) : "memory");
+}
+
 __global__ void __launch_bounds__(SB) plane_codes_kernel(int n, int nb, int nt, int* __restrict__ codes) {
   const unsigned int c = (unsigned int)blockIdx.x * SB + threadIdx.x;
   if (c >= (unsigned int)n) return;
@@ -1435,6 +1447,11 @@ void launch_kron_extract(const SellMatrix& A, const S* vals, S* svals, int* not_
   if (A.nslots <= 0) return;
   kron_extract_kernel<S><<<div_up(A.nslots, SB), SB, 0, st>>>(A.nslots, vals, svals, not_kron);
   after_launch("kron_extract");
+}
+
+void launch_publish(const DevScalars* sc, HostScalars* host, unsigned long long seq, cudaStream_t st) {
+  publish_kernel<<<1, 32, 0, st>>>(sc, host, seq);
+  after_launch("publish");
 }
 
 void launch_plane_codes(int n, int nb, int nt, int* codes, cudaStream_t st) {
