@@ -516,7 +516,7 @@ __global__ void __launch_bounds__(GB)
 // as they are formed (element_stiffness_blocks): 110 registers in FP32, 120 with FP16 blocks, 196 in FP64, no spills;
 // with 78 sums held to the end it was 128 and 176 bytes of spills.  1.02M tets, FP16 blocks: 94 us (169 at first, 102 with
 // the blocks staged through shared memory into element-major records); 192k tets, FP32 blocks: 20 us (37); FP64, 84,474
-// tets: 223 us (531), 30,498 tets: 92 us (195).
+// tets: 206 us (531), 30,498 tets: 85 us (195).
 // H16 (FP32 arithmetic only): a block is nine FP16 values scaled by 2^-k and k (the power of two that puts the block's
 // largest magnitude in [2^14, 2^15)): the first eight values in a 16-byte vector, the ninth and k in a word of a second
 // plane, 20 bytes a block instead of 36, read back with two loads (kernels_sparse.cu assemble_kernel).
