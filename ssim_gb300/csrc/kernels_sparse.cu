@@ -774,11 +774,11 @@ __device__ __forceinline__ void half_row_product(const HalfMatrix& H, int u, con
                                                  float& a0, float& a1, float& a2) {
   const int lane = u & 31, sl = u >> 5;
   const int b = H.off[sl], W = (H.off[sl + 1] - b) >> 5;
-  const int* cb = H.col + b + lane;
+  const bool packed = H.vs == 2;  // the staged word holds the column and the ninth value
+  const int* cb = (packed ? reinterpret_cast<const int*>(H.v1) : H.col) + b + lane;
   const int ns = min(W, ST_K);
   for (int k = 0; k < ns; ++k) cp_async4(&sidx[k][lane], cb + k * 32);
   cp_async_wait_all();
-  auto col = [&](int k) { return k < ST_K ? sidx[k][lane] : cb[k * 32]; };
   a0 = a1 = a2 = 0.f;
   auto fma_block = [&](const uint4& p, uint16_t h8, const float4& xv) {
     const float2 f01 = unpack_half2(p.x), f23 = unpack_half2(p.y), f45 = unpack_half2(p.z), f67 = unpack_half2(p.w);
@@ -788,15 +788,28 @@ __device__ __forceinline__ void half_row_product(const HalfMatrix& H, int u, con
     a2 += f67.x * xv.x + f67.y * xv.y + f8 * xv.z;
   };
   const size_t e0 = (size_t)b + lane;
+  auto entry = [&](int k, int& c, uint16_t& h) {
+    const int w = k < ST_K ? sidx[k][lane] : cb[k * 32];
+    c = packed ? 32 * sl + (w >> 16) : w;
+    h = packed ? (uint16_t)w : H.v1[e0 + 32 * (size_t)k];
+  };
   int k = 0;
   for (; k + 2 <= W; k += 2) {
     const uint4 p0 = H.v8[e0 + 32 * (size_t)k], p1 = H.v8[e0 + 32 * (size_t)(k + 1)];
-    const uint16_t h0 = H.v1[(e0 + 32 * (size_t)k) * H.vs], h1 = H.v1[(e0 + 32 * (size_t)(k + 1)) * H.vs];
-    const float4 x0 = x[col(k)], x1 = x[col(k + 1)];
+    int c0, c1;
+    uint16_t h0, h1;
+    entry(k, c0, h0);
+    entry(k + 1, c1, h1);
+    const float4 x0 = x[c0], x1 = x[c1];
     fma_block(p0, h0, x0);
     fma_block(p1, h1, x1);
   }
-  if (k < W) fma_block(H.v8[e0 + 32 * (size_t)k], H.v1[(e0 + 32 * (size_t)k) * H.vs], x[col(k)]);
+  if (k < W) {
+    int c0;
+    uint16_t h0;
+    entry(k, c0, h0);
+    fma_block(H.v8[e0 + 32 * (size_t)k], h0, x[c0]);
+  }
 }
 
 __global__ void __launch_bounds__(SB)

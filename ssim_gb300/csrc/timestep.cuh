@@ -1454,7 +1454,7 @@ struct TimeStep {
 
   // bytes one SpMV on the FP16 copy moves: 18 B of values and a 4-byte column per entry, the gathered vector
   // and the product once, the inverse scale for the unscaled residual norm
-  double half_spmv_bytes() const { return 22.0 * (double)nfs + 3.0 * nv * 16.0; }
+  double half_spmv_bytes() const { return (h16vs == 2 ? 20.0 : 22.0) * (double)nfs + 3.0 * nv * 16.0; }
   // bytes one PCG update pass moves: p, q, x, r read, x, r, z written, the 3x3 preconditioner blocks
   double update_bytes(size_t s) const { return 7.0 * nv * 4 * s + 3.0 * nv * 4 * s; }
 
