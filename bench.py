@@ -548,11 +548,12 @@ def main():
         variant = r.get("pcg_variant", args.pcg_variant)
         half = r.get("half_matrix", 0) == 1 and sum(s.get("half_solves", 0) for s in r["st_mixed"]) > 0
         pipe = variant == 4 or (half and variant == 3)
-        kname = ("pipe_half" if pipe else "cgcg_half") if half else ("pipe_persistent" if pipe else "cgcg_persistent")
+        kname = ("resident_half" if pipe else "cgcg_half") if half else ("pipe_persistent" if pipe else "cgcg_persistent")
         roofline = {"kernel": {
-            "pipe_half": "pipe_half_kernel (whole pipelined PCG solve in one cooperative launch on the FP16 copy of "
-                         "the Jacobi-scaled matrix, full block SELL-32; unit = one PCG iteration: SpMV of m = M w "
-                         "fused with the vector recurrences and dots, one reducing grid barrier)",
+            "resident_half": "resident_half_kernel (whole pipelined PCG solve in one cooperative launch on the FP16 "
+                             "copy of the Jacobi-scaled matrix, full block SELL-32, the rows' vectors in shared "
+                             "memory; unit = one PCG iteration: SpMV of m = M w, the vector recurrences and dots, "
+                             "one grid exchange)",
             "cgcg_half": "cgcg_half_kernel (whole Chronopoulos-Gear PCG solve in one cooperative launch on the FP16 "
                          "copy of the Jacobi-scaled matrix, full block SELL-32; unit = one PCG iteration: SpMV + "
                          "dots, grid reduction, vector update, grid barrier)",

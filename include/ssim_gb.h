@@ -160,8 +160,8 @@ typedef struct {
                              it saves.  0 keeps every solve on the FP32 values */
   double half_matrix_min_rtol; /* tighter solves (adjoint, tight forcing) stay on the FP32 values (1e-2) */
   int32_t half_hessian_blocks; /* tets: 1 (default) writes the element Hessian blocks of the assemblies whose solve
-                             runs on the FP16 copy in FP16 (a power-of-two scale per 3x3 block, 24 bytes a block
-                             instead of 36, three 8-byte loads in the assembly, FP32 sums); 0 keeps FP32 blocks */
+                             runs on the FP16 copy in FP16 (a power-of-two scale per 3x3 block, 20 bytes a block
+                             instead of 36, two loads in the assembly, FP32 sums); 0 keeps FP32 blocks */
   double half_check_slack; /* after every Newton solve on the FP16 copy the true residual |g + K d| on the FP32
                              values is computed with g . d (one fused kernel, about 25 us more than g . d alone
                              at 1M tets); above half_check_slack (1.2) times the forcing eta

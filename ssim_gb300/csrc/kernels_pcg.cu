@@ -12,9 +12,11 @@
 // trip through L2 where counted groups, their sums and a release word take three.
 //
 // Measured on a GB300 (us per iteration of a whole solve on the FP16 copy, against the earlier kernel of 256-row
-// virtual blocks with all vectors in global memory and counted group barriers): 1.02M-tet beam 10.4 (21.3), 192k-tet
-// bar 5.2 (12.6), 64-cube batch of 1.9M tets 43 (53).  Cycles of a beam iteration: SpMV 10,800, exchange 5,000, row
-// recurrences 4,600.
+// virtual blocks with all vectors in global memory and counted group barriers): 1.02M-tet beam 11.4 (21.3), 192k-tet
+// bar 5.0 (12.6), 64-cube batch of 1.9M tets 35 (53).  Cycles of a beam iteration: SpMV 10,000, exchange 5,000, row
+// recurrences 4,600.  Taking units and recurrences from one queue, so that neither waits for the other's last warp, was
+// slower on the beam (756 against 662 us a solve): the recurrences' chains of shared-memory loads stretch behind the
+// gathers.
 
 #include <cuda_fp16.h>
 
@@ -1075,7 +1077,7 @@ static HalfPlan l2_hints(HalfPlan p, int nv, const int32_t* off, size_t l2) {
 //  block, 219,000 rows on 152 SMs); beyond, passes of 32 slices and the rows that fit.  The matrix entries too
 //  where the block's part of them fits (about 70,000 rows): an iteration then reads nothing but the gathered
 //  vector from L2.
-//  L2 hints where what an iteration cycles through does not fit: swept in order, an LRU-like cache then keeps nothing.
+//  L2 hints where what an iteration cycles through does not fit (table: 22-byte entries): swept in order, an LRU-like cache then keeps nothing.
 //  The entries of the first slices of every block are loaded with evict_last, the others with evict_first.  Measured on
 //  batches of cubes, 126 MB of L2 (matrix / other bytes, MB; Newton iterations, ms): 77 / 8 6.43 without and 6.77 with
 //  60 MB kept; 92 / 17 10.1, 8.87 with 60; 108 / 28 15.1, 12.9 with 50; 118 / 35 18.0, 15.4 with 40; 157 / 60 22.7, 20.3
