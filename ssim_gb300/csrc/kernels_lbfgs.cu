@@ -309,8 +309,11 @@ __global__ void __launch_bounds__(LB)
 }
 
 // d = -(gamma g + sum_j p_j s_j + sum_j q'_j y_j) (coefficients from the multidot pass; gamma_host when
-// h.n == 0), g . d and |d|^2 into the scalars
-template <typename S>
+// h.n == 0), g . d and |d|^2 into the scalars.  L = 1: a thread per vertex; L = 4: four lanes a vertex, three of them a
+// component each, for systems that leave FP64 units idle (a thread's 51 FP64 operations at m = 8, 64 cycles each for a
+// warp, become 17): FP64, 9,225 vertices 10.9 -> 7.1 us.  The border is the multidot's
+// (twice as many warps as that leave the units two rounds of a thread per vertex).
+template <typename S, int L>
 __global__ void __launch_bounds__(LB)
     lbfgs_combine_kernel(int nv, const double* __restrict__ g, LbfgsHist<S> h, const double* __restrict__ coef,
                          double gamma_host, V4<S>* __restrict__ d, Reduce red) {
@@ -323,26 +326,41 @@ __global__ void __launch_bounds__(LB)
     cs[k] = used ? (S)(k == 2 * M && h.n == 0 ? gamma_host : coef[k]) : S(0);
   }
   __syncthreads();
-  const int u = blockIdx.x * LB + threadIdx.x;
+  const int i = blockIdx.x * LB + threadIdx.x, u = i / L;
   S part[2] = {S(0), S(0)};
   if (u < nv) {
-    const V4<S> gv = mk4<S>((S)g[3 * u], (S)g[3 * u + 1], (S)g[3 * u + 2]);
     const S gm = cs[2 * M];
-    S x = gm * gv.x, y = gm * gv.y, z = gm * gv.z;
+    if constexpr (L == 1) {
+      const V4<S> gv = mk4<S>((S)g[3 * u], (S)g[3 * u + 1], (S)g[3 * u + 2]);
+      S x = gm * gv.x, y = gm * gv.y, z = gm * gv.z;
 #pragma unroll
-    for (int j = 0; j < M; ++j) {
-      if (j < h.n) {
-        const V4<S> sv = h.s[j][u], yv = h.y[j][u];
-        const S a = cs[j], b = cs[M + j];
-        x += a * sv.x + b * yv.x;
-        y += a * sv.y + b * yv.y;
-        z += a * sv.z + b * yv.z;
+      for (int j = 0; j < M; ++j) {
+        if (j < h.n) {
+          const V4<S> sv = h.s[j][u], yv = h.y[j][u];
+          const S a = cs[j], b = cs[M + j];
+          x += a * sv.x + b * yv.x;
+          y += a * sv.y + b * yv.y;
+          z += a * sv.z + b * yv.z;
+        }
       }
+      const V4<S> dv = mk4<S>(-x, -y, -z);
+      d[u] = dv;
+      part[0] = dot3<S>(gv, dv);
+      part[1] = dot3<S>(dv, dv);
+    } else {
+      const int q = i % L;
+      const S gq = q < 3 ? (S)g[3 * (size_t)u + q] : S(0);
+      S x = gm * gq;
+      const size_t c = 4 * (size_t)u + q;
+#pragma unroll
+      for (int j = 0; j < M; ++j)
+        if (j < h.n)
+          x += cs[j] * reinterpret_cast<const S*>(h.s[j])[c] + cs[M + j] * reinterpret_cast<const S*>(h.y[j])[c];
+      x = q < 3 ? -x : S(0);
+      reinterpret_cast<S*>(d)[c] = x;
+      part[0] = gq * x;
+      part[1] = x * x;
     }
-    const V4<S> dv = mk4<S>(-x, -y, -z);
-    d[u] = dv;
-    part[0] = dot3<S>(gv, dv);
-    part[1] = dot3<S>(dv, dv);
   }
   double v2[2];
   block_sum_s<2, LB, S>(part, v2, shred);
@@ -382,7 +400,12 @@ void launch_lbfgs_multidot(int nv, const double* g, const LbfgsHist<S>& h, doubl
 template <typename S>
 void launch_lbfgs_combine(int nv, const double* g, const LbfgsHist<S>& h, const double* coef, double gamma_host,
                           V4<S>* d, const Reduce& red, cudaStream_t st) {
-  lbfgs_combine_kernel<S><<<div_up(nv, LB), LB, 0, st>>>(nv, g, h, coef, gamma_host, d, red);
+  int grid, groups;
+  multidot_shape(nv, grid, groups);
+  if (sizeof(S) == 8 && groups > 1)
+    lbfgs_combine_kernel<S, 4><<<div_up(4LL * nv, LB), LB, 0, st>>>(nv, g, h, coef, gamma_host, d, red);
+  else
+    lbfgs_combine_kernel<S, 1><<<div_up(nv, LB), LB, 0, st>>>(nv, g, h, coef, gamma_host, d, red);
   after_launch("lbfgs_combine");
 }
 
