@@ -1121,9 +1121,11 @@ static bool resident_device(int& nsm, size_t& smem_max, size_t& l2) {
   l2 = (size_t)l2b;
   return coop != 0;
 }
-static bool resident_fits(const void* fn, int threads, size_t smem) {
+// The limit on dynamic shared memory belongs to the kernel in its context, and handles launch from any thread: every call
+// sets the same value, the device's most, and never this handle's size.
+static bool resident_fits(const void* fn, int threads, size_t smem, size_t smem_max) {
   int per_sm = 0;
-  SSIM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  SSIM_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
   SSIM_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem));
   return per_sm >= 1;
 }
@@ -1146,7 +1148,7 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
                         : (const void*)resident_half_kernel<true, 8, false, k>;
   };
   const void* fn = pl.packed ? kernel(std::true_type{}) : kernel(std::false_type{});
-  if (!resident_fits(fn, HT, pl.smem)) return false;
+  if (!resident_fits(fn, HT, pl.smem, smem_max)) return false;
   GridExchange gx = grid_exchange(rs, st);
   HalfMatrix h = H;
   HalfSolveArgs ha = pa;
@@ -1195,7 +1197,7 @@ bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int
   const void* fn = !pl.cached   ? (const void*)resident64_kernel<false, 2>
                    : pl.T == 2 ? (const void*)resident64_kernel<true, 2>
                                : (const void*)resident64_kernel<true, 4>;
-  if (!resident_fits(fn, DT, pl.smem)) return false;
+  if (!resident_fits(fn, DT, pl.smem, smem_max)) return false;
   GridExchange gx = grid_exchange(rs, st);
   SellMatrix a = A;
   Solve64Args s = sa;
