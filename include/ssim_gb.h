@@ -396,9 +396,10 @@ SSIM_GB_API ssim_gb_status ssim_gb_energy_noalloc(const double* X, const double*
  * A one-time sweep on this handle's own data (call after reset(), between steps): the block sizes of the
  * FP32 element pass (64 / 128 / 256), the element Hessian (32 / 64 / 128), the assembly (128 / 256 / 512)
  * and the FP32 force gather (128 / 256 / 512), the persistent PCG's variant (mixed: standard or
- * Chronopoulos-Gear; FP64: two launches or Chronopoulos-Gear) and grid (one block per 256 rows or four per
- * SM), and the fused or two-kernel Hessian assembly.  Each candidate runs once untimed and then timed by
- * CUDA events on the handle's stream; the fastest is applied to the handle (the shapes, and pcg_persistent,
+ * Chronopoulos-Gear; FP64: two launches or Chronopoulos-Gear, for solves whose vectors do not fit on chip;
+ * those that fit keep the automatic choice's one launch, whose time is then the one reported, until
+ * ssim_gb_set_params changes pcg_persistent) and grid (one block per 256 rows or four per SM), and the
+ * fused or two-kernel Hessian assembly.  Each candidate runs once untimed and then timed by CUDA events on the handle's stream; the fastest is applied to the handle (the shapes, and pcg_persistent,
  * pcg_max_blocks, fused_assembly in its parameters).  The choice is cached for the process by (vertices,
  * cells, nonzero blocks, precision, instances, cell kind): a later handle of the same shape gets it without
  * timing (from_cache = 1).  The deformation and the other state are left as they were; the forces view is

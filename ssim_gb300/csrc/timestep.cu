@@ -326,6 +326,7 @@ ssim_gb_status ssim_gb_set_params(ssim_gb_timestep* h, const ssim_gb_params* p) 
       !(p->half_check_slack > 0) || (p->speculative_hessian != 0 && p->speculative_hessian != 1) ||
       !(p->cg_rtol >= 0) || p->cg_check_every < 1 || p->lbfgs_history < 1)
     return fail(h, SSIM_GB_ERR_INVALID_ARGUMENT, "invalid solver parameters");
+  if (p->pcg_persistent != h->ts.params.pcg_persistent) h->ts.tuned64 = false;
   h->ts.params = *p;
   h->ts.half_off = false;
   return SSIM_GB_OK;

@@ -1035,7 +1035,7 @@ struct TimeStep {
       }
     } else {
       int it = 0;
-      if (params.pcg_persistent == 3 && pcg_resident64(b, negate, eta, max_iters, rel_res, &it)) return it;
+      if ((params.pcg_persistent == 3 || tuned64) && pcg_resident64(b, negate, eta, max_iters, rel_res, &it)) return it;
     }
     launch_pcg_setup<S>(nv, b, s.dinv.p, s.x.p, s.r.p, s.z.p, s.p0.p, eta, max_iters, negate, red(), stream);
     return pcg_loop<S>(s.vals.p, s.dinv.p, max_iters, rel_res, true);
@@ -1865,6 +1865,10 @@ struct TimeStep {
     static std::mutex m;
     return m;
   }
+  // FP64: a tuning's variant (0 or 2) is the loop for solves whose vectors do not fit on chip.  Where they fit the resident
+  // solve is the faster at every size (pcg() with a tuning's variant against 2 and 0, solves to 5e-2: 1.25, 1.58 and
+  // 2.07 ms on 62,400 vertices, 2.24, 2.66 and 3.26 on 120,050), so it runs until ssim_gb_set_params changes the variant.
+  bool tuned64 = false;
   void apply_tuning(const ssim_gb_tuning& t) {
     shapes.elem = t.elem_block;
     shapes.hess = t.hessian_block;
@@ -1875,6 +1879,7 @@ struct TimeStep {
     params.pcg_max_blocks = t.pcg_max_blocks;
     params.fused_assembly = t.fused_assembly;
     params.pcg_half_matrix = t.pcg_half_matrix;
+    tuned64 = !mixed() && (t.pcg_persistent == 0 || t.pcg_persistent == 2);
   }
   ssim_gb_tuning autotune() {
     if (!has_reset) throw state_error("autotune() before reset()");
@@ -2001,6 +2006,8 @@ struct TimeStep {
     const int keep_variant = params.pcg_persistent, keep_grid = params.pcg_max_blocks;
     const int keep_half = params.pcg_half_matrix;
     const size_t log0 = solve_log.size();
+    const bool keep_tuned = tuned64;
+    tuned64 = false;
     double pbest = 1e300;
     t.pcg_persistent = keep_variant;
     t.pcg_max_blocks = keep_grid;
@@ -2012,6 +2019,7 @@ struct TimeStep {
           // the FP16 copy serves only these, and only when enabled (the sweep may turn it off, never on)
           if (half && ((v != 2 && v != 3) || !mixed() || keep_half != 1 || !half_ready())) continue;
           if (v == 3 && !half) continue;  // on the FP32 values variant 3 is variant 2
+          if (v == 3 && gcap != 0) continue;  // one block per SM, whatever a cap beyond that
           params.pcg_persistent = v;
           params.pcg_max_blocks = gcap;
           params.pcg_half_matrix = half;
@@ -2028,6 +2036,13 @@ struct TimeStep {
     params.pcg_persistent = keep_variant;
     params.pcg_max_blocks = keep_grid;
     params.pcg_half_matrix = keep_half;
+    if constexpr (std::is_same<S, double>::value) {  // what will run where the vectors fit on chip (apply_tuning)
+      int iters = 0;
+      bool fits = true;
+      const double ms = time_launches([&] { fits = pcg_resident64(rhs.p, false, 5e-2, params.cg_max_iters, nullptr, &iters); }, 2);
+      if (fits) ++count, pbest = ms, t.pcg_iterations = iters;
+    }
+    tuned64 = keep_tuned;
     solve_log.resize(log0);
     t.pcg_solve_ms = pbest;
     t.candidates = count;

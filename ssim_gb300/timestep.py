@@ -177,6 +177,12 @@ class TimeStep:
             if not hasattr(p, k):
                 raise KeyError(f"unknown solver parameter {k!r}")
             setattr(p, k, v)
+        if "pcg_persistent" in kw and p.pcg_persistent == self.params.pcg_persistent:
+            # a variant asked for by name outranks a tuning's, also where it is the same number: only a change tells
+            # the library so
+            p.pcg_persistent = 3
+            self._c(self._L.ssim_gb_set_params(self._h, C.byref(p)))
+            p.pcg_persistent = kw["pcg_persistent"]
         self._c(self._L.ssim_gb_set_params(self._h, C.byref(p)))
         return self
 
@@ -404,7 +410,7 @@ class TimeStep:
     def set_tuning(self, tuning: dict):
         """Applies a tuning found earlier (ssim_gb_set_tuning): the shape and PCG keys of an autotune() result;
         missing keys are 0 (the compiled defaults, the two-launch or standard PCG, unfused assembly, the FP32
-        matrix in every solve)."""
+        matrix in every solve).  FP64: solves whose vectors fit on chip keep their one launch, as with autotune()."""
         t = _lib.Tuning()
         for k in ("elem_block", "hessian_block", "assembly_block", "gather_block", "pcg_persistent",
                   "pcg_max_blocks", "fused_assembly", "pcg_half_matrix", "elem_regcap"):
