@@ -601,15 +601,16 @@ __host__ __device__ __forceinline__ void linear_stiffness(const S D[4][3], S lam
 // index k (l_t + l_f) / 2 on (i, j) and (l_f - l_t) / 2 between (i, j) and (j, i).  Contracted with W = D V (D the shape
 // gradients) the block of vertices v, w is K_vw = U B U^T with
 //   B(i, i) = A3+(i, i) W_vi W_wi + sum_j t_ij W_vj W_wj,   B(i, k) = A3+(i, k) W_vi W_wk + f_ik W_vk W_wi.
-// Six blocks are formed so (vertices 1 to 3); the shape gradients sum to zero, so the rows of vertex 0 are minus sums
-// of them.  About 600 operations after the SVD in place of the 1,060 of nine rank-one updates, one block at a time
-// instead of 78 live sums.  A3 is only diagonalised where its Cholesky minors do not already show every eigenvalue
-// above eps (A3+ = A3 then).
+// Every block is formed so, from its own vertices' gradients: the gradients sum to zero, and the four blocks of vertex 0
+// as minus sums of the others (six contractions instead of ten) would cancel where that vertex's gradient is small, its
+// diagonal block's relative error growing with the square of the gradients' ratio (2.5e-4 in FP32 for a tet 20 times as
+// long as wide, 2e-6 here).  One block lives at a time instead of 78 sums.  A3 is only diagonalised where its Cholesky
+// minors do not already show every eigenvalue above eps (A3+ = A3 then).
 // emit(v, w, block): the ten upper 3x3 blocks (v <= w, row-major), times scale, each once.
 template <typename S, typename EMIT>
 __host__ __device__ __forceinline__ void element_stiffness_blocks(const S* F, const S D[4][3], S lam, S mu, bool spsd,
                                                                   S scale, EMIT&& emit) {
-  S U[9], W[3][3], h[6], t[3], f[3];  // h: A3+ (00, 01, 02, 11, 12, 22); t, f by the third index
+  S U[9], W[4][3], h[6], t[3], f[3];  // h: A3+ (00, 01, 02, 11, 12, 22); t, f by the third index
   {
     S s[3], V[9];
     svd3(F, U, s, V);
@@ -622,10 +623,9 @@ __host__ __device__ __forceinline__ void element_stiffness_blocks(const S* F, co
     const S c = lam * (I3 - alpha);
     const S eps = S(1e-3);
 #pragma unroll
-    for (int v = 0; v < 3; ++v)
+    for (int v = 0; v < 4; ++v)
 #pragma unroll
-      for (int j = 0; j < 3; ++j)
-        W[v][j] = D[v + 1][0] * V[0 * 3 + j] + D[v + 1][1] * V[1 * 3 + j] + D[v + 1][2] * V[2 * 3 + j];
+      for (int j = 0; j < 3; ++j) W[v][j] = D[v][0] * V[0 * 3 + j] + D[v][1] * V[1 * 3 + j] + D[v][2] * V[2 * 3 + j];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
       S lt = a + c * s[k], lf = a - c * s[k];
@@ -666,13 +666,10 @@ __host__ __device__ __forceinline__ void element_stiffness_blocks(const S* F, co
 #pragma unroll
     for (int k = 0; k < 6; ++k) h[k] *= scale;
   }
-  S k0[3][9], k00[9];  // the rows of vertex 0
 #pragma unroll
-  for (int i = 0; i < 9; ++i) k0[0][i] = k0[1][i] = k0[2][i] = k00[i] = S(0);
+  for (int v = 0; v < 4; ++v)
 #pragma unroll
-  for (int v = 0; v < 3; ++v)
-#pragma unroll
-    for (int w = v; w < 3; ++w) {
+    for (int w = v; w < 4; ++w) {
       const S* x = W[v];
       const S* y = W[w];
       const S p0 = x[0] * y[0], p1 = x[1] * y[1], p2 = x[2] * y[2];
@@ -696,22 +693,8 @@ __host__ __device__ __forceinline__ void element_stiffness_blocks(const S* F, co
         for (int j = 0; j < 3; ++j)
           K[3 * i + j] = v == w && j < i ? K[3 * j + i]
                                          : C[3 * i] * U[3 * j] + C[3 * i + 1] * U[3 * j + 1] + C[3 * i + 2] * U[3 * j + 2];
-      emit(v + 1, w + 1, K);
-#pragma unroll
-      for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int j = 0; j < 3; ++j) {
-          k0[w][3 * i + j] -= K[3 * i + j];
-          if (v != w) k0[v][3 * i + j] -= K[3 * j + i];
-          if (j >= i) k00[3 * i + j] += v != w ? K[3 * i + j] + K[3 * j + i] : K[3 * i + j];
-        }
+      emit(v, w, K);
     }
-  k00[3] = k00[1];
-  k00[6] = k00[2];
-  k00[7] = k00[5];
-  emit(0, 0, k00);
-#pragma unroll
-  for (int w = 0; w < 3; ++w) emit(0, w + 1, k0[w]);
 }
 
 // the same as the packed upper triangle of the 12x12 matrix (78 entries)

@@ -513,10 +513,11 @@ __global__ void __launch_bounds__(GB)
 // One thread per tet: K_e = dt^2 V_e pfpx^T H+ pfpx (the gather weight V_e and alpha = dt^2 of
 // time_step.hpp:646-651 folded in), written as the 10 upper 3x3 vertex blocks, each a coalesced store
 // into its planes (store_kblock).  Bound by FP32 arithmetic (FP64: by the FP64 units).  The blocks leave
-// as they are formed (element_stiffness_blocks): 110 registers in FP32, 120 with FP16 blocks, 196 in FP64, no spills;
-// with 78 sums held to the end it was 128 and 176 bytes of spills.  1.02M tets, FP16 blocks: 94 us (169 at first, 102 with
-// the blocks staged through shared memory into element-major records); 192k tets, FP32 blocks: 20 us (37); FP64, 84,474
-// tets: 206 us (531), 30,498 tets: 85 us (195).
+// as they are formed (element_stiffness_blocks): 128 registers in FP32, 254 in FP64, no spills; with 78 sums held to the
+// end FP32 spilled 176 bytes.  1.02M tets, FP16 blocks: 101 us (169 at first; the blocks staged through shared memory into
+// element-major records cost 8 more); 192k tets, FP32 blocks: 22 us (37); FP64, 84,474 tets: 238 us (531), 30,498 tets:
+// 97 us (195).  All ten blocks are contracted: with the four of vertex 0 as sums of the others it was 94, 20, 207 and 85,
+// but those blocks lost their digits where that vertex's gradient is small.
 // H16 (FP32 arithmetic only): a block is nine FP16 values scaled by 2^-k and k (the power of two that puts the block's
 // largest magnitude in [2^14, 2^15)): the first eight values in a 16-byte vector, the ninth and k in a word of a second
 // plane, 20 bytes a block instead of 36, read back with two loads (kernels_sparse.cu assemble_kernel).
