@@ -148,9 +148,11 @@ __device__ __forceinline__ bool exchange_barrier(const GridExchange& gx, unsigne
 
 // The scalars of a solve, one copy per block (the same bits in each): Chronopoulos-Gear's
 //   beta = g / g_old,  den = d - beta g / alpha_old,  alpha = g / den   (first: 0, d, g / d)
-// from g = (r, u), d = (w, u), with the reciprocals of the last step kept: ig = 1 / g_old, c = ig / alpha_old.
+// from g = (r, u), d = (w, u), with the reciprocals of the last step kept: ig = 1 / g_old, ia = 1 / alpha_old.  The
+// correction is (g ig)(g ia): both factors have the size of a ratio or of d, where g g ig ia would leave the range of FP64
+// for residuals beyond 1e77 or below 1e-81.
 struct Scalars {
-  double ig, c, g, den, rr, rr0, tol2, alpha, beta;
+  double ig, ia, g, den, rr, rr0, tol2, alpha, beta;
   int iters, done, status;
 };
 
@@ -186,8 +188,11 @@ __device__ __forceinline__ void step_scalars(Scalars& s, bool first, double g, d
     s.done = 1;
     return;
   }
-  double den = d;
-  if (s.iters > 0) den = fma(-(g * g), s.c, d);
+  double den = d, beta = 0.0;
+  if (s.iters > 0) {
+    beta = g * s.ig;
+    den = fma(-beta, g * s.ia, d);
+  }
   if (!positive(den)) {  // breakdown: not SPD along p (or non-finite)
     s.done = 1;
     s.status = 1;
@@ -204,7 +209,7 @@ __device__ __forceinline__ void step_scalars(Scalars& s, bool first, double g, d
   } else {
     s.alpha = g / den;
   }
-  s.beta = s.iters > 0 ? g * s.ig : 0.0;
+  s.beta = beta;
   s.g = g;
   s.den = den;
   s.iters += 1;
@@ -212,7 +217,7 @@ __device__ __forceinline__ void step_scalars(Scalars& s, bool first, double g, d
 // one thread, any time before the next step_scalars: the reciprocals it will use
 __device__ __forceinline__ void next_reciprocals(Scalars& s) {
   s.ig = 1.0 / s.g;
-  s.c = s.den * s.ig * s.ig;
+  s.ia = s.den * s.ig;
 }
 // the solve's scalars for the host
 __device__ __forceinline__ void publish_scalars(const Scalars& s, DevScalars* o) {

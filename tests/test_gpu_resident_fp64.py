@@ -43,3 +43,15 @@ def test_tuned_handle_solves_on_chip():
         for variant in (0, 2, 0):
             t.set_params(pcg_persistent=variant)
             assert np.array_equal(t.pcg(b, rtol=1e-6)[0], x0) == (variant == 0)
+
+
+@pytest.mark.parametrize("hexes", [(13, 9, 7), (24, 24, 24)])
+def test_solutions_scale_with_the_right_side(hexes):
+    """A right side times a power of two gives the solution times it, bit for bit: nothing in the iteration leaves FP64's
+    range while the residual's square is inside it."""
+    ts, b = _handle(hexes)
+    for rtol in (5e-2, 1e-8):
+        x, it, rr = ts.pcg(b, rtol=rtol)
+        for k in (-400, -280, 280, 400):
+            got = ts.pcg(np.ldexp(b, k), rtol=rtol)
+            assert got[1:] == (it, rr) and np.array_equal(np.ldexp(got[0], -k), x), (rtol, k, got[1:], (it, rr))
