@@ -423,6 +423,12 @@ __host__ __device__ __forceinline__ void orthogonal_columns(const double* F, dou
   }
   const bool fine = mx > 1e-10f && mx < 1e15f;  // F^T F and 1e-15 of it are well inside FP32's range
   if (fine) {
+    // the largest entry in [1/2, 1): right_basis tests sums of F^4, which leave the range beyond 4e9 and below 3e-10
+    int ex;
+    frexpf(mx, &ex);
+    const float to1 = ldexpf(1.f, -ex);
+#pragma unroll
+    for (int k = 0; k < 9; ++k) f[k] *= to1;
     right_basis(f, v);
     double a[3] = {v[0], v[3], v[6]}, b[3] = {v[1], v[4], v[7]};
     // 1 / |a| with |a|^2 = 1 + e, e ~ 1e-6: 1 - e / 2 + 3 e^2 / 8
