@@ -15,6 +15,7 @@
 //   lf           double[4][T][4] scaled element forces (xyz0) awaiting the vertex gather; triangles [T][3][4], springs [T][4]
 //   vectors      vec4<S>[V]  CG vectors, one padded xyz triple per vertex
 #pragma once
+#include <functional>
 #include <type_traits>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -369,7 +370,7 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
                               const Reduce& red, const ResidentSync& rs, int max_blocks, cudaStream_t st);
 // FP64 PCG on the symmetric store, the whole solve in one launch (set-up, iterations and, with check, g . x and |x|^2
 // into sc->gd, dnorm2): pipelined for pipe_iters iterations, then Chronopoulos-Gear; sl_off, lo_off: host copies of
-// A's slice offsets; m: 2 nv vectors of scratch.  false if the vectors do not fit on chip or the device cannot launch it
+// A's slice offsets; scratch: gives 2 nv vectors, asked for where the solve fits.  false if the vectors do not fit on chip or the device cannot launch it
 struct Solve64Args {
   const double* b;  // right-hand side sign * b (the Newton gradient g with negate = 1)
   int negate;
@@ -379,7 +380,8 @@ struct Solve64Args {
   int check;
 };
 bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int32_t* lo_off, const double* vals,
-                           const double4_32a* dinv, double4_32a* x, double4_32a* m, const Solve64Args& a, const Reduce& red,
+                           const double4_32a* dinv, double4_32a* x, const std::function<double4_32a*()>& scratch,
+                           const Solve64Args& a, const Reduce& red,
                            const ResidentSync& rs, int max_blocks, cudaStream_t st);
 // after a solve on the FP16 copy: g . d, |d|^2 (as launch_dot_gd) and the solve's true residual on the FP32
 // symmetric values, |-g - K d|^2 and |g|^2 (sc->true_rr, sc->true_bb)

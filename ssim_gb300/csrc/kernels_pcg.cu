@@ -1190,7 +1190,8 @@ static Plan64 plan64(int nv, const int32_t* sl_off, const int32_t* lo_off, int n
 }
 
 bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int32_t* lo_off, const double* vals,
-                           const double4_32a* dinv, double4_32a* x, double4_32a* m, const Solve64Args& sa, const Reduce& red,
+                           const double4_32a* dinv, double4_32a* x, const std::function<double4_32a*()>& scratch,
+                           const Solve64Args& sa, const Reduce& red,
                            const ResidentSync& rs, int max_blocks, cudaStream_t st) {
   if (A.nv <= 0) return true;
   int nsm = 0;
@@ -1203,6 +1204,7 @@ bool launch_pcg64_resident(const SellMatrix& A, const int32_t* sl_off, const int
                    : pl.T == 2 ? (const void*)resident64_kernel<true, 2>
                                : (const void*)resident64_kernel<true, 4>;
   if (!resident_fits(fn, DT, pl.smem, smem_max)) return false;
+  double4_32a* m = scratch();
   GridExchange gx = grid_exchange(rs, st);
   SellMatrix a = A;
   Solve64Args s = sa;

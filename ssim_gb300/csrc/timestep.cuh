@@ -1091,10 +1091,13 @@ struct TimeStep {
   // 10.5 against 29.6 on 15,625 (to 1e-10)
   bool pcg_resident64(const double* b, bool negate, double eta, int max_iters, double* rel_res, int* iters) {
     Solver<double>& s = sd;
-    if (s.pm.n < 2 * (size_t)nv) s.pm.alloc(2 * (size_t)nv);
+    const auto scratch = [&] {
+      if (s.pm.n < 2 * (size_t)nv) s.pm.alloc(2 * (size_t)nv);
+      return s.pm.p;
+    };
     const Solve64Args sa{b, negate ? 1 : 0, eta, max_iters, eta >= kPipe64MinRtol ? params.pcg_pipe_iters : 0, negate ? 1 : 0};
     if (profiling) SSIM_CUDA(cudaEventRecord(ev[0], stream));
-    if (!launch_pcg64_resident(A(), topo.sl_off.data(), topo.lo_off.data(), s.vals.p, s.dinv.p, s.x.p, s.pm.p, sa, red(),
+    if (!launch_pcg64_resident(A(), topo.sl_off.data(), topo.lo_off.data(), s.vals.p, s.dinv.p, s.x.p, scratch, sa, red(),
                                resident_sync(), params.pcg_max_blocks, stream))
       return false;
     if (profiling) SSIM_CUDA(cudaEventRecord(ev[1], stream));

@@ -55,3 +55,18 @@ def test_solutions_scale_with_the_right_side(hexes):
         for k in (-400, -280, 280, 400):
             got = ts.pcg(np.ldexp(b, k), rtol=rtol)
             assert got[1:] == (it, rr) and np.array_equal(np.ldexp(got[0], -k), x), (rtol, k, got[1:], (it, rr))
+
+
+def test_solves_that_do_not_fit_take_no_scratch():
+    """132,651 vertices are beyond the chip (25 slices on each of 152 SMs): the automatic choice runs the two-launch loop,
+    bit for bit, and does not allocate the resident solve's vectors (8.5 MB; the driver hands out 2 MB at a time)."""
+    import torch
+
+    ts, b = _handle((50, 50, 50))
+    ts.set_params(pcg_persistent=0)
+    x0, it0, _ = ts.pcg(b, rtol=5e-2)
+    free = torch.cuda.mem_get_info()[0]
+    ts.set_params(pcg_persistent=3)
+    x, it, _ = ts.pcg(b, rtol=5e-2)
+    assert it == it0 and np.array_equal(x, x0)
+    assert free - torch.cuda.mem_get_info()[0] <= 4 << 20
