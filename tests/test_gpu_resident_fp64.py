@@ -70,3 +70,40 @@ def test_solves_that_do_not_fit_take_no_scratch():
     x, it, _ = ts.pcg(b, rtol=5e-2)
     assert it == it0 and np.array_equal(x, x0)
     assert free - torch.cuda.mem_get_info()[0] <= 4 << 20
+
+
+# hexes a side, grid cap, whether the vectors fit on chip
+LAYOUTS = [
+    ((13, 9, 7), 18, True),    # 35 slices, two a block: four warps a slice, entries on chip
+    ((13, 9, 7), 12, True),    # three a block
+    ((7, 7, 7), 4, True),      # 16 slices, four a block: two warps a slice, entries on chip
+    ((24, 24, 24), 0, True),   # 489 slices, three and four a block
+    ((13, 9, 7), 7, True),     # five a block, entries in global memory
+    ((15, 9, 9), 2, True),     # 50 slices, 25 a block: the most whose vectors fit
+    ((15, 12, 7), 2, False),   # 52 slices, 26 a block: the two-launch loop
+]
+
+
+@pytest.mark.parametrize("hexes,blocks,fits", LAYOUTS)
+def test_solve_matches_two_launch_in_its_layouts(hexes, blocks, fits):
+    """Against the two-launch loop, in the layouts of the FP64 kernel, with the path that ran read from the profile:
+    iteration counts within 2, true residuals at 1.5 of the tolerance, a capped solve's iterate within 1e-12."""
+    ts, b = _handle(hexes, pcg_max_blocks=blocks)
+    bn = np.linalg.norm(b)
+    for rtol in (5e-2, 1e-6, 1e-10):
+        ts.set_params(pcg_persistent=3)
+        ts.profile(True)
+        x, it, rr = ts.pcg(b, rtol=rtol)
+        one, two = (ts.profile_read(k)["launches"] for k in ("pcg_iteration", "pcg_spmv"))
+        ts.profile(False)
+        assert (one, two) == ((it, 0) if fits else (0, it))
+        ts.set_params(pcg_persistent=0)
+        _, it0, _ = ts.pcg(b, rtol=rtol)
+        assert rr <= rtol and abs(it - it0) <= 2, (rtol, it, it0)
+        assert np.linalg.norm(b - ts.spmv(x)) <= 1.5 * rtol * bn
+    for rtol, pipe in ((1e-2, 80), (1e-2, 3), (1e-12, 80)):
+        ts.set_params(pcg_persistent=3, pcg_pipe_iters=pipe)
+        x, it, _ = ts.pcg(b, rtol=rtol, max_iters=7)
+        ts.set_params(pcg_persistent=0)
+        x0, it0, _ = ts.pcg(b, rtol=rtol, max_iters=7)
+        assert it == it0 and np.linalg.norm(x - x0) <= 1e-12 * np.linalg.norm(x0)
