@@ -113,17 +113,19 @@ typedef struct {
                              scaled matrix (pcg_half_matrix, whose true-residual check covers the drift
                              below) and 2 on the FP32 values; in FP64 one launch with the vectors on chip
                              (Chronopoulos-Gear, solves to 1e-3 or looser pipelined for pcg_pipe_iters
-                             iterations first) where they fit, 0 beyond (about 129,000 vertices);
+                             iterations first) where they fit, 0 beyond (121,600 vertices on 152 SMs);
                              4: pipelined PCG in one launch (one grid barrier per iteration, two more vertex
                              vectors, Chronopoulos-Gear after pcg_pipe_iters iterations; equal to 0 up to
                              rounding, but in FP32 its true residual drifts from the recursive one with the
                              iterations and the condition number: for loose solves of well-conditioned
                              systems only) */
-  int64_t pcg_spin_limit; /* polls before a grid-barrier wait gives up (SSIM_GB_ERR_DEVICE_TIMEOUT); 0 = default
-                             (2^25 polls, about a second) */
+  int64_t pcg_spin_limit; /* polls before a grid-barrier wait gives up (SSIM_GB_ERR_DEVICE_TIMEOUT); 0 = default:
+                             2^25, and 2^21 (half a second) in the solves with the vectors on chip (3 in FP64, 3
+                             and 4 on the FP16 copy), whose polls wait for memory each */
   int32_t pcg_barrier_extra; /* test hook: arrivals a grid barrier waits for beyond the grid; 0 in normal use,
                                 > 0 makes every wait run out after pcg_spin_limit polls */
-  int32_t pcg_max_blocks; /* cap on the persistent PCG grid (0: as many 256-thread blocks as are resident) */
+  int32_t pcg_max_blocks; /* cap on the persistent PCG grid (0: as many 256-thread blocks as are resident; with the
+                             vectors on chip one block of 1,024 threads per SM, 512 in FP64) */
   int32_t ncg_max_iters;  /* nonlinear CG iteration cap: 1000 as the reference (nonlinear_cg.hpp:20) */
   double ncg_step0;       /* first trial step of the first NCG iteration: the reference's learning rate 1e-2 */
   double ncg_eta;         /* Dai-Kou truncation: beta >= ncg_eta * g.d / |d|^2 (0.5) */

@@ -64,34 +64,8 @@ __host__ __device__ __forceinline__ S snh_stress(const S* F, S lam, S mu, S* P) 
 // Energy, first Piola-Kirchhoff stress (when STRESS) and the sum of the magnitudes of the energy's terms
 // in one pass sharing I_c, J and log(I_c + 1); alpha = 1 + 3/4 mu / lambda and psi0 = the energy's value
 // at F = I (stable_neohookean.hpp:34,60) come precomputed per element.  Same formulas as snh_stress /
-// snh_energy / snh_energy_scale.
-template <typename S, bool STRESS>
-__host__ __device__ __forceinline__ S snh_eval(const S* F, S lam, S mu, S alpha, S psi0, S* P, S& scale) {
-  S Ic = 0;
-#pragma unroll
-  for (int i = 0; i < 9; ++i) Ic += F[i] * F[i];
-  S C[9];
-  S J;
-  if (STRESS) {
-    cofactor(F, C);
-    J = F[0] * C[0] + F[1] * C[1] + F[2] * C[2];
-  } else {
-    J = det3(F);
-  }
-  const S Jm = J - alpha;
-  if (STRESS) {
-    const S sF = mu * (S(1) - S(1) / (Ic + S(1)));
-    const S lj = lam * Jm;
-#pragma unroll
-    for (int i = 0; i < 9; ++i) P[i] = lj * C[i] + sF * F[i];
-  }
-  const S t1 = mu * (Ic - S(3)), t2 = lam * Jm * Jm, t3 = mu * log(Ic + S(1));
-  scale = S(0.5) * (fabs(t1) + t2 + fabs(t3)) + fabs(psi0);
-  return S(0.5) * (t1 + t2 - t3) - psi0;
-}
-
-// The same in FP64 with every operation counted (the FP64 element pass is bound by GB300's FP64 units): P times sV
-// (dt^2 V_e, folded into its two factors), and log(I_c + 1) and 1 / (I_c + 1) from the caller's lr(x, rcp).
+// snh_energy / snh_energy_scale, with every FP64 operation counted (the FP64 element pass is bound by GB300's FP64 units):
+// P comes times sV (dt^2 V_e, folded into its two factors), and log(I_c + 1) and 1 / (I_c + 1) from the caller's lr(x, rcp).
 template <bool STRESS, typename LR>
 __host__ __device__ __forceinline__ double snh_eval_scaled(const double* F, double lam, double mu, double alpha, double psi0,
                                                            double sV, double* P, double& scale, LR&& lr) {
@@ -197,7 +171,7 @@ __host__ __device__ __forceinline__ S snh_increment(const S* Gr, const S* dG, S 
 // J - 1 = tr G + (principal 2x2 minors of G) + det G, c1 = 1 - alpha = -3/4 mu / lambda:
 //   Psi - Psi(I) = 1/2 [ mu (s - log1p(s / 4)) + lambda (J - 1)(J - 1 + 2 c1) ]
 //   P = lambda (J - 1) cof F + 3/4 mu (G + G^T - tr G I - cof G) + mu s / (4 (4 + s)) F,
-// using cof(I + G) = I + tr G I - G^T + cof G.  Algebraically the same functions as snh_eval (the
+// using cof(I + G) = I + tr G I - G^T + cof G.  Algebraically the same functions as snh_eval_scaled (the
 // reference's stable_neohookean.hpp:23-62); scale returns the magnitude sum of the terms above.
 template <typename S, bool STRESS>
 __host__ __device__ __forceinline__ S snh_eval_small(const S* G, S lam, S mu, S* P, S& scale) {
@@ -262,7 +236,7 @@ __host__ __device__ __forceinline__ S snh2_eval_small(const S* G, S lam, S mu, S
   return S(0.5) * (t1 + t2);
 }
 
-// per-element constants of snh_eval
+// per-element constants of snh_eval_scaled
 template <typename S>
 __host__ __device__ __forceinline__ void snh_constants(S lam, S mu, S& alpha, S& psi0) {
   alpha = S(0.75) * mu / lam + S(1);

@@ -355,7 +355,7 @@ bool launch_pcg_half(const HalfMatrix& H, const float4* dinv16, float4* x, float
                      float4* p1, float4* q, int max_iters, const Reduce& red, unsigned long long* gsync,
                      long long spin_limit, int extra, int max_blocks, cudaStream_t st);
 // grid exchange of the resident solves (kernels_pcg.cu): resident_sync_bytes() of device memory; extra and
-// spin_limit as the persistent kernels' (0: 2^21 polls, about a second)
+// spin_limit as the persistent kernels' (0: 2^21 polls, half a second)
 struct ResidentSync {
   unsigned char* mem;
   int extra;

@@ -16,7 +16,7 @@ std::atomic<uint64_t> g_launches{0};
 namespace {
 
 constexpr int EB = 128;  // element block (energy / gradient)
-constexpr int HB = 64;   // element block (Hessian): 64 x 90 x sizeof(S) bytes of staging
+constexpr int HB = 64;   // element block (Hessian)
 
 template <typename S>
 __device__ __forceinline__ S comp(const V4<S>& v, int k) {

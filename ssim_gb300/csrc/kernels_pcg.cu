@@ -413,7 +413,7 @@ __device__ __forceinline__ void half_unit(const int* col, const uint4* v8, const
 //   prologue:  w = A u0, m_0 = M w;       partials (r, u), (w, u), (r, r)                -> exchange
 //   phase k:   n = A m_k;  z = n + beta z,  s = w + beta s,  p = M r + beta p;
 //              x += alpha p,  r -= alpha s,  w -= alpha z;  m_{k+1} = M w;  partials    -> exchange
-// One exchange per iteration both sums the dots and orders m's writes.  The scalars (cgcg_after) and the stop
+// One exchange per iteration both sums the dots and orders m's writes.  The scalars (step_scalars) and the stop
 // rule are Chronopoulos-Gear's; the third dot is (r, r) of the unscaled residual.  In FP32 the recursive residual
 // drifts from the true one with the iterations and the condition number, so after pipe_iters iterations the
 // solve continues as Chronopoulos-Gear PCG from the same state (w = A u recomputed, two exchanges a round).
@@ -1078,8 +1078,8 @@ static HalfPlan l2_hints(HalfPlan p, int nv, const int32_t* off, size_t l2) {
 // Layout of a resident solve on the FP16 copy (host arithmetic only; off: the copy's slice offsets).
 //  T: 4 warps a slice (a 15-entry slice is four entries a unit: all of a unit's loads in flight at once), 8 where a
 //  block has fewer than 8 slices (small systems: fewer dependent rounds).
-//  The vectors of all rows stay on chip while they and one pass over the block's slices fit (about 1,440 rows a
-//  block, 219,000 rows on 152 SMs); beyond, passes of 32 slices and the rows that fit.  The matrix entries too
+//  The vectors of all rows stay on chip while they and one pass over the block's slices fit (1,408 rows a block,
+//  214,000 on 152 SMs); beyond, passes of 32 slices and the rows that fit.  The matrix entries too
 //  where the block's part of them fits (about 70,000 rows): an iteration then reads nothing but the gathered
 //  vector from L2.
 //  L2 hints where what an iteration cycles through does not fit (table: 22-byte entries): swept in order, an LRU-like cache then keeps nothing.
@@ -1165,8 +1165,8 @@ bool launch_pcg_half_resident(const HalfMatrix& H, const int32_t* off_host, cons
   return true;
 }
 
-// Layout of a resident FP64 solve: all rows' vectors on chip or none (about 850 rows a block, 129,000 on 152 SMs), the
-// matrix entries too where they fit (about 24,000 rows).  grid 0: does not fit.
+// Layout of a resident FP64 solve: all rows' vectors on chip or none (25 slices a block, 121,600 rows on 152 SMs), the
+// matrix entries too where they fit (four slices of 15 entries a row, 19,000 rows).  grid 0: does not fit.
 static Plan64 plan64(int nv, const int32_t* sl_off, const int32_t* lo_off, int nsm, size_t smem_max, int max_blocks) {
   Plan64 p{};
   const int nsl = div_up(nv, 32);

@@ -18,27 +18,6 @@ __device__ __forceinline__ S comp4(const V4<S>& v, int k) {
   return k == 0 ? v.x : (k == 1 ? v.y : v.z);
 }
 
-// edge vector x_i - x_j = (X_i - X_j) + (u_i - u_j) (+ alpha (d_i - d_j)), from differences so a short
-// spring keeps its digits
-template <typename SD, bool TRIAL>
-__device__ __forceinline__ void edge_vec(const SpringData& sp, const double* __restrict__ u, const V4<SD>* d,
-                                         double alpha, int s, int& i, int& j, double (&e)[3]) {
-  const int2 c = sp.ends[s];
-  i = c.x;
-  j = c.y;
-  V4<SD> di, dj;
-  if (TRIAL) {
-    di = d[i];
-    dj = d[j];
-  }
-#pragma unroll
-  for (int k = 0; k < 3; ++k) {
-    double v = (sp.X[3 * i + k] - sp.X[3 * j + k]) + (u[3 * i + k] - u[3 * j + k]);
-    if (TRIAL) v += alpha * ((double)comp4<SD>(di, k) - (double)comp4<SD>(dj, k));
-    e[k] = v;
-  }
-}
-
 // energy share of vertex v's lumped inertia: 1/2 m_v |u_v (+ alpha d_v) - x~_v|^2
 template <typename SD, bool TRIAL>
 __device__ __forceinline__ double lumped_energy(int v, const double* __restrict__ m, const double* __restrict__ u,
@@ -258,9 +237,11 @@ __global__ void __launch_bounds__(PB)
     spring_hessian_kernel(SpringData sp, const double* __restrict__ u, double dt2, int spsd, S* __restrict__ Kbuf) {
   const int s = blockIdx.x * PB + threadIdx.x;
   if (s >= sp.ns) return;
-  int i, j;
-  double e[3];
-  edge_vec<S, false>(sp, u, nullptr, 0.0, s, i, j, e);
+  const int2 c2 = sp.ends[s];
+  const int i = c2.x, j = c2.y;
+  double e[3];  // x_i - x_j from differences, so a short spring keeps its digits
+#pragma unroll
+  for (int q = 0; q < 3; ++q) e[q] = (sp.X[3 * i + q] - sp.X[3 * j + q]) + (u[3 * i + q] - u[3 * j + q]);
   const double l = sqrt(e[0] * e[0] + e[1] * e[1] + e[2] * e[2]);
   const double L = sp.rest[s], k = sp.k[s];
   double c = l > 0 ? 1.0 - L / l : 0.0;

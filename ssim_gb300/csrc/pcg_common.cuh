@@ -1,5 +1,5 @@
-// pcg_common.cuh -- pieces shared by the PCG kernels of kernels_sparse.cu and kernels_pcg.cu: the SELL-32
-// addressing of a 3x3 block, the block-Jacobi product and the scalar epilogues of the iterations.
+// pcg_common.cuh -- the SELL-32 addressing of a 3x3 block (kernels_sparse.cu and kernels_pcg.cu), and the block-Jacobi
+// product and scalar epilogues of kernels_sparse.cu's PCG kernels (the resident solves have their own, step_scalars).
 #pragma once
 #include "kernels.cuh"
 
@@ -7,7 +7,7 @@ namespace ssim_gb {
 
 __device__ __forceinline__ size_t sell_base(int q) { return (size_t)9 * (size_t)(q & ~31) + (size_t)(q & 31); }
 
-// the scalar epilogues of standard PCG (two-launch, persistent and resident)
+// the scalar epilogues of standard PCG (two-launch and persistent)
 __device__ __forceinline__ void pcg_after_pq(DevScalars* sc, double pq) {
   sc->pq = pq;
   sc->alpha = sc->rz / pq;

@@ -1048,7 +1048,7 @@ struct TimeStep {
     half_refresh();
     const HalfMatrix H = half_matrix();
     // the automatic choice (3) on the copy is the pipelined iteration: one reducing barrier per iteration
-    // (21.1 against 23.8 us per iteration on the 1.02M-tet beam, the same iteration counts); its FP32
+    // (11.4 against 21.4 us per iteration on the 1.02M-tet beam, the same iteration counts); its FP32
     // recursive-residual drift is covered by the true-residual check of every Newton solve, which that
     // kernel runs itself after the solve (with its set-up before it: one launch, one host wait)
     const bool pipe = (params.pcg_persistent == 3 || params.pcg_persistent == 4) && max_iters > 0;
@@ -1636,10 +1636,6 @@ struct TimeStep {
         if (ls + 1 < params.max_ls_iters) alpha *= params.ls_shrink;
       }
       if (spec) SSIM_CUDA(cudaStreamWaitEvent(stream, ev_xf, 0));
-      if (params.max_ls_iters < 1) {
-        gather();
-        sync_scalars();
-      }
       launch_axpy_update<S>(nv, alpha, s.x.p, dX.p, next.p, nullptr, stream);
       if (!std::isfinite(Et) || !std::isfinite(hsc->gnorm2))
         throw numerical_error("non-finite energy or gradient (inverted or degenerate element?)");

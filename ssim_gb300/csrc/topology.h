@@ -65,7 +65,7 @@ void build_topology(int nv, int nt, const int32_t* cells, Topology& t, int cv = 
 // loose PCG solves read): slice s = block rows 32s..32s+31, width = the slice's largest degree; entry
 // off[s] + 32k + lane holds row u = 32s + lane's k-th neighbour w (ascending) in col and, in src, the upper slot
 // holding block (min(u, w), max(u, w)) with bit 31 set when the entry is that slot's transpose (w < u).
-// Padding entries: column u (0 past the last row) and the all-zero slot.  false if the entries do not fit
+// Padding entries: column u (the last row past it) and the all-zero slot.  false if the entries do not fit
 // 31-bit indices.
 bool build_full_sell(const Topology& t, std::vector<int32_t>& off, std::vector<int32_t>& col,
                      std::vector<int32_t>& src);
