@@ -1455,7 +1455,7 @@ struct TimeStep {
     return up * (9.0 * s + 4.0) + lo * 8.0 + 2.0 * (topo.nslices + 1) * 4 + 4.0 * nv * 4 * s;
   }
 
-  // bytes one SpMV on the FP16 copy moves: 18 B of values and a 4-byte column per entry, the gathered vector
+  // bytes one SpMV on the FP16 copy moves: 18 B of values and a 2- or 4-byte column per entry, the gathered vector
   // and the product once, the inverse scale for the unscaled residual norm
   double half_spmv_bytes() const { return (h16vs == 2 ? 20.0 : 22.0) * (double)nfs + 3.0 * nv * 16.0; }
   // bytes one PCG update pass moves: p, q, x, r read, x, r, z written, the 3x3 preconditioner blocks
